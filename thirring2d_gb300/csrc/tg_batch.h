@@ -2,7 +2,7 @@
 // (tg_batch.cu), shared with the C ABI in tg_capi.cu.
 #pragma once
 
-#include "tg_internal.cuh"
+#include "tg_fixed.cuh"
 
 namespace tg {
 
@@ -19,6 +19,7 @@ struct BatchChain {
 // Packed per-site fields of all chains.
 struct BatchFields {
   double2 *A, *An, *mom, *phi, *noise, *x, *Mx, *tmp, *Wt, *Wx, *r64, *p64, *p64b, *Mp64;
+  FxLink *Wtq, *Wxq;
   float2 *Wt32, *Wx32, *xs, *rs, *ps, *ps2, *Mps;  // p64/p64b, ps/ps2: CG directions of alternate iterations
 };
 

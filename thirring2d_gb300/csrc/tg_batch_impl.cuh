@@ -258,7 +258,9 @@ struct ChainCtx {
   unsigned long long seed;
   // this chain's slices of the packed fields
   double2 *A, *An, *mom, *phi, *noise, *x, *Mx, *tmp, *Wt, *Wx, *r64, *p64, *p64b, *Mp64;
+  FxLink *Wtq, *Wxq;
   float2 *Wt32, *Wx32, *xs, *rs, *ps, *ps2, *Mps;
+  OpK<double> km, kd;  // the constants of M and M^dag
 };
 
 struct CgOut {
@@ -287,7 +289,7 @@ struct CgTailMx {
 template <bool MU0, class T>
 __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
   const int V = c.g.V;
-  OpK<double> km{c.m, c.ep, -c.em, MU0}, kd{c.m, -c.em, c.ep, MU0};
+  const OpK<double>&km = c.km, &kd = c.kd;
   double a = 0;
   TG_BSITES(s, V) {
     double2 bb = b[s];
@@ -322,7 +324,7 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
       v = fma(o.x, o.x, v);
       v = fma(o.y, o.y, v);
     };
-    stencil_team<T, double, 0, MU0>(c.g, km, ld, c.Wt, c.Wx, epi);
+    stencil_team<T, double, 0, MU0>(c.g, km, ld, c.Wtq, c.Wxq, epi);
     const double alpha = T::sum_then(v, [&](double pAp) { return rr / pAp; });
     v = 0;
     auto ld2 = [&](int i) { return c.Mp64[i]; };
@@ -337,7 +339,7 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
       v = fma(rv.x, rv.x, v);
       v = fma(rv.y, rv.y, v);
     };
-    stencil_team<T, double, 1, MU0>(c.g, kd, ld2, c.Wt, c.Wx, epi2);
+    stencil_team<T, double, 1, MU0>(c.g, kd, ld2, c.Wtq, c.Wxq, epi2);
     const CgTail64 e = T::sum_then(v, [&](double rn) {
       CgTail64 o{rn, rn / rr, -1};
       if (isnan(rn)) o.status = TG_E_NAN;
@@ -362,7 +364,7 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
 template <bool MU0, class T>
 __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
   const int V = c.g.V;
-  OpK<double> km{c.m, c.ep, -c.em, MU0}, kd{c.m, -c.em, c.ep, MU0};
+  const OpK<double>&km = c.km, &kd = c.kd;
   OpK<float> km32{(float)c.m, (float)c.ep, (float)-c.em, MU0}, kd32{(float)c.m, (float)-c.em, (float)c.ep, MU0};
   double a = 0;
   TG_BSITES(s, V) {
@@ -448,11 +450,11 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
       c.xs[s] = make_float2(0.f, 0.f);
     }
     T::sync();
-    TG_BSITES(s, V) c.tmp[s] = dslash_at<double, 0, MU0>(c.g, km, x, c.Wt, c.Wx, s);
+    TG_BSITES(s, V) c.tmp[s] = dslash_at<double, 0, MU0>(c.g, km, x, c.Wtq, c.Wxq, s);
     T::sync();
     double a2 = 0;
     TG_BSITES(s, V) {
-      double2 ap = dslash_at<double, 1, MU0>(c.g, kd, c.tmp, c.Wt, c.Wx, s);
+      double2 ap = dslash_at<double, 1, MU0>(c.g, kd, c.tmp, c.Wtq, c.Wxq, s);
       double2 bb = b[s];
       double2 rv = make_double2(bb.x - ap.x, bb.y - ap.y);
       c.rs[s] = make_float2((float)rv.x, (float)rv.y);
@@ -486,7 +488,7 @@ template <bool MU0, class T>
 __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainResult* res) {
   const int V = c.g.V;
   const Geo& g = c.g;
-  OpK<double> km{c.m, c.ep, -c.em, MU0}, kd{c.m, -c.em, c.ep, MU0};
+  const OpK<double>&km = c.km, &kd = c.kd;
   const unsigned long long tr = res->traj;
   const bool noise_on = P.stochastic_term != 0;
   const double fac = kNf / c.gc;
@@ -494,7 +496,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
   double a_pf = 0, a_mom = 0, a_g = 0;
   TG_BSITES(s, V) {
     double2 a = c.A[s];
-    write_links(g, c.bc_t, c.bc_x, s, a, c.Wt, c.Wx, c.Wt32, c.Wx32);
+    write_links(g, c.bc_t, c.bc_x, s, a, LinkOut{c.Wt, c.Wx, c.Wt32, c.Wx32, c.Wtq, c.Wxq});
     double2 e = philox_gauss_pair(c.seed, tr, (unsigned)s, 0u);
     c.tmp[s] = e;
     a_pf += e.x * e.x + e.y * e.y;
@@ -508,9 +510,9 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
   const double Spf0 = T::sum(a_pf), Smom0 = T::sum(a_mom), Sg0 = fac * T::sum(a_g);
   double a_md = 0;
   TG_BSITES(s, V) {
-    c.phi[s] = dslash_at<double, 1, MU0>(g, kd, c.tmp, c.Wt, c.Wx, s);  // phi = M^dag eta
+    c.phi[s] = dslash_at<double, 1, MU0>(g, kd, c.tmp, c.Wtq, c.Wxq, s);  // phi = M^dag eta
     if (noise_on) {
-      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wt, c.Wx, s);
+      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wtq, c.Wxq, s);
       double2 n = c.noise[s];
       a_md += n.x * o.x + n.y * o.y;
     }
@@ -530,7 +532,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
         a.y = __dadd_rn(a.y, __dmul_rn(cstep, p.y));
       }
       c.An[s] = a;
-      write_links(g, c.bc_t, c.bc_x, s, a, c.Wt, c.Wx, c.Wt32, c.Wx32);
+      write_links(g, c.bc_t, c.bc_x, s, a, LinkOut{c.Wt, c.Wx, c.Wt32, c.Wx32, c.Wtq, c.Wxq});
     }
     T::sync();
     CgOut o = block_cg<MU0, T>(c, P.cg, c.phi, c.x);
@@ -543,7 +545,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     // in tmp (the same function of the same operands); otherwise apply M.
     const double2* Mx = c.tmp;
     if (P.cg.precision != TG_PREC_MIXED || o.n_ru == 0) {
-      TG_BSITES(s, V) c.Mx[s] = dslash_at<double, 0, MU0>(g, km, c.x, c.Wt, c.Wx, s);
+      TG_BSITES(s, V) c.Mx[s] = dslash_at<double, 0, MU0>(g, km, c.x, c.Wtq, c.Wxq, s);
       T::sync();
       Mx = c.Mx;
     }
@@ -571,7 +573,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     b_mom += p.x * p.x + p.y * p.y;
     b_g += (1. - cos(a.x)) + (1. - cos(a.y));
     if (noise_on) {
-      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wt, c.Wx, s);
+      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wtq, c.Wxq, s);
       double2 n = c.noise[s];
       b_md += n.x * o.x + n.y * o.y;
     }
@@ -611,6 +613,9 @@ __device__ __forceinline__ void fill_ctx(ChainCtx& c, const BatchChain& b, const
     c.A = F.A + o; c.An = F.An + o; c.mom = F.mom + o; c.phi = F.phi + o; c.noise = F.noise + o;
     c.x = F.x + o; c.Mx = F.Mx + o; c.tmp = F.tmp + o; c.Wt = F.Wt + o; c.Wx = F.Wx + o;
     c.r64 = F.r64 + o; c.p64 = F.p64 + o; c.p64b = F.p64b + o; c.Mp64 = F.Mp64 + o;
+    c.Wtq = F.Wtq + o; c.Wxq = F.Wxq + o;
+    c.km = make_opk(b.m, c.ep, -c.em, b.mu == 0.0);
+    c.kd = make_opk(b.m, -c.em, c.ep, b.mu == 0.0);
     c.Wt32 = F.Wt32 + o; c.Wx32 = F.Wx32 + o; c.xs = F.xs + o; c.rs = F.rs + o; c.ps = F.ps + o;
     c.ps2 = F.ps2 + o; c.Mps = F.Mps + o;
 }

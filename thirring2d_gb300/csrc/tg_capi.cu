@@ -109,7 +109,7 @@ struct tg_lattice {
   cudaStream_t stream = nullptr, cap2 = nullptr, cap3 = nullptr;
 
   double2 *A = nullptr, *Anew = nullptr, *Wt = nullptr, *Wx = nullptr;
-  double2 *Wt1 = nullptr, *Wx1 = nullptr;  // W / m (unit-mass FP64 CG)
+  FxLink *Wtq = nullptr, *Wxq = nullptr;  // W as fixed-point limbs (the FP64 operator)
   float2 *Wt32 = nullptr, *Wx32 = nullptr;
   double2 *mom = nullptr, *noise = nullptr, *chi = nullptr, *Mchi = nullptr, *vin = nullptr, *vout = nullptr;
   double2 *eta = nullptr, *phi = nullptr;  // [npf_alloc][V]
@@ -151,13 +151,8 @@ struct Range {
 };
 
 OpK<double> op_k(const tg_lattice* L, int dagger) {
-  double ep = exp(L->P.mu), em = exp(-L->P.mu);
-  OpK<double> k;
-  k.m = L->P.m;
-  if (!dagger) { k.cf = ep; k.cb = -em; }
-  else { k.cf = -em; k.cb = ep; }
-  k.mu0 = L->P.mu == 0.0;
-  return k;
+  const double ep = exp(L->P.mu), em = exp(-L->P.mu);
+  return dagger ? make_opk(L->P.m, -em, ep, L->P.mu == 0.0) : make_opk(L->P.m, ep, -em, L->P.mu == 0.0);
 }
 OpK<float> op_k32(const tg_lattice* L, int dagger) {
   OpK<double> k = op_k(L, dagger);
@@ -170,30 +165,8 @@ OpK<float> op_k32(const tg_lattice* L, int dagger) {
 // FP64 1.416 vs 1.342, mixed 5.56 vs 4.33 trajectories/s
 constexpr bool kDefaultPersistent = true;
 
-// The FP64 CG runs in unit-mass form (links W / m) whenever 1/m is a finite
-// nonzero number; m = 0 keeps the plain form.
-bool unit_mass(const tg_lattice* L) {
-  const double m = L->P.m;
-  return m != 0.0 && std::isfinite(1.0 / m) && std::isfinite(1.0 / (m * m)) && 1.0 / (m * m) != 0.0;
-}
-Links links(const tg_lattice* L) {
-  Links lk{L->Wt, L->Wx, L->Wt32, L->Wx32};
-  if (unit_mass(L)) {
-    lk.Wt1 = L->Wt1;
-    lk.Wx1 = L->Wx1;
-    lk.inv_m2 = 1.0 / (L->P.m * L->P.m);
-  }
-  return lk;
-}
-LinkOut link_out(const tg_lattice* L) {
-  LinkOut o{L->Wt, L->Wx, L->Wt32, L->Wx32};
-  if (unit_mass(L)) {
-    o.Wt1 = L->Wt1;
-    o.Wx1 = L->Wx1;
-    o.inv_m = 1.0 / L->P.m;
-  }
-  return o;
-}
+Links links(const tg_lattice* L) { return Links{L->Wtq, L->Wxq, L->Wt32, L->Wx32}; }
+LinkOut link_out(const tg_lattice* L) { return LinkOut{L->Wt, L->Wx, L->Wt32, L->Wx32, L->Wtq, L->Wxq}; }
 
 bool env_graph_enabled() {
   const char* e = getenv("TG_GRAPH");
@@ -318,8 +291,8 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.kd = op_k(L, 1);
     a.Wt32 = lk.Wt32;
     a.Wx32 = lk.Wx32;
-    a.Wt = lk.Wt;
-    a.Wx = lk.Wx;
+    a.Wt = lk.Wtq;
+    a.Wx = lk.Wxq;
     a.b = b;
     a.x = x;
     a.tmp = L->wmx.tmp64;
@@ -349,10 +322,8 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.g = L->g;
     a.km = op_k(L, 0);
     a.kd = op_k(L, 1);
-    const bool unit = lk.Wt1 != nullptr;
-    a.Wt = unit ? lk.Wt1 : lk.Wt;
-    a.Wx = unit ? lk.Wx1 : lk.Wx;
-    a.inv_m2 = unit ? lk.inv_m2 : 0.0;
+    a.Wt = lk.Wtq;
+    a.Wx = lk.Wxq;
     a.b = b;
     a.x = x;
     a.r = L->w64.r;
@@ -568,11 +539,11 @@ int enqueue_trajectory(tg_lattice* L, cudaStream_t s, const tg_hmc_params& p, bo
     TG_CK(cudaMemsetAsync(&ts->Spf0, 0, sizeof(double), s));
     for (int k = 0; k < p.npf; k++) {
       norm2(s, g, L->eta + (size_t)k * V, &ts->Spf0, 1, L->red);
-      dslash64(s, g, kd, 1, L->eta + (size_t)k * V, L->phi + (size_t)k * V, L->Wt, L->Wx);
+      dslash64(s, g, kd, 1, L->eta + (size_t)k * V, L->phi + (size_t)k * V, L->Wtq, L->Wxq);
     }
     norm2(s, g, L->mom, &ts->Smom0, 0, L->red);
     gauge_action(s, g, L->A, kNf / L->P.g, &ts->Sg0, L->red);
-    if (use_noise) md_action(s, g, kd, L->noise, L->Wt, L->Wx, &ts->Smd0, L->red);
+    if (use_noise) md_action(s, g, kd, L->noise, L->Wtq, L->Wxq, &ts->Smd0, L->red);
     else TG_CK(cudaMemsetAsync(&ts->Smd0, 0, sizeof(double), s));
     TG_CK(cudaMemcpyAsync(L->Anew, L->A, (size_t)V * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   }
@@ -588,7 +559,7 @@ int enqueue_trajectory(tg_lattice* L, cudaStream_t s, const tg_hmc_params& p, bo
                       1 | (use_noise ? 2 : 0));
     for (int k = 0; k < p.npf; k++) {
       TG_TRY(cg(L->phi + (size_t)k * V, L->chi));
-      dslash64(s, g, km, 0, L->chi, L->Mchi, L->Wt, L->Wx);
+      dslash64(s, g, km, 0, L->chi, L->Mchi, L->Wtq, L->Wxq);
       int flags = (k == 0 ? 1 : 0) | ((k == p.npf - 1 && use_noise) ? 2 : 0);
       momentum_update(s, g, L->P.bc_t, L->P.bc_x, ep, em, L->Anew, L->Wt, L->Wx, L->chi, L->Mchi, L->noise, L->mom, eps, gfac, flags);
     }
@@ -603,7 +574,7 @@ int enqueue_trajectory(tg_lattice* L, cudaStream_t s, const tg_hmc_params& p, bo
   }
   norm2(s, g, L->mom, &ts->Smom1, 0, L->red);
   gauge_action(s, g, L->Anew, kNf / L->P.g, &ts->Sg1, L->red);
-  if (use_noise) md_action(s, g, kd, L->noise, L->Wt, L->Wx, &ts->Smd1, L->red);
+  if (use_noise) md_action(s, g, kd, L->noise, L->Wtq, L->Wxq, &ts->Smd1, L->red);
   else TG_CK(cudaMemsetAsync(&ts->Smd1, 0, sizeof(double), s));
   finish_trajectory(s, ts);
   accept_copy(s, g, ts, L->A, L->Anew);
@@ -786,9 +757,11 @@ int tg_create(const tg_lattice_params* p, tg_lattice** out) {
     return bail(fail(TG_E_CUDA, "stream creation failed"));
   size_t n = (size_t)V;
   int rc = TG_OK;
-  double2** d2[] = {&L->A, &L->Anew, &L->Wt, &L->Wx, &L->Wt1, &L->Wx1, &L->mom, &L->noise, &L->chi, &L->Mchi, &L->vin, &L->vout,
+  double2** d2[] = {&L->A, &L->Anew, &L->Wt, &L->Wx, &L->mom, &L->noise, &L->chi, &L->Mchi, &L->vin, &L->vout,
                     &L->w64.r, &L->w64.p[0], &L->w64.p[1], &L->w64.Mp, &L->wmx.tmp64};
   for (auto pp : d2)
+    if ((rc = dmalloc(pp, n)) != TG_OK) return bail(rc);
+  for (auto pp : {&L->Wtq, &L->Wxq})
     if ((rc = dmalloc(pp, n)) != TG_OK) return bail(rc);
   float2** f2[] = {&L->Wt32, &L->Wx32, &L->wmx.xs, &L->wmx.rs, &L->wmx.ps[0], &L->wmx.ps[1], &L->wmx.Mps,
                    &L->wmx.ss};
@@ -830,7 +803,7 @@ int tg_destroy(tg_lattice* L) {
     if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
   }
   for (auto e : L->ev) cudaEventDestroy(e);
-  void* dev[] = {L->A, L->Anew, L->Wt, L->Wx, L->Wt1, L->Wx1, L->mom, L->noise, L->chi, L->Mchi, L->vin, L->vout, L->w64.r,
+  void* dev[] = {L->A, L->Anew, L->Wt, L->Wx, L->Wtq, L->Wxq, L->mom, L->noise, L->chi, L->Mchi, L->vin, L->vout, L->w64.r,
                  L->w64.p[0], L->w64.p[1], L->w64.Mp, L->wmx.tmp64, L->Wt32, L->Wx32, L->wmx.xs, L->wmx.rs,
                  L->wmx.ps[0], L->wmx.ps[1], L->wmx.Mps, L->wmx.ss,
                  L->st, L->log, L->ts, L->red.partials, L->red.counter, L->bar, L->pcg_part, L->eta, L->phi, L->unif, L->mask,
@@ -854,8 +827,6 @@ int tg_set_couplings(tg_lattice* L, double m, double g, double mu) {
   L->P.g = g;
   L->P.mu = mu;
   L->version++;
-  link_phase(L->stream, L->g, L->P.bc_t, L->P.bc_x, L->A, link_out(L));  // W / m follows m
-  TG_CK(cudaGetLastError());
   return TG_OK;
 }
 
@@ -897,7 +868,7 @@ int tg_get_gauge(tg_lattice* L, double* A) {
 int tg_apply(tg_lattice* L, const double* in, double* out, int dagger) {
   if (!L || !in || !out) return fail(TG_E_ARG, "null argument");
   TG_TRY(upload(L, L->vin, in, 2 * (size_t)L->V));
-  dslash64(L->stream, L->g, op_k(L, dagger), dagger, L->vin, L->vout, L->Wt, L->Wx);
+  dslash64(L->stream, L->g, op_k(L, dagger), dagger, L->vin, L->vout, L->Wtq, L->Wxq);
   TG_CK(cudaGetLastError());
   return download(L, out, L->vout, 2 * (size_t)L->V);
 }
@@ -905,7 +876,7 @@ int tg_apply(tg_lattice* L, const double* in, double* out, int dagger) {
 int tg_apply_dev(tg_lattice* L, const void* in, void* out, int dagger, int precision) {
   if (!L || !in || !out) return fail(TG_E_ARG, "null argument");
   if (precision == TG_PREC_FP64)
-    dslash64(L->stream, L->g, op_k(L, dagger), dagger, (const double2*)in, (double2*)out, L->Wt, L->Wx);
+    dslash64(L->stream, L->g, op_k(L, dagger), dagger, (const double2*)in, (double2*)out, L->Wtq, L->Wxq);
   else if (precision == TG_PREC_MIXED)
     dslash32(L->stream, L->g, op_k32(L, dagger), dagger, (const float2*)in, (float2*)out, L->Wt32, L->Wx32);
   else
@@ -924,7 +895,7 @@ int tg_time_apply(tg_lattice* L, int n, int dagger, int precision, double* ms_pe
     if (precision == TG_PREC_FP64) {
       const double2* in = (i & 1) ? L->vout : L->vin;
       double2* out = (i & 1) ? L->vin : L->vout;
-      dslash64(L->stream, L->g, op_k(L, dagger), dagger, in, out, L->Wt, L->Wx);
+      dslash64(L->stream, L->g, op_k(L, dagger), dagger, in, out, L->Wtq, L->Wxq);
     } else {
       const float2* in = (i & 1) ? L->wmx.Mps : L->wmx.ps[0];
       float2* out = (i & 1) ? L->wmx.ps[0] : L->wmx.Mps;
@@ -988,7 +959,7 @@ int tg_pseudofermion_action(tg_lattice* L, const tg_cg_params* cp, const double*
 int tg_md_action(tg_lattice* L, const double* n, double* S) {
   if (!L || !n || !S) return fail(TG_E_ARG, "null argument");
   TG_TRY(upload(L, L->vin, n, 2 * (size_t)L->V));
-  md_action(L->stream, L->g, op_k(L, 1), L->vin, L->Wt, L->Wx, &L->ts->Smd0, L->red);
+  md_action(L->stream, L->g, op_k(L, 1), L->vin, L->Wtq, L->Wxq, &L->ts->Smd0, L->red);
   TG_CK(cudaGetLastError());
   TG_CK(cudaMemcpyAsync(S, &L->ts->Smd0, sizeof(double), cudaMemcpyDeviceToHost, L->stream));
   TG_CK(cudaStreamSynchronize(L->stream));
@@ -1006,7 +977,7 @@ int tg_force(tg_lattice* L, int npf, const double* chi, const double* noise, dou
                 1 | (noise ? 2 : 0));
   for (int k = 0; k < npf; k++) {
     TG_TRY(upload(L, L->chi, chi + 2 * V * k, 2 * V));
-    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wt, L->Wx);
+    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wtq, L->Wxq);
     int flags = (k == 0 ? 1 : 0) | ((k == npf - 1 && noise) ? 2 : 0);
     force_field(L->stream, L->g, L->P.bc_t, L->P.bc_x, ep, em, L->A, L->Wt, L->Wx, L->chi, L->Mchi, L->noise, L->vout, kNf / L->P.g,
                 flags);
@@ -1032,7 +1003,7 @@ int tg_pf_force(tg_lattice* L, const tg_cg_params* cp, int npf, const double* ph
     if (r.status > acc.status) acc.status = r.status;
     acc.rr = r.rr;
     acc.rr0 = r.rr0;
-    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wt, L->Wx);
+    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wtq, L->Wxq);
     force_field(L->stream, L->g, L->P.bc_t, L->P.bc_x, ep, em, L->A, L->Wt, L->Wx, L->chi, L->Mchi, nullptr, L->vout, 0.0, 0);
   }
   TG_CK(cudaGetLastError());
@@ -1064,7 +1035,7 @@ int tg_momentum_step(tg_lattice* L, const tg_cg_params* cp, double* mom, int npf
     if (r.status > acc.status) acc.status = r.status;
     acc.rr = r.rr;
     acc.rr0 = r.rr0;
-    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wt, L->Wx);
+    dslash64(L->stream, L->g, op_k(L, 0), 0, L->chi, L->Mchi, L->Wtq, L->Wxq);
     int flags = (k == 0 ? 1 : 0) | ((k == npf - 1 && noise) ? 2 : 0);
     momentum_update(L->stream, L->g, L->P.bc_t, L->P.bc_x, ep, em, L->A, L->Wt, L->Wx, L->chi, L->Mchi, L->noise, L->mom, eps, gfac,
                     flags);
@@ -1242,7 +1213,7 @@ int tg_fermion_phase(tg_lattice* L, int sources, const double* noise, double* ph
       src = draw.data();
     }
     TG_TRY(upload(L, L->vin, src, 2 * V));
-    dslash64(L->stream, L->g, op_k(L, 1), 1, L->vin, L->vout, L->Wt, L->Wx);
+    dslash64(L->stream, L->g, op_k(L, 1), 1, L->vin, L->vout, L->Wtq, L->Wxq);
     imdot(L->stream, L->g, L->vin, L->vout, &L->ts->Smd1, 1, L->red);
     TG_CK(cudaGetLastError());
   }
@@ -1259,7 +1230,7 @@ int tg_chiral_condensate(tg_lattice* L, const tg_cg_params* cp, int sources, uns
   std::vector<double> vals(sources);
   for (int k = 0; k < sources; k++) {
     philox_gauss(L->stream, L->g, seed, L->ts, 64u + (unsigned)k, L->vin);    // eta
-    dslash64(L->stream, L->g, op_k(L, 1), 1, L->vin, L->Mchi, L->Wt, L->Wx);  // M^dag eta
+    dslash64(L->stream, L->g, op_k(L, 1), 1, L->vin, L->Mchi, L->Wtq, L->Wxq);  // M^dag eta
     TG_CK(cudaGetLastError());
     tg_cg_result r{};
     TG_TRY(solve_dev(L, *cp, L->Mchi, L->chi, &r));                         // M^-1 eta
@@ -1664,6 +1635,8 @@ int tg_batch_create(const tg_chain_params* chains, int nchains, int device, tg_b
                     &B->F.Wt, &B->F.Wx, &B->F.r64, &B->F.p64, &B->F.p64b, &B->F.Mp64};
   for (auto pp : d2)
     if ((rc = dmalloc(pp, (size_t)total)) != TG_OK) return bail(rc);
+  for (auto pp : {&B->F.Wtq, &B->F.Wxq})
+    if ((rc = dmalloc(pp, (size_t)total)) != TG_OK) return bail(rc);
   float2** f2[] = {&B->F.Wt32, &B->F.Wx32, &B->F.xs, &B->F.rs, &B->F.ps, &B->F.ps2, &B->F.Mps};
   for (auto pp : f2)
     if ((rc = dmalloc(pp, (size_t)total)) != TG_OK) return bail(rc);
@@ -1703,7 +1676,7 @@ int tg_batch_destroy(tg_batch* B) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
   }
-  void* dev[] = {B->F.A, B->F.An, B->F.mom, B->F.phi, B->F.noise, B->F.x, B->F.Mx, B->F.tmp, B->F.Wt, B->F.Wx,
+  void* dev[] = {B->F.A, B->F.An, B->F.mom, B->F.phi, B->F.noise, B->F.x, B->F.Mx, B->F.tmp, B->F.Wt, B->F.Wx, B->F.Wtq, B->F.Wxq,
                  B->F.r64, B->F.p64, B->F.p64b, B->F.Mp64, B->F.Wt32, B->F.Wx32, B->F.xs, B->F.rs, B->F.ps,
                  B->F.ps2, B->F.Mps,
                  B->d_chains, B->d_order, B->d_res, B->d_queue};

@@ -29,43 +29,31 @@ __device__ __forceinline__ void link_vals(const Geo& g, int bc_t, int bc_x, int 
   wx = make_double2(fx * cx, fx * sx);
 }
 
-__device__ __forceinline__ void write_links(const Geo& g, int bc_t, int bc_x, int s, double2 a, double2* Wt,
-                                            double2* Wx, float2* Wt32, float2* Wx32) {
-  double2 wt, wx;
-  link_vals(g, bc_t, bc_x, s, a, wt, wx);
-  Wt[s] = wt;
-  Wx[s] = wx;
-  Wt32[s] = make_float2((float)wt.x, (float)wt.y);
-  Wx32[s] = make_float2((float)wx.x, (float)wx.y);
-}
-
-// ... and W / m for the unit-mass operator M / m = 1 + D / m when o.Wt1 is set
 __device__ __forceinline__ void write_links(const Geo& g, int bc_t, int bc_x, int s, double2 a, const LinkOut& o) {
   double2 wt, wx;
   link_vals(g, bc_t, bc_x, s, a, wt, wx);
-  o.Wt[s] = wt;
-  o.Wx[s] = wx;
+  if (o.Wt != nullptr) {
+    o.Wt[s] = wt;
+    o.Wx[s] = wx;
+  }
   o.Wt32[s] = make_float2((float)wt.x, (float)wt.y);
   o.Wx32[s] = make_float2((float)wx.x, (float)wx.y);
-  if (o.Wt1 != nullptr) {
-    o.Wt1[s] = make_double2(wt.x * o.inv_m, wt.y * o.inv_m);
-    o.Wx1[s] = make_double2(wx.x * o.inv_m, wx.y * o.inv_m);
-  }
+  o.Wtq[s] = to_fx_link(wt);
+  o.Wxq[s] = to_fx_link(wx);
 }
 
 // ---------------------------------------------------------------------------
 // The staggered operator at one site: hmc.c:132-183 for M (DAG = 0) and the
 // true adjoint M^dagger = m - D(-mu) (DAG = 1).  MU0 drops the e^{+-mu}
-// factors (mu = 0): 18 FMA/MUL per site instead of 22.  UNIT applies
-// M / m = 1 + D / m instead (the links passed in are then W / m): the mass
-// product goes, 16 FMA per site.
+// factors (mu = 0): 18 FMA/MUL per site instead of 22.  This is the FP32
+// operator, and the FP64 one where fx_dslash (tg_fixed.cuh) is out of range.
 // ---------------------------------------------------------------------------
-template <typename R, int DAG, bool MU0, bool UNIT = false>
+template <typename R, int DAG, bool MU0>
 __device__ __forceinline__ C2<R> dslash_vals(const OpK<R>& k, C2<R> pc, C2<R> ptu, C2<R> ptd, C2<R> pxu, C2<R> pxd,
                                              C2<R> wt, C2<R> wtd, C2<R> wx, C2<R> wxd) {
   // pc = in(s); ptu/ptd = in(s+t)/in(s-t); pxu/pxd = in(s+x)/in(s-x);
   // wt = Wt(s), wtd = Wt(s-t), wx = Wx(s), wxd = Wx(s-x)
-  C2<R> o = UNIT ? pc : mk<R>(k.m * pc.x, k.m * pc.y);
+  C2<R> o = mk<R>(k.m * pc.x, k.m * pc.y);
   if (MU0) {
     if (DAG == 0) {
       cmac<R>(o, wt, ptu);
@@ -92,20 +80,40 @@ __device__ __forceinline__ C2<R> dslash_vals(const OpK<R>& k, C2<R> pc, C2<R> pt
   return o;
 }
 
-template <typename R, int DAG, bool MU0>
-__device__ __forceinline__ C2<R> dslash_site(const OpK<R>& k, const C2<R>* __restrict__ in,
-                                             const C2<R>* __restrict__ Wt, const C2<R>* __restrict__ Wx, int s,
-                                             const Nbr& n) {
-  return dslash_vals<R, DAG, MU0>(k, in[s], in[n.tp], in[n.tm], in[n.xp], in[n.xm], Wt[s], Wt[n.tm], Wx[s],
-                                  Wx[n.xm]);
+// The links an operator of precision R reads: FP32 values, or the limbs of the
+// FP64 operator.
+template <typename R> struct LkT;
+template <> struct LkT<float> { using type = float2; };
+template <> struct LkT<double> { using type = FxLink; };
+template <typename R> using Lk = typename LkT<R>::type;
+
+// The operator at site s = (t, x) with operands from ld; own = the operand at s.
+template <typename R, int DAG, bool MU0, class Ld>
+__device__ __forceinline__ C2<R> dslash_ld(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
+                                           const Lk<R>* __restrict__ Wx, int s, int t, int x, C2<R>& own) {
+  const Nbr n = neighbours(g, s, t, x);
+  own = ld(s);
+  const C2<R> tu = ld(n.tp), td = ld(n.tm), xu = ld(n.xp), xd = ld(n.xm);
+  const Lk<R> wt = Wt[s], wtd = Wt[n.tm], wx = Wx[s], wxd = Wx[n.xm];
+  if constexpr (sizeof(R) == 4) {
+    return dslash_vals<R, DAG, MU0>(k, own, tu, td, xu, xd, wt, wtd, wx, wxd);
+  } else {
+    double2 o;
+    if (!fx_dslash<DAG, MU0>(k, to_fx(own), to_fx(tu), to_fx(td), to_fx(xu), to_fx(xd), wt, wtd, wx, wxd, o))
+      o = dslash_vals<R, DAG, MU0>(k, own, tu, td, xu, xd, fx_link_value(wt), fx_link_value(wtd), fx_link_value(wx),
+                                   fx_link_value(wxd));
+    return o;
+  }
 }
 
 template <typename R, int DAG, bool MU0>
 __device__ __forceinline__ C2<R> dslash_at(const Geo& g, const OpK<R>& k, const C2<R>* __restrict__ in,
-                                           const C2<R>* __restrict__ Wt, const C2<R>* __restrict__ Wx, int s) {
+                                           const Lk<R>* __restrict__ Wt, const Lk<R>* __restrict__ Wx, int s) {
   int t, x;
   site_tx(g, s, t, x);
-  return dslash_site<R, DAG, MU0>(k, in, Wt, Wx, s, neighbours(g, s, t, x));
+  auto ld = [&](int i) { return in[i]; };
+  C2<R> own;
+  return dslash_ld<R, DAG, MU0>(g, k, ld, Wt, Wx, s, t, x, own);
 }
 
 template <typename R> __device__ __forceinline__ C2<R> shfl_down1(C2<R> v) {

@@ -73,7 +73,7 @@ struct Geo {
 // leaves 3 coalesced loads (psi(t+1), Wt, Wx) instead of 9.
 constexpr int kMarchT = 4;
 // Minimum resident blocks per SM the stencil kernels are compiled for.
-constexpr int kStencilBlocksPerSM = 1;  // no register cap: capping at 42 spilled heavily
+constexpr int kStencilBlocksPerSM = 2;
 
 __device__ __forceinline__ void site_tx(const Geo& g, int s, int& t, int& x) {
   // V < 2^24 keeps float(s) exact; the fix-up absorbs the rounding of s/nx.
@@ -97,6 +97,7 @@ __device__ __forceinline__ Nbr neighbours(const Geo& g, int s, int t, int x) {
 // M: cf = e^mu, cb = -e^-mu, sx = +1 (hmc.c:137-180); M^dag: cf = -e^-mu, cb = e^mu, sx = -1.
 // sx is a template parameter of the kernels; mu0 = (mu == 0) selects the
 // variant without the e^{+-mu} multiplies (18 instead of 22 FMA/MUL per site).
+// (OpK<double>, tg_fixed.cuh, also holds them as integer limbs.)
 template <typename R> struct OpK {
   R m, cf, cb;
   int mu0;

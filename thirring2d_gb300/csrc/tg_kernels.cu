@@ -118,10 +118,10 @@ bool staged_enabled(const Geo& g) {
 
 template <typename R, int DAG, bool MU0, bool STAGED = false>
 __global__ void __launch_bounds__(kBlock, kFp32BlocksPerSM<R>) k_dslash(Geo g, OpK<R> k, const C2<R>* __restrict__ in,
-                                                   C2<R>* __restrict__ out, const C2<R>* __restrict__ Wt,
-                                                   const C2<R>* __restrict__ Wx) {
+                                                   C2<R>* __restrict__ out, const Lk<R>* __restrict__ Wt,
+                                                   const Lk<R>* __restrict__ Wx) {
   auto epi = [&](int s, C2<R> o, C2<R>) { out[s] = o; };
-  if constexpr (STAGED) stencil_staged<R, DAG, MU0, false>(g, k, SrcOne<R>{in}, Wt, Wx, epi);
+  if constexpr (STAGED) stencil_staged<R, DAG, MU0>(g, k, SrcOne<R>{in}, Wt, Wx, epi);
   else stencil_all<R, DAG, MU0>(g, k, in, Wt, Wx, epi);
 }
 
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kBlock, kFp32BlocksPerSM<R>) k_dslash(Geo g, O
   } while (0)
 
 void dslash64(cudaStream_t s, const Geo& g, const OpK<double>& k, int dag, const double2* in, double2* out,
-              const double2* Wt, const double2* Wx) {
+              const FxLink* Wt, const FxLink* Wx) {
   const int w = stencil_work(g);
   if (dag)
     TG_OP_DISPATCH(k, (k_dslash<double, 1, MU0><<<occ_grid(k_dslash<double, 1, MU0>, w), kBlock, 0, s>>>(
@@ -237,11 +237,11 @@ __global__ void __launch_bounds__(kBlock) k_cg_init(Geo g, const double2* __rest
   }
 }
 
-template <typename R, bool MU0, bool UNIT = false, bool STAGED = false>
+template <typename R, bool MU0, bool STAGED = false>
 __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? kFp32BlocksPerSM<R> : 2) k_cg1(Geo g, OpK<R> k, const C2<R>* __restrict__ r,
                                                 const C2<R>* __restrict__ p_old, C2<R>* __restrict__ p_new,
-                                                C2<R>* __restrict__ Mp, const C2<R>* __restrict__ Wt,
-                                                const C2<R>* __restrict__ Wx, CgState* st, Red red) {
+                                                C2<R>* __restrict__ Mp, const Lk<R>* __restrict__ Wt,
+                                                const Lk<R>* __restrict__ Wx, CgState* st, Red red) {
   if (st->done) return;
   const R b = (R)st->beta;
   R v = 0;
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? kFp32BlocksPerSM<R> :
     v = fma(o.x, o.x, v);
     v = fma(o.y, o.y, v);
   };
-  if constexpr (STAGED) stencil_staged<R, 0, MU0, UNIT>(g, k, SrcAxpy<R>{r, p_old, b}, Wt, Wx, epi);
-  else stencil_ld<R, 0, MU0, UNIT>(g, k, ld, Wt, Wx, epi);
+  if constexpr (STAGED) stencil_staged<R, 0, MU0>(g, k, SrcAxpy<R>{r, p_old, b}, Wt, Wx, epi);
+  else stencil_ld<R, 0, MU0>(g, k, ld, Wt, Wx, epi);
   double tot;
   if (grid_sum<kBlock, R>(v, red.partials, red.counter, &tot) && threadIdx.x == 0) {
     st->alpha = st->rr / tot;
@@ -266,23 +266,19 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? kFp32BlocksPerSM<R> :
 }
 
 // FP64: convergence tested on the recursive residual, as hmc.c:381.
-// UNIT: the pair runs CG on N^dag N with N = M / m (links W / m).  Its residual
-// b - N^dag N (m^2 x) is b's residual for x, so r, p, beta and the stopping test
-// are M's, and alpha_N = m^2 alpha_M: x advances by (alpha_N / m^2) p.
-template <bool MU0, bool UNIT = false>
+template <bool MU0>
 __global__ void __launch_bounds__(kBlock, 2) k_cg2_64(Geo g, OpK<double> k, const double2* __restrict__ Mp,
                                                    const double2* __restrict__ p, double2* __restrict__ x,
-                                                   double2* __restrict__ r, const double2* __restrict__ Wt,
-                                                   const double2* __restrict__ Wx, CgState* st, CgLog* log,
-                                                   Red red, Cond c, double inv_m2 = 1.0) {
+                                                   double2* __restrict__ r, const FxLink* __restrict__ Wt,
+                                                   const FxLink* __restrict__ Wx, CgState* st, CgLog* log,
+                                                   Red red, Cond c) {
   if (st->done) return;
   const double a = st->alpha;
-  const double ax = UNIT ? a * inv_m2 : a;
   double v = 0;
   auto epi = [&](int s, double2 ap, double2) {
     double2 xv = x[s], pv = p[s], rv = r[s];
-    xv.x += ax * pv.x;
-    xv.y += ax * pv.y;
+    xv.x += a * pv.x;
+    xv.y += a * pv.y;
     rv.x -= a * ap.x;
     rv.y -= a * ap.y;
     x[s] = xv;
@@ -290,7 +286,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cg2_64(Geo g, OpK<double> k, cons
     v = fma(rv.x, rv.x, v);
     v = fma(rv.y, rv.y, v);
   };
-  stencil_all<double, 1, MU0, UNIT>(g, k, Mp, Wt, Wx, epi);
+  stencil_all<double, 1, MU0>(g, k, Mp, Wt, Wx, epi);
   double rn;
   if (grid_sum<kBlock, double>(v, red.partials, red.counter, &rn) && threadIdx.x == 0) {
     st->iter += 1;
@@ -315,17 +311,10 @@ void cg64_iter(cudaStream_t s, const Geo& g, const OpK<double>& km, const OpK<do
   const int wk = stencil_work(g);
   const double2* p_old = w.p[half];
   double2* p_new = w.p[half ^ 1];
-  if (L.Wt1 != nullptr) {
-    TG_OP_DISPATCH(km, (k_cg1<double, MU0, true><<<occ_grid(k_cg1<double, MU0, true>, wk), kBlock, 0, s>>>(
-                            g, km, w.r, p_old, p_new, w.Mp, L.Wt1, L.Wx1, st, red)));
-    TG_OP_DISPATCH(kd, (k_cg2_64<MU0, true><<<occ_grid(k_cg2_64<MU0, true>, wk), kBlock, 0, s>>>(
-                            g, kd, w.Mp, p_new, x, w.r, L.Wt1, L.Wx1, st, log, red, c, L.inv_m2)));
-    return;
-  }
   TG_OP_DISPATCH(km, (k_cg1<double, MU0><<<occ_grid(k_cg1<double, MU0>, wk), kBlock, 0, s>>>(
-                          g, km, w.r, p_old, p_new, w.Mp, L.Wt, L.Wx, st, red)));
-  TG_OP_DISPATCH(kd, (k_cg2_64<MU0><<<occ_grid(k_cg2_64<MU0>, wk), kBlock, 0, s>>>(g, kd, w.Mp, p_new, x, w.r, L.Wt,
-                                                                                 L.Wx, st, log, red, c)));
+                          g, km, w.r, p_old, p_new, w.Mp, L.Wtq, L.Wxq, st, red)));
+  TG_OP_DISPATCH(kd, (k_cg2_64<MU0><<<occ_grid(k_cg2_64<MU0>, wk), kBlock, 0, s>>>(g, kd, w.Mp, p_new, x, w.r, L.Wtq,
+                                                                                 L.Wxq, st, log, red, c)));
 }
 
 // ---------------------------------------------------------------------------
@@ -354,7 +343,7 @@ __global__ void __launch_bounds__(kBlock, kFp32BlocksPerSM<float>) k_cgmx2(Geo g
     v = fmaf(rv.x, rv.x, v);
     v = fmaf(rv.y, rv.y, v);
   };
-  if constexpr (STAGED) stencil_staged<float, 1, MU0, false>(g, k, SrcOne<float>{Mp}, Wt, Wx, epi);
+  if constexpr (STAGED) stencil_staged<float, 1, MU0>(g, k, SrcOne<float>{Mp}, Wt, Wx, epi);
   else stencil_all<float, 1, MU0>(g, k, Mp, Wt, Wx, epi);
   double rn;
   if (grid_sum<kBlock, float>(v, red.partials, red.counter, &rn) && threadIdx.x == 0) {
@@ -386,8 +375,8 @@ __global__ void __launch_bounds__(kBlock) k_ru1(int n, double2* x, float2* xs, c
 // reliable update 2: tmp = M x (FP64)
 template <bool MU0>
 __global__ void __launch_bounds__(kBlock, kStencilBlocksPerSM) k_ru2(Geo g, OpK<double> k, const double2* __restrict__ x,
-                                                double2* __restrict__ tmp, const double2* __restrict__ Wt,
-                                                const double2* __restrict__ Wx, const CgState* st) {
+                                                double2* __restrict__ tmp, const FxLink* __restrict__ Wt,
+                                                const FxLink* __restrict__ Wx, const CgState* st) {
   if (!st->need_ru || st->done) return;
   auto epi = [&](int s, double2 o, double2) { tmp[s] = o; };
   stencil_all<double, 0, MU0>(g, k, x, Wt, Wx, epi);
@@ -397,7 +386,7 @@ __global__ void __launch_bounds__(kBlock, kStencilBlocksPerSM) k_ru2(Geo g, OpK<
 template <bool MU0>
 __global__ void __launch_bounds__(kBlock, kStencilBlocksPerSM) k_ru3(Geo g, OpK<double> k, const double2* __restrict__ b,
                                                 const double2* __restrict__ tmp, float2* __restrict__ rs,
-                                                const double2* __restrict__ Wt, const double2* __restrict__ Wx,
+                                                const FxLink* __restrict__ Wt, const FxLink* __restrict__ Wx,
                                                 CgState* st, CgLog* log, Red red, Cond c) {
   if (!st->need_ru || st->done) return;
   double v = 0;
@@ -438,7 +427,7 @@ void cgmx_iter(cudaStream_t s, const Geo& g, const OpK<float>& km, const OpK<flo
   float2* p_new = w.ps[half ^ 1];
   if (staged_enabled(g)) {
     constexpr int sm1 = staged_smem_bytes<float, 2>(), sm2 = staged_smem_bytes<float, 1>();
-    TG_OP_DISPATCH(km, (k_cg1<float, MU0, false, true><<<occ_grid_smem(k_cg1<float, MU0, false, true>, wk, sm1),
+    TG_OP_DISPATCH(km, (k_cg1<float, MU0, true><<<occ_grid_smem(k_cg1<float, MU0, true>, wk, sm1),
                                                          kBlock, sm1, s>>>(g, km, w.rs, p_old, p_new, w.Mps, L.Wt32,
                                                                            L.Wx32, st, red)));
     TG_OP_DISPATCH(kd, (k_cgmx2<MU0, true><<<occ_grid_smem(k_cgmx2<MU0, true>, wk, sm2), kBlock, sm2, s>>>(
@@ -456,8 +445,8 @@ void cgmx_reliable(cudaStream_t s, const Geo& g, const OpK<double>& km, const Op
                    Cond c) {
   const int wk = stencil_work(g);
   k_ru1<<<stream_grid(g.V), kBlock, 0, s>>>(g.V, x, w.xs, st);
-  TG_OP_DISPATCH(km, (k_ru2<MU0><<<occ_grid(k_ru2<MU0>, wk), kBlock, 0, s>>>(g, km, x, w.tmp64, L.Wt, L.Wx, st)));
-  TG_OP_DISPATCH(kd, (k_ru3<MU0><<<occ_grid(k_ru3<MU0>, wk), kBlock, 0, s>>>(g, kd, b, w.tmp64, w.rs, L.Wt, L.Wx, st,
+  TG_OP_DISPATCH(km, (k_ru2<MU0><<<occ_grid(k_ru2<MU0>, wk), kBlock, 0, s>>>(g, km, x, w.tmp64, L.Wtq, L.Wxq, st)));
+  TG_OP_DISPATCH(kd, (k_ru3<MU0><<<occ_grid(k_ru3<MU0>, wk), kBlock, 0, s>>>(g, kd, b, w.tmp64, w.rs, L.Wtq, L.Wxq, st,
                                                                            log, red, c)));
 }
 
@@ -501,7 +490,7 @@ __global__ void __launch_bounds__(kBlock) k_gauge_action(int n, const double2* _
 
 template <bool MU0>
 __global__ void __launch_bounds__(kBlock, kStencilBlocksPerSM) k_md_action(Geo g, OpK<double> k, const double2* __restrict__ nz,
-                                                      const double2* __restrict__ Wt, const double2* __restrict__ Wx,
+                                                      const FxLink* __restrict__ Wt, const FxLink* __restrict__ Wx,
                                                       double* dst, Red red) {
   double a = 0;
   auto epi = [&](int, double2 o, double2 v) { a += v.x * o.x + v.y * o.y; };
@@ -520,8 +509,8 @@ void redot(cudaStream_t s, const Geo& g, const double2* u, const double2* v, dou
 void gauge_action(cudaStream_t s, const Geo& g, const double2* A, double fac, double* dst, const Red& red) {
   k_gauge_action<<<occ_grid(k_gauge_action, nblocks(g.V)), kBlock, 0, s>>>(g.V, A, fac, dst, red);
 }
-void md_action(cudaStream_t s, const Geo& g, const OpK<double>& kd, const double2* nz, const double2* Wt,
-               const double2* Wx, double* dst, const Red& red) {
+void md_action(cudaStream_t s, const Geo& g, const OpK<double>& kd, const double2* nz, const FxLink* Wt,
+               const FxLink* Wx, double* dst, const Red& red) {
   TG_OP_DISPATCH(kd, (k_md_action<MU0><<<occ_grid(k_md_action<MU0>, stencil_work(g)), kBlock, 0, s>>>(
                           g, kd, nz, Wt, Wx, dst, red)));
 }
@@ -672,9 +661,8 @@ int resident_grid_nocache(const void* kernel, int work) {
   return grid < work ? grid : (work > 0 ? work : 1);
 }
 
-void link_phase_fixed(cudaStream_t s, const Geo& g, int bc_t, int bc_x, const double2* A, double2* Wt, double2* Wx,
-                      float2* Wt32, float2* Wx32) {
-  k_link_phase<<<stream_grid(g.V), kBlock, 0, s>>>(g, bc_t, bc_x, A, LinkOut{Wt, Wx, Wt32, Wx32});
+void link_phase_fixed(cudaStream_t s, const Geo& g, int bc_t, int bc_x, const double2* A, const LinkOut& o) {
+  k_link_phase<<<stream_grid(g.V), kBlock, 0, s>>>(g, bc_t, bc_x, A, o);
 }
 
 void cg64_init_fixed(cudaStream_t s, const Geo& g, const double2* b, double2* x, const CgBufs64& w, CgState* st,
@@ -690,9 +678,9 @@ void cg64_iter_fixed(cudaStream_t s, const Geo& g, const OpK<double>& km, const 
   const double2* p_old = w.p[half];
   double2* p_new = w.p[half ^ 1];
   TG_OP_DISPATCH(km, (k_cg1<double, MU0><<<resident_grid_nocache((const void*)k_cg1<double, MU0>, wk), kBlock, 0,
-                                          s>>>(g, km, w.r, p_old, p_new, w.Mp, L.Wt, L.Wx, st, red)));
+                                          s>>>(g, km, w.r, p_old, p_new, w.Mp, L.Wtq, L.Wxq, st, red)));
   TG_OP_DISPATCH(kd, (k_cg2_64<MU0><<<resident_grid_nocache((const void*)k_cg2_64<MU0>, wk), kBlock, 0, s>>>(
-                          g, kd, w.Mp, p_new, x, w.r, L.Wt, L.Wx, st, nullptr, red, Cond{0, 0, 0})));
+                          g, kd, w.Mp, p_new, x, w.r, L.Wtq, L.Wxq, st, nullptr, red, Cond{0, 0, 0})));
 }
 
 // Stage waits of the staged kernels of this file that ran out (0 in a healthy run).

@@ -1,7 +1,7 @@
 // tg_launch.h -- host-side launch interface between tg_kernels.cu and tg_capi.cu.
 #pragma once
 
-#include "tg_internal.cuh"
+#include "tg_fixed.cuh"
 
 namespace tg {
 
@@ -28,20 +28,19 @@ struct Red {               // reduction scratch
   unsigned* counter;
 };
 
+// The links the operators read: fixed-point limbs (the FP64 operator,
+// tg_fixed.cuh) and FP32.
 struct Links {
-  const double2 *Wt, *Wx;
+  const FxLink *Wtq, *Wxq;
   const float2 *Wt32, *Wx32;
-  // W / m and 1 / m^2 for the unit-mass form of the FP64 CG (null when m = 0)
-  const double2 *Wt1 = nullptr, *Wx1 = nullptr;
-  double inv_m2 = 0;
 };
 
-// Where the link kernels write: W (FP64, FP32) and, when Wt1 is non-null, W / m
+// Where the link kernels write W: FP64 (the force and the dense matrix read it;
+// null: not written), FP32 and fixed-point limbs
 struct LinkOut {
   double2 *Wt, *Wx;
   float2 *Wt32, *Wx32;
-  double2 *Wt1 = nullptr, *Wx1 = nullptr;
-  double inv_m = 0;
+  FxLink *Wtq, *Wxq;
 };
 
 // link coefficients of A (both precisions)
@@ -51,7 +50,7 @@ void gauge_step(cudaStream_t s, const Geo& g, int bc_t, int bc_x, double2* A, co
                 int nadd, const LinkOut& o);
 // out = M in (dag = 0) or M^dag in (dag = 1); k must be the constants of that operator
 void dslash64(cudaStream_t s, const Geo& g, const OpK<double>& k, int dag, const double2* in, double2* out,
-              const double2* Wt, const double2* Wx);
+              const FxLink* Wt, const FxLink* Wx);
 void dslash32(cudaStream_t s, const Geo& g, const OpK<float>& k, int dag, const float2* in, float2* out,
               const float2* Wt, const float2* Wx);
 
@@ -76,8 +75,8 @@ void norm2(cudaStream_t s, const Geo& g, const double2* v, double* dst, int accu
 void redot(cudaStream_t s, const Geo& g, const double2* u, const double2* v, double* dst, int accumulate,
            const Red& red);
 void gauge_action(cudaStream_t s, const Geo& g, const double2* A, double fac, double* dst, const Red& red);
-void md_action(cudaStream_t s, const Geo& g, const OpK<double>& kd, const double2* nz, const double2* Wt,
-               const double2* Wx, double* dst, const Red& red);
+void md_action(cudaStream_t s, const Geo& g, const OpK<double>& kd, const double2* nz, const FxLink* Wt,
+               const FxLink* Wx, double* dst, const Red& red);
 
 // mom -= eps*F; flags bit0: gauge force first (gfac = eps*Nf/g), bit1: stochastic-term force last
 // (bc_t, bc_x: the lattice's boundary conditions, which the link coefficients carry)
@@ -131,8 +130,7 @@ constexpr int kPcgMaxGrid = 4096;
 struct Pcg64Args {
   Geo g;
   OpK<double> km, kd;
-  const double2 *Wt, *Wx;  // W, or W / m with inv_m2 = 1 / m^2 (unit-mass form); inv_m2 = 0: plain
-  double inv_m2;
+  const FxLink *Wt, *Wx;
   const double2* b;
   double2 *x, *r, *p0, *p1, *Mp;
   CgState* st;
@@ -149,7 +147,7 @@ struct PcgMxArgs {
   OpK<float> km32, kd32;
   OpK<double> km, kd;
   const float2 *Wt32, *Wx32;
-  const double2 *Wt, *Wx;
+  const FxLink *Wt, *Wx;
   const double2* b;
   double2 *x, *tmp;
   float2 *xs, *r, *p0, *p1, *Mp;
@@ -198,8 +196,7 @@ void dfma_peak(cudaStream_t s, int grid, int iters, double* sink);
 
 // Explicit-grid launchers used by the allocation-free CG entry point.
 int resident_grid_nocache(const void* kernel, int work);
-void link_phase_fixed(cudaStream_t s, const Geo& g, int bc_t, int bc_x, const double2* A, double2* Wt, double2* Wx,
-                      float2* Wt32, float2* Wx32);
+void link_phase_fixed(cudaStream_t s, const Geo& g, int bc_t, int bc_x, const double2* A, const LinkOut& o);
 void cg64_init_fixed(cudaStream_t s, const Geo& g, const double2* b, double2* x, const CgBufs64& w, CgState* st,
                      const Red& red, double rel_tol, double abs_tol2, int maxiter);
 void cg64_iter_fixed(cudaStream_t s, const Geo& g, const OpK<double>& km, const OpK<double>& kd, const Links& L,

@@ -29,7 +29,7 @@ constexpr size_t kVec32 = align_up(sizeof(float2) * kNoAllocMaxSites);
 constexpr size_t kPartials = align_up(sizeof(double) * (kNoAllocMaxSites / kBlock + 64));
 constexpr size_t kStateBytes = align_up(sizeof(CgState));
 constexpr size_t kCounterBytes = align_up(sizeof(unsigned));
-// Wt, Wx, r, p0, p1, Mp (FP64) + Wt32, Wx32 (FP32 links the link kernel also
+// Wtq, Wxq, r, p0, p1, Mp (16 bytes a site) + Wt32, Wx32 (FP32 links the link kernel also
 // writes) + block partials + solver state + reduction counter: about 1.9 MB.
 constexpr size_t kScratchBytes = 6 * kVec64 + 2 * kVec32 + kPartials + kStateBytes + kCounterBytes;
 
@@ -111,8 +111,8 @@ extern "C" int tg_cg_noalloc(const tg_lattice_params* p, const tg_cg_params* cp,
   // carve the scratch
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char* q = base + off; off += bytes; return q; };
-  double2* Wt = (double2*)take(kVec64);
-  double2* Wx = (double2*)take(kVec64);
+  FxLink* Wtq = (FxLink*)take(kVec64);
+  FxLink* Wxq = (FxLink*)take(kVec64);
   CgBufs64 w;
   w.r = (double2*)take(kVec64);
   w.p[0] = (double2*)take(kVec64);
@@ -126,11 +126,11 @@ extern "C" int tg_cg_noalloc(const tg_lattice_params* p, const tg_cg_params* cp,
   red.counter = (unsigned*)take(kCounterBytes);
 
   const double ep = exp(p->mu), em = exp(-p->mu);
-  OpK<double> km{p->m, ep, -em, p->mu == 0.0}, kd{p->m, -em, ep, p->mu == 0.0};
-  Links lk{Wt, Wx, Wt32, Wx32};
+  const OpK<double> km = make_opk(p->m, ep, -em, p->mu == 0.0), kd = make_opk(p->m, -em, ep, p->mu == 0.0);
+  const Links lk{Wtq, Wxq, Wt32, Wx32};
   // the reduction counter must start at 0; everything else is written before it is read
   if ((rc = ck(cudaMemsetAsync(red.counter, 0, sizeof(unsigned), s))) != TG_OK) return rc;
-  link_phase_fixed(s, g, p->bc_t, p->bc_x, (const double2*)A_dev, Wt, Wx, Wt32, Wx32);
+  link_phase_fixed(s, g, p->bc_t, p->bc_x, (const double2*)A_dev, LinkOut{nullptr, nullptr, Wt32, Wx32, Wtq, Wxq});
   cg64_init_fixed(s, g, (const double2*)b_dev, (double2*)x_dev, w, st, red, cp->rel_tol, cp->abs_tol2, cp->maxiter);
   if ((rc = ck(cudaGetLastError())) != TG_OK) return rc;
   CgState hs;

@@ -34,8 +34,7 @@ constexpr long long kBarrierSpinLimit = 1LL << 24;
 // Threads per block of the persistent kernels (512 / BS blocks per SM, 128
 // registers): one block of 512 threads per SM on lattices that fill the GPU --
 // fewer arrivals at each grid barrier -- and two of 256 on smaller ones, whose
-// march work (at least kMarchT rows per warp) would otherwise occupy too few
-// SMs.
+// rows would otherwise occupy too few SMs (pcg_launch).
 constexpr int pcg_min_blocks(int bs) { return 512 / bs; }
 
 // The number of grid barriers this block has passed in this launch (thread 0
@@ -305,9 +304,6 @@ __device__ __forceinline__ bool grid_total(double v, double* part, const GridBar
 }
 
 // What the iterations need after their sums.
-struct PcgStep64 {
-  double alpha, ax;  // x advances by ax p (alpha / m^2 in the unit-mass form)
-};
 struct PcgTail64 {
   double rn, beta;
   int status;  // -1: go on
@@ -349,9 +345,9 @@ __device__ __forceinline__ double stop_of(double rr0, double rel_tol, double abs
 }
 
 // ---------------------------------------------------------------------------
-// FP64: the iteration of k_cg1 + k_cg2_64 (unit-mass form when UNIT)
+// FP64: the iteration of k_cg1 + k_cg2_64
 // ---------------------------------------------------------------------------
-template <int BS, bool MU0, bool UNIT, bool ONE = false>
+template <int BS, bool MU0, bool ONE = false>
 __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
   if (threadIdx.x == 0) barrier_epoch() = 0;
   const Geo& g = a.g;
@@ -391,22 +387,18 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
       va = fma(o.x, o.x, va);
       va = fma(o.y, o.y, va);
     };
-    stencil_ld<double, 0, MU0, UNIT>(g, a.km, ld_a, a.Wt, a.Wx, epi_a);
-    PcgStep64 st;
-    if (!grid_total_then<BS>(va, partA, a.bar, [&](double pap) {
-          const double al = rr / pap;
-          return PcgStep64{al, UNIT ? al * a.inv_m2 : al};
-        }, st)) {
+    stencil_ld<double, 0, MU0>(g, a.km, ld_a, a.Wt, a.Wx, epi_a);
+    double alpha;
+    if (!grid_total_then<BS>(va, partA, a.bar, [&](double pap) { return rr / pap; }, alpha)) {
       status = TG_E_TIMEOUT;
       break;
     }
-    const double alpha = st.alpha, ax = st.ax;
     double vb = 0;
     auto ld_b = [&](int i) { return ldv<ONE>(a.Mp + i); };
     auto epi_b = [&](int s, double2 ap, double2) {
       double2 xv = ldv<ONE>(a.x + s), pv = ldv<ONE>(p_new + s), rv = ldv<ONE>(a.r + s);
-      xv.x += ax * pv.x;
-      xv.y += ax * pv.y;
+      xv.x += alpha * pv.x;
+      xv.y += alpha * pv.y;
       rv.x -= alpha * ap.x;
       rv.y -= alpha * ap.y;
       a.x[s] = xv;
@@ -414,7 +406,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
       vb = fma(rv.x, rv.x, vb);
       vb = fma(rv.y, rv.y, vb);
     };
-    stencil_ld<double, 1, MU0, UNIT>(g, a.kd, ld_b, a.Wt, a.Wx, epi_b);
+    stencil_ld<double, 1, MU0>(g, a.kd, ld_b, a.Wt, a.Wx, epi_b);
     PcgTail64 e;
     if (!grid_total_then<BS>(vb, partB, a.bar, [&](double rn) {
           PcgTail64 o{rn, rn / rr, -1};
@@ -865,13 +857,14 @@ template <class K, class Args> cudaError_t coop_launch(K kernel, int grid, int b
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
-// blocks of bs threads the stencil can use: at least kMarchT rows per warp
-int pcg_work(const Geo& g, int bs) {
-  return g.march ? ((g.nx >> 5) * ((g.nt + kMarchT - 1) / kMarchT) + bs / 32 - 1) / (bs / 32) : nblocks(g.V, bs);
+// Blocks of bs threads the stencil can use with at least `rows` rows of 32
+// columns per warp (column march) or one site per thread.
+int pcg_work(const Geo& g, int bs, int rows) {
+  return g.march ? ((g.nx >> 5) * ((g.nt + rows - 1) / rows) + bs / 32 - 1) / (bs / 32) : nblocks(g.V, bs);
 }
 
 int pcg_grid(const Geo& g, int resident, int bs) {
-  int grid = std::min(resident, pcg_work(g, bs));
+  int grid = std::min(resident, pcg_work(g, bs, 1));
   if (grid > kPcgMaxGrid) grid = kPcgMaxGrid;
   return grid > 0 ? grid : 1;
 }
@@ -887,33 +880,29 @@ int pcg_block_override() {
   return (v == 512 || v == 256) ? v : 0;
 }
 
-// the 512-thread kernel when its blocks fill every SM, else the 256-thread one;
-// a lattice whose work fits one 256-thread block runs the one-block instance
-// (k1; L1-cached loads, block totals kept on chip)
+// The 512-thread kernel when its blocks fill every SM with a row per warp,
+// else the 256-thread one.  A small lattice spreads to one row per warp: its
+// passes are bound by each warp's own latency, and more blocks cost the grid
+// sums little (us per iteration at four rows / one row per warp: FP64 64^2 16.5
+// / 11.0, 128^2 17.3 / 11.1, 256^2 17.4 / 13.5; mixed 64^2 8.5 / 7.7, 256^2 9.4 /
+// 8.6; two rows lie between; blocks of 128 and 64 threads gain 0.1-0.8 us
+// up to 128^2 and lose up to 8 us from 256^2 on).  A lattice whose work fits
+// one 256-thread block at one_rows rows per warp runs the one-block instance
+// (k1; L1-cached loads, block totals kept on chip): FP32 sums gain more from
+// that than from four blocks (32^2 4.7 against 6.9 us), FP64 less (12.2, 10.1).
 template <class K512, class K256, class K1, class Args>
-cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, cudaStream_t s, const Args& a) {
+cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, cudaStream_t s, const Args& a) {
   const int r512 = pcg_resident(k512, 512);
   const int force = pcg_block_override();
   if (force == 512) return coop_launch(k512, std::min(r512, kPcgMaxGrid), 512, s, a);
-  if (force == 0 && pcg_work(g, 512) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a);
-  const int grid = pcg_grid(g, pcg_resident(k256, 256), 256);
-  if (grid == 1) return coop_launch(k1, 1, 256, s, a);
-  return coop_launch(k256, grid, 256, s, a);
+  if (force == 0 && pcg_work(g, 512, 1) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a);
+  if (one_rows > 0 && pcg_work(g, 256, one_rows) == 1) return coop_launch(k1, 1, 256, s, a);
+  return coop_launch(k256, pcg_grid(g, pcg_resident(k256, 256), 256), 256, s, a);
 }
 
 cudaError_t pcg64(cudaStream_t s, bool mu0, Pcg64Args a) {
-  const bool unit = a.inv_m2 != 0.0;
-  if (mu0) {
-    if (unit)
-      return pcg_launch(a.g, k_pcg64<512, true, true>, k_pcg64<256, true, true>, k_pcg64<256, true, true, true>, s, a);
-    return pcg_launch(a.g, k_pcg64<512, true, false>, k_pcg64<256, true, false>, k_pcg64<256, true, false, true>, s,
-                      a);
-  }
-  if (unit)
-    return pcg_launch(a.g, k_pcg64<512, false, true>, k_pcg64<256, false, true>, k_pcg64<256, false, true, true>, s,
-                      a);
-  return pcg_launch(a.g, k_pcg64<512, false, false>, k_pcg64<256, false, false>, k_pcg64<256, false, false, true>, s,
-                    a);
+  if (mu0) return pcg_launch(a.g, k_pcg64<512, true>, k_pcg64<256, true>, k_pcg64<256, true, true>, 1, s, a);
+  return pcg_launch(a.g, k_pcg64<512, false>, k_pcg64<256, false>, k_pcg64<256, false, true>, 1, s, a);
 }
 
 cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, long long limit, int* status) {
@@ -930,14 +919,14 @@ cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, lon
 }
 
 cudaError_t pcgmx(cudaStream_t s, bool mu0, PcgMxArgs a) {
-  if (mu0) return pcg_launch(a.g, k_pcgmx<512, true>, k_pcgmx<256, true>, k_pcgmx<256, true, true>, s, a);
-  return pcg_launch(a.g, k_pcgmx<512, false>, k_pcgmx<256, false>, k_pcgmx<256, false, true>, s, a);
+  if (mu0) return pcg_launch(a.g, k_pcgmx<512, true>, k_pcgmx<256, true>, k_pcgmx<256, true, true>, kMarchT, s, a);
+  return pcg_launch(a.g, k_pcgmx<512, false>, k_pcgmx<256, false>, k_pcgmx<256, false, true>, kMarchT, s, a);
 }
 
 cudaError_t pcgcg(cudaStream_t s, bool mu0, PcgMxArgs a) {
   if (!a.g.march) return cudaErrorInvalidValue;
-  if (mu0) return pcg_launch(a.g, k_pcgcg<512, true>, k_pcgcg<256, true>, k_pcgcg<256, true>, s, a);
-  return pcg_launch(a.g, k_pcgcg<512, false>, k_pcgcg<256, false>, k_pcgcg<256, false>, s, a);
+  if (mu0) return pcg_launch(a.g, k_pcgcg<512, true>, k_pcgcg<256, true>, k_pcgcg<256, true>, 0, s, a);
+  return pcg_launch(a.g, k_pcgcg<512, false>, k_pcgcg<256, false>, k_pcgcg<256, false>, 0, s, a);
 }
 
 }  // namespace tg

@@ -11,11 +11,11 @@
 
 namespace tg {
 
-// One row t of a warp's march: the operator at the 32 sites (t, x0 + lane)
+// One row t of a warp's FP32 march: the operator at the 32 sites (t, x0 + lane)
 // from psi(t-1) = pm, psi(t) = pc, psi(t+1) = pp and the links, with the
 // operand across the warp's edge pe (used by lanes 0 and 31) and the x link
 // entering column x0 we (used by lane 0).  Rotates pm, pc, wtm for row t+1.
-template <typename R, int DAG, bool MU0, bool UNIT, class Epi>
+template <typename R, int DAG, bool MU0, class Epi>
 __device__ __forceinline__ void march_row(const OpK<R>& k, int s, int lane, C2<R>& pm, C2<R>& pc, C2<R>& wtm,
                                           C2<R> pp, C2<R> wt, C2<R> wx, C2<R> pe, C2<R> we, Epi& epi) {
   C2<R> pr = shfl_down1<R>(pc);
@@ -26,7 +26,7 @@ __device__ __forceinline__ void march_row(const OpK<R>& k, int s, int lane, C2<R
     pl = pe;
     wl = we;
   }
-  epi(s, dslash_vals<R, DAG, MU0, UNIT>(k, pc, pp, pm, pr, pl, wt, wtm, wx, wl), pc);
+  epi(s, dslash_vals<R, DAG, MU0>(k, pc, pp, pm, pr, pl, wt, wtm, wx, wl), pc);
   pm = pc;
   pc = pp;
   wtm = wt;
@@ -57,10 +57,15 @@ __device__ __forceinline__ void edge_operands(const Geo& g, Ld& ld, const C2<R>*
 // x0+31, lane = column.  ld(i) yields the operand at site i (a plain load, or a
 // vector recombined on the fly); epi(s, out(s), operand(s)) consumes each
 // site's result.  psi(t-1), psi(t) and Wt(t-1) stay in registers from row to
-// row; x neighbours come from warp shuffles.
-template <typename R, int DAG, bool MU0, bool UNIT = false, class Ld, class Epi>
-__device__ __forceinline__ void march_segment(const Geo& g, const OpK<R>& k, Ld& ld, const C2<R>* __restrict__ Wt,
-                                              const C2<R>* __restrict__ Wx, int xw, int ta, int tb, Epi& epi) {
+// row; x neighbours come from warp shuffles.  Every load of a chunk of rows is
+// issued before its first result is stored: the epilogue's stores may alias
+// the operands as far as the compiler knows, and would otherwise hold each
+// row's loads behind the previous row's stores, one memory latency per row.
+template <int DAG, bool MU0, class Ld, class Epi>
+__device__ __forceinline__ void march_segment32(const Geo& g, const OpK<float>& k, Ld& ld,
+                                                const float2* __restrict__ Wt, const float2* __restrict__ Wx, int xw,
+                                                int ta, int tb, Epi& epi) {
+  using R = float;
   const int nx = g.nx;
   const int lane = threadIdx.x & 31;
   const int x0 = xw << 5;
@@ -71,44 +76,131 @@ __device__ __forceinline__ void march_segment(const Geo& g, const OpK<R>& k, Ld&
   C2<R> pm = ld(tm * nx + x);
   C2<R> wtm = Wt[tm * nx + x];
   C2<R> pc = ld(ta * nx + x);
-  auto row = [&](int t, C2<R> pe, C2<R> we) {
-    const int tp = (t + 1 == g.nt) ? 0 : t + 1;
-    const int s = t * nx + x;
-    march_row<R, DAG, MU0, UNIT>(k, s, lane, pm, pc, wtm, ld(tp * nx + x), Wt[s], Wx[s], pe, we, epi);
-  };
   int t = ta;
   for (; t + kMarchT <= tb; t += kMarchT) {
     C2<R> ep, ew;
     edge_operands<R>(g, ld, Wx, t, xle, xre, lane, ep, ew);
-    if constexpr (sizeof(R) == 4) {
-      // FP32 (memory- or latency-bound): every load of the chunk is issued
-      // before its first result is stored.  The epilogue's stores may alias the
-      // operands as far as the compiler knows, and would otherwise hold each
-      // row's loads behind the previous row's stores, one memory latency per
-      // row.  (The FP64 march is bound by the FP64 pipe and keeps its
-      // registers.)
-      C2<R> pp[kMarchT], wt[kMarchT], wx[kMarchT];
+    C2<R> pp[kMarchT], wt[kMarchT], wx[kMarchT];
 #pragma unroll
-      for (int i = 0; i < kMarchT; i++) {
-        const int tt = t + i;
+    for (int i = 0; i < kMarchT; i++) {
+      const int tt = t + i;
+      const int tp = (tt + 1 == g.nt) ? 0 : tt + 1;
+      pp[i] = ld(tp * nx + x);
+      wt[i] = Wt[tt * nx + x];
+      wx[i] = Wx[tt * nx + x];
+    }
+#pragma unroll
+    for (int i = 0; i < kMarchT; i++)
+      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, pm, pc, wtm, pp[i], wt[i], wx[i],
+                             shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
+  }
+  for (; t < tb; t++) {  // the last rows of the segment: lanes 0 and 31 fetch their own
+    const int xe = (lane == 31) ? xre : xle;
+    const int tp = (t + 1 == g.nt) ? 0 : t + 1;
+    const int s = t * nx + x;
+    march_row<R, DAG, MU0>(k, s, lane, pm, pc, wtm, ld(tp * nx + x), Wt[s], Wx[s], ld(t * nx + xe), Wx[t * nx + xle],
+                           epi);
+  }
+}
+
+// Warp shuffles of block-floating operands and links (tg_fixed.cuh).
+__device__ __forceinline__ FxC shfl_fx(const FxC& v, int src) {
+  FxC o;
+  o.re = __shfl_sync(0xffffffffu, v.re, src);
+  o.im = __shfl_sync(0xffffffffu, v.im, src);
+  o.e = __shfl_sync(0xffffffffu, v.e, src);
+  return o;
+}
+__device__ __forceinline__ FxLink shfl_lk(FxLink w, int src) {
+  return make_int4(__shfl_sync(0xffffffffu, w.x, src), __shfl_sync(0xffffffffu, w.y, src),
+                   __shfl_sync(0xffffffffu, w.z, src), __shfl_sync(0xffffffffu, w.w, src));
+}
+__device__ __forceinline__ FxC sel_fx(bool c, const FxC& a, const FxC& b) {
+  return FxC{c ? a.re : b.re, c ? a.im : b.im, c ? a.e : b.e};
+}
+
+// Rows whose loads are in flight together in the FP64 march.
+constexpr int kChunk64 = 2;
+
+// The FP64 march: march_segment32 with the operator on the integer pipes.  Each
+// loaded operand is converted to block floating point once and shared with the
+// neighbouring columns and rows in that form.
+template <int DAG, bool MU0, class Ld, class Epi>
+__device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>& k, Ld& ld,
+                                                const FxLink* __restrict__ Wt, const FxLink* __restrict__ Wx, int xw,
+                                                int ta, int tb, Epi& epi) {
+  static_assert(kMarchT % kChunk64 == 0, "a chunk's edge operands are fetched kMarchT rows at a time");
+  const int nx = g.nx;
+  const int lane = threadIdx.x & 31;
+  const int x0 = xw << 5;
+  const int x = x0 + lane;
+  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
+  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;
+  const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
+  FxC pm = to_fx(ld(tm * nx + x));
+  FxLink wtm = Wt[tm * nx + x];
+  double2 own = ld(ta * nx + x);
+  FxC pc = to_fx(own);
+  // row t: in(t+1) = pp, in beyond the warp's edge pe (lanes 0 and 31), the x link entering x0 we (lane 0)
+  auto row = [&](int t, double2 pp, FxLink wt, FxLink wx, const FxC& pe, FxLink we) {
+    const int s = t * nx + x;
+    const FxC pr = sel_fx(lane == 31, pe, shfl_fx(pc, lane + 1));
+    const FxC pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
+    FxLink wl = shfl_lk(wx, lane - 1);
+    if (lane == 0) wl = we;
+    const FxC pn = to_fx(pp);
+    double2 o;
+    if (!fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o)) {
+      const Nbr n = neighbours(g, s, t, x);
+      o = dslash_vals<double, DAG, MU0>(k, ld(s), ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), fx_link_value(wt),
+                                        fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
+    }
+    epi(s, o, own);
+    pm = pc;
+    pc = pn;
+    own = pp;
+    wtm = wt;
+  };
+  int t = ta;
+  for (; t + kMarchT <= tb; t += kMarchT) {
+    // lane i < kMarchT: left of x0 in row t+i (and the link entering x0); lane kMarchT+i: right of x0+31
+    double2 ep = make_double2(0, 0);
+    FxLink ew = make_int4(0, 0, 0, 0);
+    if (lane < 2 * kMarchT) {
+      const int rr = t + (lane < kMarchT ? lane : lane - kMarchT);
+      ep = ld(rr * nx + (lane < kMarchT ? xle : xre));
+      if (lane < kMarchT) ew = Wx[rr * nx + xle];
+    }
+    const FxC ef = to_fx(ep);
+#pragma unroll
+    for (int h = 0; h < kMarchT; h += kChunk64) {
+      double2 pp[kChunk64];
+      FxLink wt[kChunk64], wx[kChunk64];
+#pragma unroll
+      for (int i = 0; i < kChunk64; i++) {
+        const int tt = t + h + i;
         const int tp = (tt + 1 == g.nt) ? 0 : tt + 1;
         pp[i] = ld(tp * nx + x);
         wt[i] = Wt[tt * nx + x];
         wx[i] = Wx[tt * nx + x];
       }
 #pragma unroll
-      for (int i = 0; i < kMarchT; i++)
-        march_row<R, DAG, MU0, UNIT>(k, (t + i) * nx + x, lane, pm, pc, wtm, pp[i], wt[i], wx[i],
-                                     shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
-    } else {
-#pragma unroll
-      for (int i = 0; i < kMarchT; i++) row(t + i, shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i));
+      for (int i = 0; i < kChunk64; i++)
+        row(t + h + i, pp[i], wt[i], wx[i], shfl_fx(ef, (lane == 31) ? kMarchT + h + i : h + i), shfl_lk(ew, h + i));
     }
   }
-  for (; t < tb; t++) {  // the last rows of the segment: lanes 0 and 31 fetch their own
-    const int xe = (lane == 31) ? xre : xle;
-    row(t, ld(t * nx + xe), Wx[t * nx + xle]);
+  for (; t < tb; t++) {
+    const int tp = (t + 1 == g.nt) ? 0 : t + 1;
+    row(t, ld(tp * nx + x), Wt[t * nx + x], Wx[t * nx + x], to_fx(ld(t * nx + ((lane == 31) ? xre : xle))),
+        Wx[t * nx + xle]);
   }
+}
+
+template <typename R, int DAG, bool MU0, class Ld, class Epi>
+__device__ __forceinline__ void march_segment(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
+                                              const Lk<R>* __restrict__ Wx, int xw, int ta, int tb, Epi& epi) {
+  if constexpr (sizeof(R) == 4) march_segment32<DAG, MU0>(g, k, ld, Wt, Wx, xw, ta, tb, epi);
+  else march_segment64<DAG, MU0>(g, k, ld, Wt, Wx, xw, ta, tb, epi);
 }
 
 // The (strip, t) rows of the lattice in strip-major order, split into one
@@ -133,29 +225,27 @@ template <class F> __device__ __forceinline__ void for_warp_rows(const Geo& g, F
 
 // Apply the operator to every site and hand each result to epi: column march
 // where the lattice allows it, else one site per thread.
-template <typename R, int DAG, bool MU0, bool UNIT = false, class Ld, class Epi>
-__device__ __forceinline__ void stencil_ld(const Geo& g, const OpK<R>& k, Ld& ld, const C2<R>* __restrict__ Wt,
-                                           const C2<R>* __restrict__ Wx, Epi& epi) {
+template <typename R, int DAG, bool MU0, class Ld, class Epi>
+__device__ __forceinline__ void stencil_ld(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
+                                           const Lk<R>* __restrict__ Wx, Epi& epi) {
   if (g.march) {
-    for_warp_rows(g, [&](int xw, int ta, int tb) { march_segment<R, DAG, MU0, UNIT>(g, k, ld, Wt, Wx, xw, ta, tb, epi); });
+    for_warp_rows(g, [&](int xw, int ta, int tb) { march_segment<R, DAG, MU0>(g, k, ld, Wt, Wx, xw, ta, tb, epi); });
   } else {
     TG_SITES(s, g.V) {
       int t, x;
       site_tx(g, s, t, x);
-      const Nbr n = neighbours(g, s, t, x);
-      const C2<R> pc = ld(s);
-      epi(s, dslash_vals<R, DAG, MU0, UNIT>(k, pc, ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), Wt[s], Wt[n.tm], Wx[s],
-                                            Wx[n.xm]),
-          pc);
+      C2<R> own;
+      const C2<R> o = dslash_ld<R, DAG, MU0>(g, k, ld, Wt, Wx, s, t, x, own);
+      epi(s, o, own);
     }
   }
 }
 
-template <typename R, int DAG, bool MU0, bool UNIT = false, class Epi>
+template <typename R, int DAG, bool MU0, class Epi>
 __device__ __forceinline__ void stencil_all(const Geo& g, const OpK<R>& k, const C2<R>* __restrict__ in,
-                                            const C2<R>* __restrict__ Wt, const C2<R>* __restrict__ Wx, Epi& epi) {
+                                            const Lk<R>* __restrict__ Wt, const Lk<R>* __restrict__ Wx, Epi& epi) {
   auto ld = [&](int i) { return in[i]; };
-  stencil_ld<R, DAG, MU0, UNIT>(g, k, ld, Wt, Wx, epi);
+  stencil_ld<R, DAG, MU0>(g, k, ld, Wt, Wx, epi);
 }
 
 // The operator over one small lattice run by a team of thread blocks (the
@@ -165,8 +255,8 @@ __device__ __forceinline__ void stencil_all(const Geo& g, const OpK<R>& k, const
 // splits them over a grid; lattices whose nx is not a multiple of 32 go one
 // site per thread.
 template <class T, typename R, int DAG, bool MU0, class Ld, class Epi>
-__device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& ld, const C2<R>* __restrict__ Wt,
-                                             const C2<R>* __restrict__ Wx, Epi& epi) {
+__device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
+                                             const Lk<R>* __restrict__ Wx, Epi& epi) {
   const int wpb = blockDim.x >> 5;
   if ((g.nx & 31) == 0) {
     const int nw = T::nblocks() * wpb, w = T::rank() * wpb + (threadIdx.x >> 5);
@@ -184,17 +274,17 @@ __device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& 
     for (int s = T::rank() * (int)blockDim.x + (int)threadIdx.x; s < g.V; s += T::nblocks() * (int)blockDim.x) {
       int t, x;
       site_tx(g, s, t, x);
-      const Nbr n = neighbours(g, s, t, x);
-      const C2<R> pc = ld(s);
-      epi(s, dslash_vals<R, DAG, MU0>(k, pc, ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), Wt[s], Wt[n.tm], Wx[s], Wx[n.xm]),
-          pc);
+      C2<R> own;
+      const C2<R> o = dslash_ld<R, DAG, MU0>(g, k, ld, Wt, Wx, s, t, x, own);
+      epi(s, o, own);
     }
   }
 }
 
-// Blocks of work of a stencil kernel (march: at least kMarchT rows per warp).
+// Blocks of work of a stencil kernel (march: at least one row per warp, so that
+// a small lattice spreads over more SMs).
 inline int stencil_work(const Geo& g) {
-  return g.march ? ((g.nx >> 5) * ((g.nt + kMarchT - 1) / kMarchT) + kBlock / 32 - 1) / (kBlock / 32) : nblocks(g.V);
+  return g.march ? ((g.nx >> 5) * g.nt + kBlock / 32 - 1) / (kBlock / 32) : nblocks(g.V);
 }
 
 // ---------------------------------------------------------------------------
@@ -288,7 +378,7 @@ __device__ __forceinline__ void stage_wait(unsigned long long* bar, unsigned par
   if ((threadIdx.x & 31) == 0) atomicAdd(&g_stage_faults, 1u);
 }
 
-template <typename R, int DAG, bool MU0, bool UNIT, class Src, class Epi>
+template <typename R, int DAG, bool MU0, class Src, class Epi>
 __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>& k, const Src& src,
                                                      const C2<R>* __restrict__ Wt, const C2<R>* __restrict__ Wx,
                                                      int xw, int ta, int tb, Epi& epi, unsigned char* stage,
@@ -340,7 +430,7 @@ __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>&
       C2<R> v[Src::n];
 #pragma unroll
       for (int j = 0; j < Src::n; j++) v[j] = sv[(j * kMarchT + i) * 32 + lane];
-      march_row<R, DAG, MU0, UNIT>(k, (t + i) * nx + x, lane, pm, pc, wtm, src.combine(v),
+      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, pm, pc, wtm, src.combine(v),
                                    sv[(Src::n * kMarchT + i) * 32 + lane], sv[((Src::n + 1) * kMarchT + i) * 32 + lane],
                                    shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
     }
@@ -354,7 +444,7 @@ __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>&
     const int tp = (t + 1 == g.nt) ? 0 : t + 1;
     const int s = t * nx + x;
     const int xe = (lane == 31) ? xre : xle;
-    march_row<R, DAG, MU0, UNIT>(k, s, lane, pm, pc, wtm, src(tp * nx + x), Wt[s], Wx[s], src(t * nx + xe),
+    march_row<R, DAG, MU0>(k, s, lane, pm, pc, wtm, src(tp * nx + x), Wt[s], Wx[s], src(t * nx + xe),
                                  Wx[t * nx + xle], epi);
   }
 }
@@ -362,12 +452,12 @@ __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>&
 // stencil_ld with the operand from Src, staged through shared memory on
 // marching lattices.  The kernel must be launched with
 // staged_smem_bytes<R, Src::n>() of dynamic shared memory.
-template <typename R, int DAG, bool MU0, bool UNIT, class Src, class Epi>
+template <typename R, int DAG, bool MU0, class Src, class Epi>
 __device__ __forceinline__ void stencil_staged(const Geo& g, const OpK<R>& k, const Src& src,
                                                const C2<R>* __restrict__ Wt, const C2<R>* __restrict__ Wx, Epi& epi) {
   if (!g.march) {
     Src ld = src;
-    stencil_ld<R, DAG, MU0, UNIT>(g, k, ld, Wt, Wx, epi);
+    stencil_ld<R, DAG, MU0>(g, k, ld, Wt, Wx, epi);
     return;
   }
   extern __shared__ __align__(128) unsigned char tg_dyn_smem[];
@@ -383,7 +473,7 @@ __device__ __forceinline__ void stencil_staged(const Geo& g, const OpK<R>& k, co
   __syncwarp();
   unsigned phases = 0;
   for_warp_rows(g, [&](int xw, int ta, int tb) {
-    march_segment_staged<R, DAG, MU0, UNIT>(g, k, src, Wt, Wx, xw, ta, tb, epi, stage, bars, phases);
+    march_segment_staged<R, DAG, MU0>(g, k, src, Wt, Wx, xw, ta, tb, epi, stage, bars, phases);
   });
 }
 
