@@ -75,7 +75,9 @@ typedef struct {
 #define TG_SOLVER_DEFAULT 0     /* the faster of the two on this library's measurements:
                                    persistent (TG_SOLVER=launches|persistent overrides)    */
 #define TG_SOLVER_LAUNCHES 1    /* two kernel launches per iteration (graph WHILE node)       */
-#define TG_SOLVER_PERSISTENT 2  /* one cooperative launch per solve, grid barriers inside     */
+#define TG_SOLVER_PERSISTENT 2  /* one launch per solve: a cooperative grid with barriers inside, or,
+                                   for small lattices, one thread-block cluster that keeps the
+                                   solve in its shared memory                              */
 
 typedef struct {
   int iterations;       /* CG iterations (each = one M and one M^dagger apply) */

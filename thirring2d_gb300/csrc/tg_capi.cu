@@ -280,7 +280,8 @@ bool use_single_reduction(const tg_lattice* L) {
 int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const double2* b, double2* x, int log_index) {
   const Links lk = links(L);
   const GridBar bar{L->bar, reinterpret_cast<unsigned long long*>(L->bar + 2)};
-  TG_CK(cudaMemsetAsync(L->bar, 0, kBarWords * sizeof(unsigned), s));
+  const CcgShape small = ccg_shape(L->g, cp.precision == TG_PREC_MIXED);
+  if (small.blocks == 0) TG_CK(cudaMemsetAsync(L->bar, 0, kBarWords * sizeof(unsigned), s));
   cudaError_t e;
   if (cp.precision == TG_PREC_MIXED) {
     PcgMxArgs a{};
@@ -310,7 +311,9 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.abs_tol2 = cp.abs_tol2;
     a.maxiter = cp.maxiter;
     a.ru_interval = cp.ru_interval;
-    if (use_single_reduction(L)) {
+    if (small.blocks > 0) {
+      e = ccgmx(s, L->P.mu == 0.0, a, small);
+    } else if (use_single_reduction(L)) {
       a.w0 = L->wmx.Mps;
       a.s0 = L->wmx.ss;
       e = pcgcg(s, L->P.mu == 0.0, a);
@@ -338,7 +341,7 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.rel_tol = cp.rel_tol;
     a.abs_tol2 = cp.abs_tol2;
     a.maxiter = cp.maxiter;
-    e = pcg64(s, L->P.mu == 0.0, a);
+    e = small.blocks > 0 ? ccg64(s, L->P.mu == 0.0, a, small) : pcg64(s, L->P.mu == 0.0, a);
   }
   if (e != cudaSuccess) return fail(TG_E_CUDA, std::string("persistent CG launch: ") + cudaGetErrorString(e));
   return TG_OK;

@@ -120,6 +120,21 @@ TG_HD FxC to_fx(double2 v) {
   return f;
 }
 
+// The operand as FP64 again, for the FP64 form where only the block-floating
+// one was kept: operands that are not finite give NaN, zero and denormal ones 0.
+TG_HD double2 fx_value(const FxC& f) {
+  double2 v;
+  if (f.e == 0) {
+    v.x = v.y = 0.0;
+  } else if (f.e == 2047) {
+    v.x = v.y = dbl_of(0x7ff8000000000000ull);
+  } else {
+    v.x = ldexp((double)f.re, f.e - 1082);
+    v.y = ldexp((double)f.im, f.e - 1082);
+  }
+  return v;
+}
+
 // W (|parts| <= 1/2) at the scale 2^60, rounded to even multiples; a part that
 // is not finite sets bit 0 of the real low limb.
 TG_HD FxLink to_fx_link(double2 w) {

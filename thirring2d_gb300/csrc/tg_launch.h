@@ -168,6 +168,15 @@ cudaError_t pcgmx(cudaStream_t s, bool mu0, PcgMxArgs a);
 // arguments and results): per iteration an elementwise update and one pass of
 // the fused M^dag M march (k_pcgcg)
 cudaError_t pcgcg(cudaStream_t s, bool mu0, PcgMxArgs a);
+// The same solves on one thread-block cluster, in its shared memory
+// (tg_cluster_cg.cu), for the lattices it takes: ccg_shape gives the cluster's
+// blocks and threads per block, 0 blocks where the grid solvers are to be used.
+struct CcgShape {
+  int blocks, threads;
+};
+CcgShape ccg_shape(const Geo& g, bool mixed);
+cudaError_t ccg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& sh);
+cudaError_t ccgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh);
 // one grid barrier (4 blocks, cooperative) that also waits for `phantom` absent
 // blocks, giving up after `limit` polls: *status = TG_OK or TG_E_TIMEOUT
 cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, long long limit, int* status);
