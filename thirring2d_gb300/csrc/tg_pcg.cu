@@ -25,6 +25,7 @@
 #include <unordered_map>
 
 #include "tg_fused.cuh"
+#include "tg_scalar.cuh"
 
 namespace tg {
 
@@ -52,18 +53,27 @@ __device__ __forceinline__ unsigned& barrier_epoch() {
 //
 // warp0_grid_wait is the barrier's core, run by warp 0 after a block barrier
 // that follows the block's writes; it returns false in every lane if the wait
-// gave up.  The arrival (lane 0) is a release and each poll an acquire at GPU
+// gave up.  prep() runs in lane 0 between the arrival and the first poll: the
+// reciprocals that the scalars after the sum need (an FP64 division has a
+// latency of 574 clocks) are computed there, while the other blocks arrive.  The arrival (lane 0) is a release and each poll an acquire at GPU
 // scope: the block's writes, ordered before lane 0 by that block barrier, are
 // visible to every block that sees the count complete.  The warp barrier hands
 // the acquire on to the other lanes, and the caller's next block barrier to the
 // other warps.  Measured 0.35 us faster per barrier than a fence, a relaxed
 // atomic and a second fence, with the same 152 blocks.  A one-block grid (small
 // lattices) needs no arrival: its block barrier orders its global writes.
-__device__ __forceinline__ bool warp0_grid_wait(const GridBar& b, unsigned nblocks, long long limit) {
+struct NoPrep {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <class Prep = NoPrep>
+__device__ __forceinline__ bool warp0_grid_wait(const GridBar& b, unsigned nblocks, long long limit, Prep prep = {}) {
   int ok = 1;
-  if (nblocks > 1 && (threadIdx.x & 31) == 0) {
+  if (nblocks == 1) {
+    if ((threadIdx.x & 31) == 0) prep();
+  } else if ((threadIdx.x & 31) == 0) {
     const unsigned target = (barrier_epoch() += 1) * nblocks;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(b.count) : "memory");
+    prep();
     long long spins = 0;
     while (true) {
       unsigned c;
@@ -153,8 +163,9 @@ __device__ __forceinline__ void warp_read_partials(const double* part, double (&
 // retires two per SM per clock.
 // Two block barriers in all: one after the warps' sums (it also orders the
 // block's writes before the arrival), one to hand the result to the block.
-template <int BS, typename T, class F>
-__device__ __forceinline__ bool grid_total_then(T v, double* part, const GridBar& bar, F f, decltype(f(0.0))& out) {
+template <int BS, typename T, class F, class Prep = NoPrep>
+__device__ __forceinline__ bool grid_total_then(T v, double* part, const GridBar& bar, F f, decltype(f(0.0))& out,
+                                                Prep prep = {}) {
   using S = decltype(f(0.0));
   __shared__ T sh[BS / 32];
   __shared__ S s_out;
@@ -168,12 +179,13 @@ __device__ __forceinline__ bool grid_total_then(T v, double* part, const GridBar
     b = warp_sum(b);
     if (gridDim.x == 1) {  // a one-block grid: its total is the grid's, no round trip through memory
       if (lane == 0) {
+        prep();
         s_out = f((double)b);
         s_ok = 1;
       }
     } else {
       if (lane == 0) part[blockIdx.x] = (double)b;
-      const bool ok = warp0_grid_wait(bar, gridDim.x, kBarrierSpinLimit);
+      const bool ok = warp0_grid_wait(bar, gridDim.x, kBarrierSpinLimit, prep);
       if (ok) {
         double s[1];
         warp_read_partials<1>(part, s);
@@ -235,11 +247,11 @@ constexpr unsigned kFxMaxGrid = 511;
 constexpr double kFxBlockCap = 137438953472.0;  // 2^37
 constexpr int kFxMinBits = 26;                   // the exact path below 2^26 per block
 
-template <int BS, class F>
+template <int BS, class F, class Prep = NoPrep>
 __device__ __forceinline__ bool grid_total_fx(float v, double* part, const GridBar& bar, FxSum& fx, F f,
-                                              decltype(f(0.0))& out) {
+                                              decltype(f(0.0))& out, Prep prep = {}) {
   using S = decltype(f(0.0));
-  if (gridDim.x == 1 || gridDim.x > kFxMaxGrid) return grid_total_then<BS>(v, part, bar, f, out);
+  if (gridDim.x == 1 || gridDim.x > kFxMaxGrid) return grid_total_then<BS>(v, part, bar, f, out, prep);
   __shared__ float sh[BS / 32];
   __shared__ S s_out;
   __shared__ int s_ok;
@@ -260,6 +272,7 @@ __device__ __forceinline__ bool grid_total_fx(float v, double* part, const GridB
       const unsigned long long add =
           (fits ? ((unsigned long long)__double2ll_rn(sc) << kFxSumShift) : (1ull << kFxOvfShift)) | 1ull;
       asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(fx.word), "l"(add) : "memory");
+      prep();
       unsigned long long cur, d;
       long long spins = 0;
       while (true) {
@@ -347,8 +360,18 @@ __device__ __forceinline__ double stop_of(double rr0, double rel_tol, double abs
 // ---------------------------------------------------------------------------
 // FP64: the iteration of k_cg1 + k_cg2_64
 // ---------------------------------------------------------------------------
+// Rows in flight per warp in the FP64 march, and the shared memory they take
+// (12.8 KB a warp, 205 KB a 512-thread block).  The prefetched march against one
+// with two rows' loads in registers, us per iteration: 1024^2 53.2 / 58.7, 512^2
+// 21.2 / 21.2.  16 warps per SM beat 12 (61.5 at 1024^2), 18 and 20 (62.5, 58.5: 88 B of
+// spills); two rows per step, interleaved, gave 56.4.
+constexpr int kRingRows = 4;
+constexpr int kRingWarp = ring_bytes<kRingRows, 1, 3>() > ring_bytes<kRingRows, 2, 0>()
+                              ? ring_bytes<kRingRows, 1, 3>() : ring_bytes<kRingRows, 2, 0>();
 template <int BS, bool MU0, bool ONE = false>
 __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
+  extern __shared__ __align__(16) unsigned char pcg_ring[];
+  unsigned char* const ring = pcg_ring + (threadIdx.x >> 5) * kRingWarp;
   if (threadIdx.x == 0) barrier_epoch() = 0;
   const Geo& g = a.g;
   double* partA = a.part;
@@ -366,7 +389,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
   int status = -1, iter = 0;
   if (!grid_total<BS>(v, partB, a.bar, rr)) status = TG_E_TIMEOUT;
   const double rr0 = rr;
-  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2);
+  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2), limit = 1e10 * rr0;
   if (status < 0) {
     if (isnan(rr)) status = TG_E_NAN;
     else if (!(rr >= stop) || rr == 0.0) status = TG_OK;  // hmc.c:359-361
@@ -387,16 +410,24 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
       va = fma(o.x, o.x, va);
       va = fma(o.y, o.y, va);
     };
-    stencil_ld<double, 0, MU0>(g, a.km, ld_a, a.Wt, a.Wx, epi_a);
+    if (!ONE && g.march) {
+      const double2* const src[2] = {a.r, p_old};
+      auto comb = [&](const double2* v) { return make_double2(fma(beta, v[1].x, v[0].x), fma(beta, v[1].y, v[0].y)); };
+      auto epi = [&](int s, double2 o, double2 pc, const double2*) { epi_a(s, o, pc); };
+      for_warp_rows(g, [&](int xw, int ta, int tb) {
+        march_ring64<0, MU0, kRingRows, 2, 0>(g, a.km, src, nullptr, comb, a.Wt, a.Wx, xw, ta, tb, epi, ring);
+      });
+    } else {
+      stencil_ld<double, 0, MU0>(g, a.km, ld_a, a.Wt, a.Wx, epi_a);
+    }
     double alpha;
-    if (!grid_total_then<BS>(va, partA, a.bar, [&](double pap) { return rr / pap; }, alpha)) {
+    if (!grid_total_then<BS>(va, partA, a.bar, [&](double pap) { return div_newton(rr, pap); }, alpha)) {
       status = TG_E_TIMEOUT;
       break;
     }
     double vb = 0;
     auto ld_b = [&](int i) { return ldv<ONE>(a.Mp + i); };
-    auto epi_b = [&](int s, double2 ap, double2) {
-      double2 xv = ldv<ONE>(a.x + s), pv = ldv<ONE>(p_new + s), rv = ldv<ONE>(a.r + s);
+    auto update = [&](int s, double2 ap, double2 xv, double2 pv, double2 rv) {
       xv.x += alpha * pv.x;
       xv.y += alpha * pv.y;
       rv.x -= alpha * ap.x;
@@ -406,16 +437,30 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
       vb = fma(rv.x, rv.x, vb);
       vb = fma(rv.y, rv.y, vb);
     };
-    stencil_ld<double, 1, MU0>(g, a.kd, ld_b, a.Wt, a.Wx, epi_b);
+    if (!ONE && g.march) {
+      const double2* const src[1] = {a.Mp};
+      const double2* const ext[3] = {a.x, p_new, a.r};
+      auto comb = [](const double2* v) { return v[0]; };
+      auto epi = [&](int s, double2 ap, double2, const double2* e) { update(s, ap, e[0], e[32], e[64]); };
+      for_warp_rows(g, [&](int xw, int ta, int tb) {
+        march_ring64<1, MU0, kRingRows, 1, 3>(g, a.kd, src, ext, comb, a.Wt, a.Wx, xw, ta, tb, epi, ring);
+      });
+    } else {
+      auto epi = [&](int s, double2 ap, double2) {
+        update(s, ap, ldv<ONE>(a.x + s), ldv<ONE>(p_new + s), ldv<ONE>(a.r + s));
+      };
+      stencil_ld<double, 1, MU0>(g, a.kd, ld_b, a.Wt, a.Wx, epi);
+    }
     PcgTail64 e;
+    double inv_rr = 0;  // thread 0's
     if (!grid_total_then<BS>(vb, partB, a.bar, [&](double rn) {
-          PcgTail64 o{rn, rn / rr, -1};
+          PcgTail64 o{rn, rn * inv_rr, -1};
           if (isnan(rn)) o.status = TG_E_NAN;
-          else if (rn < stop) o.status = TG_OK;                // hmc.c:381
-          else if (rn / rr0 > 1e10) o.status = TG_E_DIVERGED;  // hmc.c:383-386
+          else if (rn < stop) o.status = TG_OK;           // hmc.c:381
+          else if (rn > limit) o.status = TG_E_DIVERGED;  // hmc.c:383-386
           else if (iter + 1 >= a.maxiter) o.status = TG_E_NOCONV;
           return o;
-        }, e)) {
+        }, e, [&]() { inv_rr = 1.0 / rr; })) {
       status = TG_E_TIMEOUT;
       break;
     }
@@ -455,7 +500,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgmx(PcgMxArgs a) {
   int status = -1, iter = 0, n_ru = 0, since_ru = 0;
   if (!grid_total<BS>(v, partB, a.bar, rr)) status = TG_E_TIMEOUT;
   const double rr0 = rr;
-  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2);
+  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2), limit = 1e10 * rr0;
   double rr_true = rr;
   if (status < 0) {
     if (isnan(rr)) status = TG_E_NAN;
@@ -483,7 +528,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgmx(PcgMxArgs a) {
     };
     stencil_ld<float, 0, MU0>(g, a.km32, ld_a, a.Wt32, a.Wx32, epi_a);
     float af;
-    if (!grid_total_fx<BS>(va, partA, a.bar, fxA, [&](double pap) { return (float)(rr / pap); }, af)) {
+    if (!grid_total_fx<BS>(va, partA, a.bar, fxA, [&](double pap) { return (float)div_newton<false>(rr, pap); }, af)) {
       status = TG_E_TIMEOUT;
       break;
     }
@@ -502,12 +547,13 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgmx(PcgMxArgs a) {
     };
     stencil_ld<float, 1, MU0>(g, a.kd32, ld_b, a.Wt32, a.Wx32, epi_b);
     PcgTailMx e;
+    double inv_rr = 0;  // thread 0's
     if (!grid_total_fx<BS>(vb, partB, a.bar, fxB, [&](double rn) {
-          PcgTailMx o{rn, (float)(rn / rr), 0};
+          PcgTailMx o{rn, (float)(rn * inv_rr), 0};
           o.need = since_ru + 1 >= a.ru_interval || rn < stop || rn < kRuDrop * rr_true || iter + 1 >= a.maxiter ||
-                   rn / rr0 > 1e10 || isnan(rn);
+                   rn > limit || isnan(rn);
           return o;
-        }, e)) {
+        }, e, [&]() { inv_rr = 1.0 / rr; })) {
       status = TG_E_TIMEOUT;
       break;
     }
@@ -639,12 +685,16 @@ __device__ __forceinline__ void cgcg_update(const Geo& g, float4* __restrict__ r
 
 // Grid totals of a pair of partials (gamma, delta): block sums in FP32,
 // written to part as FP64 pairs; after the grid barrier, warp 0 of every block
-// adds all blocks' pairs (warp_read_partials) and hands the totals to the block
-// through one block barrier, two block barriers in all.
-template <int BS>
-__device__ __forceinline__ bool grid_total2(float va, float vb, double* part, const GridBar& bar, double2& out) {
+// adds all blocks' pairs (warp_read_partials) and hands f of the totals, computed
+// in its lane 0, to the block through one block barrier, two block barriers in
+// all.  (Every thread computing alpha and beta itself took four FP64 divisions
+// per thread and iteration, which the SM's FP64 pipe runs one warp at a time.)
+template <int BS, class F, class Prep = NoPrep>
+__device__ __forceinline__ bool grid_total2(float va, float vb, double* part, const GridBar& bar, F f,
+                                            decltype(f(0.0, 0.0))& out, Prep prep = {}) {
+  using S = decltype(f(0.0, 0.0));
   __shared__ float sha[BS / 32], shb[BS / 32];
-  __shared__ double2 s_out;
+  __shared__ S s_out;
   __shared__ int s_ok;
   va = warp_sum(va);
   vb = warp_sum(vb);
@@ -662,11 +712,11 @@ __device__ __forceinline__ bool grid_total2(float va, float vb, double* part, co
       part[2 * blockIdx.x] = (double)a;
       part[2 * blockIdx.x + 1] = (double)b;
     }
-    const bool ok = warp0_grid_wait(bar, gridDim.x, kBarrierSpinLimit);
+    const bool ok = warp0_grid_wait(bar, gridDim.x, kBarrierSpinLimit, prep);
     if (ok) {
       double t[2];
       warp_read_partials<2>(part, t);
-      if (lane == 0) s_out = make_double2(t[0], t[1]);
+      if (lane == 0) s_out = f(t[0], t[1]);
     }
     if (lane == 0) s_ok = ok;
   }
@@ -732,6 +782,12 @@ __device__ __forceinline__ int ru_status(double rt, double stop, double rr0, int
   return -1;
 }
 
+// An iteration's scalars: (r, r), alpha, beta, and whether a reliable update is due.
+struct CgcgStep {
+  double gam, alpha, beta;
+  int need;
+};
+
 template <int BS, bool MU0>
 __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
   if (threadIdx.x == 0) barrier_epoch() = 0;
@@ -746,14 +802,14 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
   int status = -1, iter = 0, n_ru = 0, since_ru = 0;
   if (!cgcg_start<BS>(a, r, p, sv, part, rr)) status = TG_E_TIMEOUT;
   const double rr0 = rr;
-  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2);
+  const double stop = stop_of(rr0, a.rel_tol, a.abs_tol2), limit = 1e10 * rr0;
   double rr_true = rr;
   if (status < 0) {
     if (isnan(rr)) status = TG_E_NAN;
     else if (!(rr >= stop) || rr == 0.0) status = TG_OK;
   }
-  // phase B: w = A r and the totals of (r, r) and (r, A r)
-  auto apply_sum = [&](double2& gd) -> bool {
+  // phase B: w = A r; f of the totals of (r, r) and (r, A r) into out
+  auto apply_sum = [&](auto f, CgcgStep& out, auto prep) -> bool {
     float ga = 0.f, de = 0.f;
     const PlainLd ld{r};
     auto epi = [&](int s, float2 wv, float2 u, const PlainOp& o) {
@@ -762,14 +818,14 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
       de = fmaf(u.x, u.x, fmaf(u.y, u.y, de));
     };
     stencil_mdagm<MU0>(g, a.km32, a.kd32, ld, a.Wt32, a.Wx32, epi);
-    return grid_total2<BS>(ga, de, part(), a.bar, gd);
+    return grid_total2<BS>(ga, de, part(), a.bar, f, out, prep);
   };
   double gam = 0, alpha = 0, beta = 0;
+  CgcgStep st;
   if (status < 0) {
-    double2 gd;
-    if (apply_sum(gd)) {
-      gam = gd.x;
-      alpha = gd.x / gd.y;
+    if (apply_sum([](double gn, double dn) { return CgcgStep{gn, gn / dn, 0.0, 0}; }, st, NoPrep{})) {
+      gam = st.gam;
+      alpha = st.alpha;
     } else {
       status = TG_E_TIMEOUT;
     }
@@ -777,21 +833,26 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
   while (status < 0) {
     cgcg_update(g, reinterpret_cast<float4*>(r), reinterpret_cast<const float4*>(w), reinterpret_cast<float4*>(sv),
                 reinterpret_cast<float4*>(p), reinterpret_cast<float4*>(a.xs), (float)alpha, (float)beta);
-    double2 gd;
-    if (!grid_barrier(a.bar) || !apply_sum(gd)) {
+    double inv_gam = 0, inv_alpha = 0;  // thread 0's
+    if (!grid_barrier(a.bar) || !apply_sum([&](double gn, double dn) {
+          const double be = gn * inv_gam;
+          const int need = since_ru + 1 >= a.ru_interval || gn < stop || gn < kRuDrop * rr_true ||
+                           iter + 1 >= a.maxiter || gn > limit || isnan(gn) || isnan(dn);
+          return CgcgStep{gn, div_newton(gn, dn - be * gn * inv_alpha), be, need};
+        }, st, [&]() {
+          inv_gam = 1.0 / gam;
+          inv_alpha = 1.0 / alpha;
+        })) {
       status = TG_E_TIMEOUT;
       break;
     }
-    const double gn = gd.x, dn = gd.y;
-    const bool need = since_ru + 1 >= a.ru_interval || gn < stop || gn < kRuDrop * rr_true ||
-                      iter + 1 >= a.maxiter || gn / rr0 > 1e10 || isnan(gn) || isnan(dn);
+    const int need = st.need;
     iter += 1;
     since_ru += 1;
     const double alpha_prev = alpha, gam_prev = gam;
-    beta = gn / gam;
-    alpha = gn / (dn - beta * gn / alpha);
-    gam = gn;
-    rr = gn;
+    beta = st.beta;
+    alpha = st.alpha;
+    gam = rr = st.gam;
     if (!need) continue;
     // reliable update, then w = A r for the replaced r
     double rt;
@@ -806,18 +867,17 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
     n_ru += 1;
     status = ru_status(rt, stop, rr0, iter, a.maxiter);
     if (status >= 0) break;
-    if (!apply_sum(gd)) {
+    if (!apply_sum([&](double gn, double dn) {
+          if (restart) return CgcgStep{gn, gn / dn, 0.0, 0};  // p and s restart from r and w
+          const double be = gn / gam_prev;
+          return CgcgStep{gn, gn / (dn - be * gn / alpha_prev), be, 0};
+        }, st, NoPrep{})) {
       status = TG_E_TIMEOUT;
       break;
     }
-    if (restart) {  // p and s restart from r and w
-      beta = 0;
-      alpha = gd.x / gd.y;
-    } else {
-      beta = gd.x / gam_prev;
-      alpha = gd.x / (gd.y - beta * gd.x / alpha_prev);
-    }
-    gam = gd.x;
+    beta = st.beta;
+    alpha = st.alpha;
+    gam = st.gam;
   }
   pcg_report(a.st, a.log, a.log_index, rr, rr0, stop, iter, n_ru, status);
 }
@@ -827,7 +887,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
 // stencil's work; cooperative launch so the barrier cannot wait on a block
 // that is not running.
 // ---------------------------------------------------------------------------
-template <class K> int pcg_resident(K kernel, int bs) {
+template <class K> int pcg_resident(K kernel, int bs, int smem = 0) {
   static std::mutex mu;
   static std::unordered_map<const void*, int> cache;
   std::lock_guard<std::mutex> lock(mu);
@@ -836,18 +896,20 @@ template <class K> int pcg_resident(K kernel, int bs) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, bs, 0) != cudaSuccess || per_sm <= 0)
+  if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, bs, smem) != cudaSuccess || per_sm <= 0)
     per_sm = 1;
   const int n = per_sm * sms;
   cache.emplace((const void*)kernel, n);
   return n;
 }
 
-template <class K, class Args> cudaError_t coop_launch(K kernel, int grid, int bs, cudaStream_t s, const Args& a) {
+template <class K, class Args>
+cudaError_t coop_launch(K kernel, int grid, int bs, cudaStream_t s, const Args& a, int smem = 0) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)bs);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -891,18 +953,19 @@ int pcg_block_override() {
 // (k1; L1-cached loads, block totals kept on chip): FP32 sums gain more from
 // that than from four blocks (32^2 4.7 against 6.9 us), FP64 less (12.2, 10.1).
 template <class K512, class K256, class K1, class Args>
-cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, cudaStream_t s, const Args& a) {
-  const int r512 = pcg_resident(k512, 512);
+cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, cudaStream_t s, const Args& a,
+                       int warp_smem = 0) {
+  const int r512 = pcg_resident(k512, 512, 16 * warp_smem);
   const int force = pcg_block_override();
-  if (force == 512) return coop_launch(k512, std::min(r512, kPcgMaxGrid), 512, s, a);
-  if (force == 0 && pcg_work(g, 512, 1) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a);
+  if (force == 512) return coop_launch(k512, std::min(r512, kPcgMaxGrid), 512, s, a, 16 * warp_smem);
+  if (force == 0 && pcg_work(g, 512, 1) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a, 16 * warp_smem);
   if (one_rows > 0 && pcg_work(g, 256, one_rows) == 1) return coop_launch(k1, 1, 256, s, a);
-  return coop_launch(k256, pcg_grid(g, pcg_resident(k256, 256), 256), 256, s, a);
+  return coop_launch(k256, pcg_grid(g, pcg_resident(k256, 256, 8 * warp_smem), 256), 256, s, a, 8 * warp_smem);
 }
 
 cudaError_t pcg64(cudaStream_t s, bool mu0, Pcg64Args a) {
-  if (mu0) return pcg_launch(a.g, k_pcg64<512, true>, k_pcg64<256, true>, k_pcg64<256, true, true>, 1, s, a);
-  return pcg_launch(a.g, k_pcg64<512, false>, k_pcg64<256, false>, k_pcg64<256, false, true>, 1, s, a);
+  if (mu0) return pcg_launch(a.g, k_pcg64<512, true>, k_pcg64<256, true>, k_pcg64<256, true, true>, 1, s, a, kRingWarp);
+  return pcg_launch(a.g, k_pcg64<512, false>, k_pcg64<256, false>, k_pcg64<256, false, true>, 1, s, a, kRingWarp);
 }
 
 cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, long long limit, int* status) {

@@ -32,6 +32,8 @@ __device__ __forceinline__ void march_row(const OpK<R>& k, int s, int lane, C2<R
   wtm = wt;
 }
 
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
 template <typename R> __device__ __forceinline__ C2<R> shfl_c2(C2<R> v, int src) {
   return mk<R>(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
@@ -196,6 +198,129 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
   }
 }
 
+// ---------------------------------------------------------------------------
+// The FP64 march with its rows prefetched through shared memory: each lane copies
+// its own column of the next rows -- the operand's sources, the links and the
+// vectors the epilogue reads -- with cp.async (16 bytes, through L2), D rows
+// ahead, and reads back only what it copied itself, so no barrier is needed.
+// Prefetched rows cost no registers, and the epilogue's reads no longer wait
+// behind the operator.  The edge operands of kMarchT rows are fetched likewise
+// by the first lanes.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Shared memory per warp: D rows of NS + 2 + NE arrays, two chunks of edges.
+template <int D, int NS, int NE> __host__ __device__ constexpr int ring_bytes() {
+  return D * (NS + 2 + NE) * 512 + 2 * (NS + 1) * 2 * kMarchT * 16;
+}
+
+// src[NS]: the operand's sources (comb(v) gives the operand from their values at
+// a site); ext[NE]: what the epilogue reads, handed to epi(s, out, operand, e).
+template <int DAG, bool MU0, int D, int NS, int NE, class Comb, class Epi>
+__device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k, const double2* const (&src)[NS],
+                                             const double2* const* ext, Comb comb, const FxLink* __restrict__ Wt,
+                                             const FxLink* __restrict__ Wx, int xw, int ta, int tb, Epi& epi,
+                                             unsigned char* ring) {
+  constexpr int NA = NS + 2 + NE, EL = 2 * kMarchT;
+  const int nx = g.nx, n = tb - ta;
+  const int lane = threadIdx.x & 31;
+  const int x0 = xw << 5, x = x0 + lane;
+  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
+  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;
+  double2* const rows = reinterpret_cast<double2*>(ring) + lane;
+  double2* const edges = reinterpret_cast<double2*>(ring + D * NA * 512) + (lane & (EL - 1));
+  const unsigned rows_a = smem_addr(rows), edges_a = smem_addr(edges);
+  // row ta + i into slot `slot`; with every kMarchT-th row the edges of its chunk
+  auto issue = [&](int i, int slot) {
+    const int t = ta + i, tp = (t + 1 == g.nt) ? 0 : t + 1;
+    const unsigned d = rows_a + slot * (NA * 512);
+    const int so = t * nx + x, sp = tp * nx + x;
+#pragma unroll
+    for (int j = 0; j < NS; j++) cp_async16(d + j * 512, src[j] + sp);
+    cp_async16(d + NS * 512, Wt + so);
+    cp_async16(d + (NS + 1) * 512, Wx + so);
+#pragma unroll
+    for (int j = 0; j < NE; j++) cp_async16(d + (NS + 2 + j) * 512, ext[j] + so);
+    if ((i & (kMarchT - 1)) == 0 && lane < EL) {
+      const int rr = min(t + (lane & (kMarchT - 1)), tb - 1);
+      const int c = rr * nx + (lane < kMarchT ? xle : xre);
+      const unsigned e = edges_a + ((i / kMarchT) & 1) * ((NS + 1) * EL * 16);
+#pragma unroll
+      for (int j = 0; j < NS; j++) cp_async16(e + j * (EL * 16), src[j] + c);
+      if (lane < kMarchT) cp_async16(e + NS * (EL * 16), Wx + c);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < D - 1; i++) {
+    if (i < n) issue(i, i);
+    cp_async_commit();
+  }
+  auto at = [&](int s) {
+    double2 v[NS];
+#pragma unroll
+    for (int j = 0; j < NS; j++) v[j] = __ldcg(src[j] + s);
+    return comb(v);
+  };
+  const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
+  const double2 below = at(tm * nx + x);
+  double2 own = at(ta * nx + x);
+  FxLink wtm = Wt[tm * nx + x];
+  FxC pm = to_fx(below), pc = to_fx(own), ef;
+  FxLink ew;
+  static_assert(D == kMarchT, "a chunk's rows and slots coincide");
+  for (int i0 = 0; i0 < n; i0 += kMarchT) {
+#pragma unroll
+    for (int ic = 0; ic < kMarchT; ic++) {
+      const int i = i0 + ic;
+      if (i >= n) break;
+      if (i + D - 1 < n) issue(i + D - 1, (ic + D - 1) % D);
+      cp_async_commit();
+      cp_async_wait<D - 1>();
+      if (ic == 0) {
+        const double2* e = edges + ((i0 / kMarchT) & 1) * ((NS + 1) * EL);
+        double2 v[NS];
+#pragma unroll
+        for (int j = 0; j < NS; j++) v[j] = e[j * EL];
+        ef = to_fx(comb(v));
+        ew = *reinterpret_cast<const FxLink*>(e + NS * EL);
+      }
+      const double2* rw = rows + ic * (NA * 32);
+      double2 v[NS];
+#pragma unroll
+      for (int j = 0; j < NS; j++) v[j] = rw[j * 32];
+      const FxLink wt = *reinterpret_cast<const FxLink*>(rw + NS * 32);
+      const FxLink wx = *reinterpret_cast<const FxLink*>(rw + (NS + 1) * 32);
+      const double2 pp = comb(v);
+      const FxC pe = shfl_fx(ef, (lane == 31) ? kMarchT + ic : ic);
+      const FxC pr = sel_fx(lane == 31, pe, shfl_fx(pc, lane + 1));
+      const FxC pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
+      const FxLink we = shfl_lk(ew, ic);
+      FxLink wl = shfl_lk(wx, lane - 1);
+      if (lane == 0) wl = we;
+      const FxC pn = to_fx(pp);
+      const int t = ta + i, s = t * nx + x;
+      double2 o;
+      if (!fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o)) {
+        const Nbr nb = neighbours(g, s, t, x);
+        o = dslash_vals<double, DAG, MU0>(k, own, at(nb.tp), at(nb.tm), at(nb.xp), at(nb.xm), fx_link_value(wt),
+                                          fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
+      }
+      epi(s, o, own, rw + (NS + 2) * 32);
+      pm = pc;
+      pc = pn;
+      own = pp;
+      wtm = wt;
+    }
+  }
+  cp_async_wait<0>();  // (only empty groups are left; the ring is free for the next segment)
+}
+
 template <typename R, int DAG, bool MU0, class Ld, class Epi>
 __device__ __forceinline__ void march_segment(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
                                               const Lk<R>* __restrict__ Wx, int xw, int ta, int tb, Epi& epi) {
@@ -340,7 +465,6 @@ template <typename R, int NSRC> __host__ __device__ constexpr int staged_smem_by
 constexpr int kStageWaitLimit = 1 << 22;
 static __device__ unsigned g_stage_faults;
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
