@@ -38,33 +38,47 @@ static int cluster_kernel_of(int cfg) {
 
 template <int BS, int MINB> const void* batch_kernel() { return (const void*)k_batch_trajectory<BS, MINB>; }
 
-static const void* batch_kernel_of(int cfg) {
+// The kernel that runs instance cfg.  The 64-register ones (8 blocks of 128 or 4 of
+// 256 threads per SM) run FP64 trajectories at 128 registers and half the
+// blocks: the integer limbs of the FP64 operator need about 125 in the march and
+// spill 2 KB at 64.  64 chains of 16^2 ... 128^2 at 4 blocks of 256:
+// 296 ms so, 549 at 64 registers; 512 chains of 16^2 at 8 blocks of 128: 5.3, 7.6.
+static const void* batch_kernel_of(int cfg, bool fp64) {
   switch (cfg) {
-    case 0: return batch_kernel<128, 8>();
-    case 1: return batch_kernel<256, 4>();
+    case 0: return fp64 ? batch_kernel<128, 4>() : batch_kernel<128, 8>();
+    case 1: return fp64 ? batch_kernel<256, 2>() : batch_kernel<256, 4>();
     case 2: return batch_kernel<256, 2>();
     case 3: return batch_kernel<256, 1>();
     case 4: return batch_kernel<384, 1>();
     default: return batch_kernel<512, 1>();
   }
 }
+static int batch_min_blocks(int cfg, bool fp64) {
+  return fp64 && cfg <= 1 ? kBatchCfgs[cfg].minb / 2 : kBatchCfgs[cfg].minb;
+}
+
+// One block's share of an SM's shared memory at its minimum resident blocks, less
+// the kernels' static part and the 1 KB the hardware keeps per block.
+int batch_smem_limit(int cfg) {
+  const int per_block = 228 * 1024 / (kBatchCfgs[cfg].cluster > 1 ? 1 : batch_min_blocks(cfg, true));
+  return std::min(per_block - 1024, 227 * 1024) - kBatchStaticSmem;
+}
 
 static void launch_blocks(cudaStream_t s, int cfg, int grid, const BatchChain* chains, const int* order, int n,
                           const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
-  switch (cfg) {
-    case 0: k_batch_trajectory<128, 8><<<grid, 128, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 1: k_batch_trajectory<256, 4><<<grid, 256, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 2: k_batch_trajectory<256, 2><<<grid, 256, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 3: k_batch_trajectory<256, 1><<<grid, 256, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 4: k_batch_trajectory<384, 1><<<grid, 384, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    default: k_batch_trajectory<512, 1><<<grid, 512, 0, s>>>(chains, order, n, F, P, results, queue); break;
-  }
+  const void* k = batch_kernel_of(cfg, P.cg.precision == TG_PREC_FP64);
+  const int sm = P.cg.smem;
+  if (sm > 0) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  BatchFields f = F;
+  BatchTraj p = P;
+  void* args[] = {&chains, &order, &n, &f, &p, &results, &queue};
+  cudaLaunchKernel(k, dim3((unsigned)grid), dim3((unsigned)kBatchCfgs[cfg].block), args, (size_t)sm, s);
 }
 
-int batch_teams(int cfg, int sms) {
+int batch_teams(int cfg, int sms, bool fp64) {
   if (kBatchCfgs[cfg].cluster > 1) return batch_cluster_max(cluster_kernel_of(cfg));
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_kernel_of(cfg), kBatchCfgs[cfg].block, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_kernel_of(cfg, fp64), kBatchCfgs[cfg].block, 0) !=
       cudaSuccess)
     return 0;
   return nb * sms;
@@ -83,15 +97,18 @@ void batch_filler_launch(cudaStream_t s, int cfg, int blocks, const BatchChain* 
   f.from_back = 1;
   // the one-block instance of the cluster kernel's block size: its solo chains
   // run the same code, so a chain's result does not depend on which block ran it
-  if (kBatchCfgs[cfg].block == 512)
-    k_batch_trajectory<512, 1><<<blocks, 512, 0, s>>>(chains, order, n, F, f, results, queue);
-  else
-    k_batch_trajectory<256, 1><<<blocks, 256, 0, s>>>(chains, order, n, F, f, results, queue);
+  const bool wide = kBatchCfgs[cfg].block == 512;
+  const int sm = P.cg.smem;
+  if (sm > 0)
+    cudaFuncSetAttribute(wide ? batch_kernel<512, 1>() : batch_kernel<256, 1>(),
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (wide) k_batch_trajectory<512, 1><<<blocks, 512, sm, s>>>(chains, order, n, F, f, results, queue);
+  else k_batch_trajectory<256, 1><<<blocks, 256, sm, s>>>(chains, order, n, F, f, results, queue);
 }
 
 void batch_trajectory(cudaStream_t s, int cfg, int sms, const BatchChain* chains, const int* order, int n,
                       const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
-  const int teams = std::min(n, std::max(1, batch_teams(cfg, sms)));
+  const int teams = std::min(n, std::max(1, batch_teams(cfg, sms, P.cg.precision == TG_PREC_FP64)));
   if (kBatchCfgs[cfg].cluster > 1)
     batch_cluster_launch(s, cluster_kernel_of(cfg), teams, chains, order, n, F, P, results, queue);
   else launch_blocks(s, cfg, teams, chains, order, n, F, P, results, queue);

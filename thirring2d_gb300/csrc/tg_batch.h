@@ -26,6 +26,7 @@ struct BatchFields {
 struct BatchCg {
   double rel_tol, abs_tol2;
   int maxiter, precision, ru_interval;
+  int smem;  // dynamic shared memory of a block (FP64: one-block chains that fit keep their vectors there)
 };
 
 struct BatchTraj {
@@ -80,8 +81,13 @@ void batch_trajectory(cudaStream_t s, int cfg, int sms, const BatchChain* chains
 int batch_filler_blocks(int cfg, int sms);
 void batch_filler_launch(cudaStream_t s, int cfg, int blocks, const BatchChain* chains, const int* order, int n,
                          const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue);
+// Bytes of shared memory per site of an FP64 chain that one block solves in its
+// shared memory (block_cg64_small), the kernels' static shared memory at most,
+// and what instance cfg has for it per block.
+constexpr int kSmallSite = 5 * 16 + 2 * 4, kBatchStaticSmem = 1536;
+int batch_smem_limit(int cfg);
 // teams (blocks or clusters) of instance cfg that can be resident at once (0: cannot launch)
-int batch_teams(int cfg, int sms);
+int batch_teams(int cfg, int sms, bool fp64);
 // the tuned instance as reported to callers: block * 100 + 10 * cluster (if > 1)
 // + min blocks per SM, + 100000 * (solo_sites / 1024), + 1000000 with pairs
 inline int batch_cfg_id(const BatchCfg& c) {

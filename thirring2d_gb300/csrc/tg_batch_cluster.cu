@@ -36,15 +36,22 @@ int batch_cluster_max(int which) {
   }
 }
 
+template <int BS, int CL, bool PAIRS = false>
+static void launch_cluster(cudaStream_t s, int clusters, const BatchChain* chains, const int* order, int n,
+                           const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
+  const int sm = P.cg.smem;
+  if (sm > 0)
+    cudaFuncSetAttribute(k_batch_cluster<BS, CL, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  k_batch_cluster<BS, CL, PAIRS><<<clusters * CL, BS, sm, s>>>(chains, order, n, F, P, results, queue);
+}
+
 void batch_cluster_launch(cudaStream_t s, int which, int clusters, const BatchChain* chains, const int* order, int n,
                           const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
   switch (which) {
-    case 0: k_batch_cluster<512, 2><<<clusters * 2, 512, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 1: k_batch_cluster<512, 4><<<clusters * 4, 512, 0, s>>>(chains, order, n, F, P, results, queue); break;
-    case 3:
-      k_batch_cluster<512, 4, true><<<clusters * 4, 512, 0, s>>>(chains, order, n, F, P, results, queue);
-      break;
-    default: k_batch_cluster<256, 4><<<clusters * 4, 256, 0, s>>>(chains, order, n, F, P, results, queue); break;
+    case 0: launch_cluster<512, 2>(s, clusters, chains, order, n, F, P, results, queue); break;
+    case 1: launch_cluster<512, 4>(s, clusters, chains, order, n, F, P, results, queue); break;
+    case 3: launch_cluster<512, 4, true>(s, clusters, chains, order, n, F, P, results, queue); break;
+    default: launch_cluster<256, 4>(s, clusters, chains, order, n, F, P, results, queue); break;
   }
 }
 

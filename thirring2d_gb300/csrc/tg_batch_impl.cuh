@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "tg_batch.h"
+#include "tg_scalar.cuh"
 #include "tg_stencil.cuh"
 
 namespace tg {
@@ -38,6 +39,7 @@ __device__ __forceinline__ double warp_allsum(double v) {
 // sum.
 struct TeamScratch {
   double part[32];
+  longlong2 ipart[32];  // integer partials (sum_int)
   double total[2];  // a cluster's block totals alternate between two slots
   double out[4];
   int phase;        // the slot of the next sum (thread 0 only)
@@ -61,7 +63,10 @@ template <typename P> __device__ __forceinline__ double block_total_warp0(P v, T
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (lane == 0) sc.part[w] = (double)v;
   __syncthreads();  // also publishes every global write made before the call
-  return w == 0 ? warp_allsum(lane < nw ? sc.part[lane] : 0.0) : 0.0;
+  if (w != 0) return 0.0;
+  double t = lane < nw ? sc.part[lane] : 0.0;
+  for (int o = nw > 8 ? 16 : 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return __shfl_sync(0xffffffffu, t, 0);
 }
 
 // A team runs one chain.  It gives the chain-wide loop over sites, barrier and
@@ -69,12 +74,14 @@ template <typename P> __device__ __forceinline__ double block_total_warp0(P v, T
 // the same decisions and the team's control flow stays uniform.
 //
 // sum_then(v, f): the team's total of the threads' partials v, handed to f,
-// which runs once per block (thread 0); every thread gets f's result (a small
-// trivially copyable struct).  Scalars derived from a sum -- CG step lengths,
+// which runs in warp 0 of each block (all lanes, with the same total, so that it can
+// take two quotients at once: first_quotients); every thread gets lane 0's result (a
+// small trivially copyable struct).  Scalars derived from a sum -- CG step lengths,
 // the stopping tests -- are computed there once instead of in every thread:
-// the FP64 pipe retires two operations per SM per clock, and one double
-// division is about ten of them.
+// the FP64 pipe retires two operations per SM per clock, and a double division
+// is about ten of them with a latency of 574 clocks.
 struct BlockTeam {  // one thread block
+  static constexpr int nblocks_const = 1;
   __device__ static int rank() { return 0; }
   __device__ static int nblocks() { return 1; }
   __device__ static void sync() { __syncthreads(); }
@@ -83,7 +90,10 @@ struct BlockTeam {  // one thread block
     static_assert(sizeof(S) <= sizeof(TeamScratch::out), "sum_then result too large");
     TeamScratch& sc = team_scratch();
     const double t = block_total_warp0(v, sc);
-    if (threadIdx.x == 0) *reinterpret_cast<S*>(sc.out) = f(t);
+    if (threadIdx.x < 32) {
+      const S r = f(t);
+      if (threadIdx.x == 0) *reinterpret_cast<S*>(sc.out) = r;
+    }
     __syncthreads();
     return *reinterpret_cast<const S*>(sc.out);
   }
@@ -102,6 +112,7 @@ struct BlockTeam {  // one thread block
 // totals through distributed shared memory, in the same order in every block,
 // so the blocks stay in lockstep.
 template <int CL> struct ClusterTeam {
+  static constexpr int nblocks_const = CL;
   __device__ static int rank() { return (int)cooperative_groups::this_cluster().block_rank(); }
   __device__ static int nblocks() { return CL; }
   __device__ static void sync() { cooperative_groups::this_cluster().sync(); }
@@ -117,11 +128,18 @@ template <int CL> struct ClusterTeam {
     }
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     cl.sync();  // every block's total is written, with every write made before the call
-    if (threadIdx.x == 0) {
-      double s = 0;
-      for (int r = 0; r < CL; r++) s += cl.map_shared_rank(sc.total, r)[ph];
-      *reinterpret_cast<S*>(sc.out) = f(s);
-      sc.phase = ph ^ 1;
+    if (threadIdx.x < 32) {
+      // lane r reads block r's total; CL is a power of two, and the butterfly adds in
+      // the same order in every lane and block
+      ph = __shfl_sync(0xffffffffu, ph, 0);
+      double s = (threadIdx.x < CL) ? cl.map_shared_rank(sc.total, threadIdx.x)[ph] : 0.0;
+#pragma unroll
+      for (int o = CL / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const S r = f(__shfl_sync(0xffffffffu, s, 0));
+      if (threadIdx.x == 0) {
+        *reinterpret_cast<S*>(sc.out) = r;
+        sc.phase = ph ^ 1;
+      }
     }
     // A block barrier publishes out.  The slot just read is written again two
     // sums later, after the next sum's cluster barrier, which no block passes
@@ -207,6 +225,7 @@ __device__ __forceinline__ void pair_barrier() {
 }
 
 struct PairTeam {
+  static constexpr int nblocks_const = 2;
   __device__ static int rank() { return (int)(cooperative_groups::this_cluster().block_rank() & 1u); }
   __device__ static int nblocks() { return 2; }
   __device__ static void sync() { pair_barrier(); }
@@ -221,13 +240,14 @@ struct PairTeam {
       sc.total[ph] = b;
     }
     pair_barrier();  // both totals written
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
       cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-      const double mine = sc.total[ph];
-      const double other = cl.map_shared_rank(sc.total, cl.block_rank() ^ 1u)[ph];
-      const double s = (rank() == 0) ? mine + other : other + mine;  // pair rank 0's total first
-      *reinterpret_cast<S*>(sc.out) = f(s);
-      sc.phase = ph ^ 1;
+      ph = __shfl_sync(0xffffffffu, ph, 0);
+      const S r = f(sc.total[ph] + cl.map_shared_rank(sc.total, cl.block_rank() ^ 1u)[ph]);
+      if (threadIdx.x == 0) {
+        *reinterpret_cast<S*>(sc.out) = r;
+        sc.phase = ph ^ 1;
+      }
     }
     // as in ClusterTeam: the slot just read is written again two sums later,
     // after the next sum's pair barrier
@@ -267,9 +287,13 @@ struct CgOut {
   int iter, status, n_ru;
 };
 
-// What the CG loops need after the |r|^2 sum: the sum, beta, and the verdict
-// of the stopping tests (FP64: a status, or -1 to go on; mixed: whether a
-// reliable update is due, which runs the tests on the true residual).
+// What the CG loops need after their sums: alpha and 1 / |r|^2 after the first;
+// |r|^2, beta and the verdict of the stopping tests after the second (FP64: a
+// status, or -1 to go on; mixed: whether a reliable update is due, which runs the
+// tests on the true residual).
+struct CgStep {
+  double alpha, inv_rr;
+};
 struct CgTail64 {
   double rn, beta;
   int status;
@@ -280,6 +304,56 @@ struct CgTailMx {
   int need;
 };
 
+// rr / pap and 1 / rr, in lanes 0 and 1 of one warp: one division's latency.
+__device__ __forceinline__ CgStep first_quotients(double rr, double pap) {
+  const bool second = (threadIdx.x & 31) == 1;
+  const double q = div_newton(second ? 1.0 : rr, second ? rr : pap);
+  return CgStep{__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1)};
+}
+
+struct Cg64Tests {
+  double stop, limit;
+  int maxiter;
+  __device__ __forceinline__ int operator()(double rn, int iter) const {
+    if (isnan(rn)) return TG_E_NAN;
+    if (rn < stop) return TG_OK;
+    if (rn > limit) return TG_E_DIVERGED;
+    return iter >= maxiter ? TG_E_NOCONV : -1;
+  }
+};
+
+// The block's total as sum_then, by integers at the scale of the last total of
+// the kind (tg_scalar.cuh): the FP64 pipe, which bounds a block of many chains,
+// is left out of it.  A sum whose scale does not fit is taken again in FP64.
+template <class F> __device__ __forceinline__ auto block_sum_int(double v, int& ref, F f) -> decltype(f(0.0)) {
+  using S = decltype(f(0.0));
+  static_assert(sizeof(S) <= sizeof(TeamScratch::out), "sum result too large");
+  __shared__ int s_ref;
+  TeamScratch& sc = team_scratch();
+  const longlong2 q = fx_warp_partial(fx_term(v, ref));
+  if ((threadIdx.x & 31) == 0) sc.ipart[threadIdx.x >> 5] = q;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double t;
+    const bool ok = fx_partials_total(sc.ipart, blockDim.x >> 5, ref, t);
+    const S r = f(t);
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<S*>(sc.out) = r;
+      s_ref = ok ? fx_total_ref(t) : -1;
+    }
+  }
+  __syncthreads();
+  if (s_ref < 0) {
+    return BlockTeam::sum_then(v, [&](double t) {
+      ref = 0;
+      if (threadIdx.x == 0) s_ref = fx_total_ref(t);
+      return f(t);
+    });
+  }
+  ref = s_ref;
+  return *reinterpret_cast<const S*>(sc.out);
+}
+
 // ---------------------------------------------------------------------------
 // CG on M^dag M inside one block.  Same recurrences, stopping rules and
 // reliable-update rules as the single-lattice solver (tg_kernels.cu): p is
@@ -287,7 +361,8 @@ struct CgTailMx {
 // after a restart), pAp = |Mp|^2.
 // ---------------------------------------------------------------------------
 template <bool MU0, class T>
-__device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
+__device__ __noinline__ CgOut block_cg64(const ChainCtx& ctx, const BatchCg& P, const double2* b, double2* x) {
+  const ChainCtx c = ctx;  // out of shared memory: what the loops use of it stays in registers
   const int V = c.g.V;
   const OpK<double>&km = c.km, &kd = c.kd;
   double a = 0;
@@ -306,6 +381,7 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
     out.status = isnan(rr0) ? TG_E_NAN : TG_OK;
     return out;
   }
+  const Cg64Tests tests{stop, 1e10 * rr0, P.maxiter};
   double rr = rr0, beta = 0;
   int half = 0;
   while (true) {
@@ -325,7 +401,8 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
       v = fma(o.y, o.y, v);
     };
     stencil_team<T, double, 0, MU0>(c.g, km, ld, c.Wtq, c.Wxq, epi);
-    const double alpha = T::sum_then(v, [&](double pAp) { return rr / pAp; });
+    const CgStep st = T::sum_then(v, [&](double pAp) { return first_quotients(rr, pAp); });
+    const double alpha = st.alpha;
     v = 0;
     auto ld2 = [&](int i) { return c.Mp64[i]; };
     auto epi2 = [&](int s, double2 ap, double2) {
@@ -341,12 +418,7 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
     };
     stencil_team<T, double, 1, MU0>(c.g, kd, ld2, c.Wtq, c.Wxq, epi2);
     const CgTail64 e = T::sum_then(v, [&](double rn) {
-      CgTail64 o{rn, rn / rr, -1};
-      if (isnan(rn)) o.status = TG_E_NAN;
-      else if (rn < stop) o.status = TG_OK;
-      else if (rn / rr0 > 1e10) o.status = TG_E_DIVERGED;
-      else if (out.iter + 1 >= P.maxiter) o.status = TG_E_NOCONV;
-      return o;
+      return CgTail64{rn, rn * st.inv_rr, tests(rn, out.iter + 1)};
     });
     half ^= 1;
     out.iter++;
@@ -361,10 +433,145 @@ __device__ CgOut block_cg64(const ChainCtx& c, const BatchCg& P, const double2* 
   return out;
 }
 
+// The same for a chain whose vectors fit the block's dynamic shared memory (kept:
+// kSmallSite bytes a site): p' and M p' are converted to block floating point
+// once, where they are computed, instead of at each of the five sites that read
+// them, and the sums are integers.
+template <bool MU0>
+__device__ __noinline__ CgOut block_cg64_small(const ChainCtx& ctx, const BatchCg& P, const double2* b, double2* xout) {
+  const ChainCtx c = ctx;
+  extern __shared__ __align__(16) unsigned char batch_smem[];
+  const Geo g = c.g;
+  const int V = g.V, T = blockDim.x, tid = threadIdx.x;
+  longlong2* const pm = reinterpret_cast<longlong2*>(batch_smem);
+  longlong2* const qm = pm + V;
+  double2* const p = reinterpret_cast<double2*>(qm + V);
+  double2* const r = p + V;
+  double2* const x = r + V;
+  int* const pe = reinterpret_cast<int*>(x + V);
+  int* const qe = pe + V;
+  const FxLink* const Wt = c.Wtq;
+  const FxLink* const Wx = c.Wxq;
+  double a = 0;
+  for (int s = tid; s < V; s += T) {
+    const double2 bb = b[s];
+    x[s] = make_double2(0, 0);
+    r[s] = bb;
+    p[s] = bb;
+    a += bb.x * bb.x + bb.y * bb.y;
+  }
+  const double rr0 = BlockTeam::sum(a);
+  double stop = P.abs_tol2;
+  if (P.rel_tol > 0 && P.rel_tol * P.rel_tol * rr0 > stop) stop = P.rel_tol * P.rel_tol * rr0;
+  CgOut out{0, TG_OK, 0};
+  const bool none = !(rr0 >= stop) || rr0 == 0.0;
+  if (none) out.status = isnan(rr0) ? TG_E_NAN : TG_OK;
+  const Cg64Tests tests{stop, 1e10 * rr0, P.maxiter};
+  double rr = rr0, beta = 0;
+  int refA = fx_total_ref(rr0), refB = refA;
+  auto get = [](const longlong2* m, const int* e, int i) { return FxC{m[i].x, m[i].y, e[i]}; };
+  while (!none) {
+    for (int s = tid; s < V; s += T) {
+      const double2 rv = r[s], pv = p[s];
+      const double2 pn = make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y));
+      const FxC f = to_fx(pn);
+      p[s] = pn;
+      pm[s] = make_longlong2(f.re, f.im);
+      pe[s] = f.e;
+    }
+    __syncthreads();
+    double v = 0;
+    for (int s = tid; s < V; s += T) {
+      int t, xx;
+      site_tx(g, s, t, xx);
+      const Nbr n = neighbours(g, s, t, xx);
+      const FxLink wt = Wt[s], wtd = Wt[n.tm], wx = Wx[s], wxd = Wx[n.xm];
+      double2 o;
+      if (!fx_dslash<0, MU0>(c.km, get(pm, pe, s), get(pm, pe, n.tp), get(pm, pe, n.tm), get(pm, pe, n.xp),
+                             get(pm, pe, n.xm), wt, wtd, wx, wxd, o))
+        o = dslash_vals<double, 0, MU0>(c.km, p[s], p[n.tp], p[n.tm], p[n.xp], p[n.xm], fx_link_value(wt),
+                                        fx_link_value(wtd), fx_link_value(wx), fx_link_value(wxd));
+      const FxC f = to_fx(o);
+      qm[s] = make_longlong2(f.re, f.im);
+      qe[s] = f.e;
+      v = fma(o.x, o.x, v);
+      v = fma(o.y, o.y, v);
+    }
+    const CgStep st = block_sum_int(v, refA, [&](double pap) { return first_quotients(rr, pap); });
+    const double alpha = st.alpha;
+    v = 0;
+    for (int s = tid; s < V; s += T) {
+      int t, xx;
+      site_tx(g, s, t, xx);
+      const Nbr n = neighbours(g, s, t, xx);
+      const FxLink wt = Wt[s], wtd = Wt[n.tm], wx = Wx[s], wxd = Wx[n.xm];
+      double2 o;
+      if (!fx_dslash<1, MU0>(c.kd, get(qm, qe, s), get(qm, qe, n.tp), get(qm, qe, n.tm), get(qm, qe, n.xp),
+                             get(qm, qe, n.xm), wt, wtd, wx, wxd, o))
+        o = dslash_vals<double, 1, MU0>(c.kd, fx_value(get(qm, qe, s)), fx_value(get(qm, qe, n.tp)),
+                                        fx_value(get(qm, qe, n.tm)), fx_value(get(qm, qe, n.xp)),
+                                        fx_value(get(qm, qe, n.xm)), fx_link_value(wt), fx_link_value(wtd),
+                                        fx_link_value(wx), fx_link_value(wxd));
+      double2 xv = x[s], rv = r[s];
+      const double2 pv = p[s];
+      xv.x += alpha * pv.x;
+      xv.y += alpha * pv.y;
+      rv.x -= alpha * o.x;
+      rv.y -= alpha * o.y;
+      x[s] = xv;
+      r[s] = rv;
+      v = fma(rv.x, rv.x, v);
+      v = fma(rv.y, rv.y, v);
+    }
+    const CgTail64 e = block_sum_int(v, refB, [&](double rn) {
+      return CgTail64{rn, rn * st.inv_rr, tests(rn, out.iter + 1)};
+    });
+    out.iter++;
+    beta = e.beta;
+    rr = e.rn;
+    if (e.status >= 0) {
+      out.status = e.status;
+      break;
+    }
+  }
+  for (int s = tid; s < V; s += T) xout[s] = x[s];
+  __syncthreads();
+  return out;
+}
+
+// The mixed CG's reliable update: x += xs, xs = 0; r = b - M^dag M x in FP64, kept
+// in FP32; returns |r|^2.  (Apart from the iterations, which it would otherwise cost
+// registers.)
 template <bool MU0, class T>
-__device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
+__device__ __noinline__ double block_reliable(const ChainCtx& ctx, const double2* b, double2* x) {
+  const ChainCtx c = ctx;
   const int V = c.g.V;
-  const OpK<double>&km = c.km, &kd = c.kd;
+  TG_BSITES(s, V) {
+    float2 d = c.xs[s];
+    double2 xv = x[s];
+    xv.x += (double)d.x;
+    xv.y += (double)d.y;
+    x[s] = xv;
+    c.xs[s] = make_float2(0.f, 0.f);
+  }
+  T::sync();
+  TG_BSITES(s, V) c.tmp[s] = dslash_at<double, 0, MU0>(c.g, c.km, x, c.Wtq, c.Wxq, s);
+  T::sync();
+  double a = 0;
+  TG_BSITES(s, V) {
+    double2 ap = dslash_at<double, 1, MU0>(c.g, c.kd, c.tmp, c.Wtq, c.Wxq, s);
+    double2 bb = b[s];
+    double2 rv = make_double2(bb.x - ap.x, bb.y - ap.y);
+    c.rs[s] = make_float2((float)rv.x, (float)rv.y);
+    a = fma(rv.x, rv.x, a);
+    a = fma(rv.y, rv.y, a);
+  }
+  return T::sum(a);
+}
+
+template <bool MU0, class T>
+__device__ __noinline__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
+  const int V = c.g.V;
   OpK<float> km32{(float)c.m, (float)c.ep, (float)-c.em, MU0}, kd32{(float)c.m, (float)-c.em, (float)c.ep, MU0};
   double a = 0;
   TG_BSITES(s, V) {
@@ -384,7 +591,8 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
     out.status = isnan(rr0) ? TG_E_NAN : TG_OK;
     return out;
   }
-  double rr = rr0, rr_true = rr0;
+  const double limit = 1e10 * rr0;
+  double rr = rr0, drop = kRuDrop * rr0;
   float fb = 0.f;
   int since = 0, half = 0;
   // The FP32 iteration's operands, out of the shared-memory context: read
@@ -413,7 +621,8 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
       v = fmaf(o.y, o.y, v);
     };
     stencil_team<T, float, 0, MU0>(g, km32, ld, Wt32, Wx32, epi);
-    const float fa = T::sum_then(v, [&](double pAp) { return (float)(rr / pAp); });
+    const CgStep st = T::sum_then(v, [&](double pAp) { return first_quotients(rr, pAp); });
+    const float fa = (float)st.alpha;
     v = 0;
     auto ld2 = [&](int i) { return Mps[i]; };
     auto epi2 = [&](int s, float2 ap, float2) {
@@ -429,9 +638,9 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
     };
     stencil_team<T, float, 1, MU0>(g, kd32, ld2, Wt32, Wx32, epi2);
     const CgTailMx e = T::sum_then(v, [&](double rn) {
-      CgTailMx o{rn, (float)(rn / rr), 0};
-      o.need = since + 1 >= P.ru_interval || rn < stop || rn < kRuDrop * rr_true || out.iter + 1 >= P.maxiter ||
-               rn / rr0 > 1e10 || isnan(rn);
+      CgTailMx o{rn, (float)(rn * st.inv_rr), 0};
+      o.need = since + 1 >= P.ru_interval || rn < stop || rn < drop || out.iter + 1 >= P.maxiter || rn > limit ||
+               isnan(rn);
       return o;
     });
     half ^= 1;
@@ -440,36 +649,15 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
     fb = e.fb;
     rr = e.rn;
     if (!e.need) continue;
-    // reliable update: x += xs, r = b - M^dag M x in FP64
-    TG_BSITES(s, V) {
-      float2 d = c.xs[s];
-      double2 xv = x[s];
-      xv.x += (double)d.x;
-      xv.y += (double)d.y;
-      x[s] = xv;
-      c.xs[s] = make_float2(0.f, 0.f);
-    }
-    T::sync();
-    TG_BSITES(s, V) c.tmp[s] = dslash_at<double, 0, MU0>(c.g, km, x, c.Wtq, c.Wxq, s);
-    T::sync();
-    double a2 = 0;
-    TG_BSITES(s, V) {
-      double2 ap = dslash_at<double, 1, MU0>(c.g, kd, c.tmp, c.Wtq, c.Wxq, s);
-      double2 bb = b[s];
-      double2 rv = make_double2(bb.x - ap.x, bb.y - ap.y);
-      c.rs[s] = make_float2((float)rv.x, (float)rv.y);
-      a2 = fma(rv.x, rv.x, a2);
-      a2 = fma(rv.y, rv.y, a2);
-    }
-    const double rt = T::sum(a2);
+    const double rt = block_reliable<MU0, T>(c, b, x);
     if (rt > kRuRestart * rr) fb = 0.f;  // recursive residual far too optimistic: restart p from r
     rr = rt;
-    rr_true = rt;
+    drop = kRuDrop * rt;
     since = 0;
     out.n_ru++;
     if (isnan(rt)) { out.status = TG_E_NAN; break; }
     if (rt < stop) { out.status = TG_OK; break; }
-    if (rt / rr0 > 1e10) { out.status = TG_E_DIVERGED; break; }
+    if (rt > limit) { out.status = TG_E_DIVERGED; break; }
     if (out.iter >= P.maxiter) { out.status = TG_E_NOCONV; break; }
   }
   T::sync();
@@ -478,17 +666,35 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
 
 template <bool MU0, class T>
 __device__ __forceinline__ CgOut block_cg(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
-  return P.precision == TG_PREC_MIXED ? block_cg_mixed<MU0, T>(c, P, b, x) : block_cg64<MU0, T>(c, P, b, x);
+  if (P.precision == TG_PREC_MIXED) return block_cg_mixed<MU0, T>(c, P, b, x);
+  if constexpr (T::nblocks_const == 1) {
+    // (8^2 chains: 1.8 ms per 512-chain trajectory here, 1.6 on the global path)
+    if (c.g.V >= 128 && c.g.V * kSmallSite <= P.smem) return block_cg64_small<MU0>(c, P, b, x);
+  }
+  return block_cg64<MU0, T>(c, P, b, x);
 }
 
 // ---------------------------------------------------------------------------
 // One trajectory of one chain (update_gauge, hmc.c:671-746), by one block.
 // ---------------------------------------------------------------------------
+// out = M in (DAG = 0) or M^dag in (1) over the team's sites; returns the thread's
+// share of Re <in, out>
+template <int DAG, bool MU0, class T>
+__device__ __noinline__ double team_apply(const ChainCtx& ctx, const double2* in, double2* out) {
+  const ChainCtx c = ctx;
+  double a = 0;
+  TG_BSITES(s, c.g.V) {
+    const double2 o = dslash_at<double, DAG, MU0>(c.g, DAG ? c.kd : c.km, in, c.Wtq, c.Wxq, s), n = in[s];
+    if (out != nullptr) out[s] = o;
+    a += n.x * o.x + n.y * o.y;
+  }
+  return a;
+}
+
 template <bool MU0, class T>
 __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainResult* res) {
   const int V = c.g.V;
   const Geo& g = c.g;
-  const OpK<double>&km = c.km, &kd = c.kd;
   const unsigned long long tr = res->traj;
   const bool noise_on = P.stochastic_term != 0;
   const double fac = kNf / c.gc;
@@ -508,16 +714,8 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     c.An[s] = a;
   }
   const double Spf0 = T::sum(a_pf), Smom0 = T::sum(a_mom), Sg0 = fac * T::sum(a_g);
-  double a_md = 0;
-  TG_BSITES(s, V) {
-    c.phi[s] = dslash_at<double, 1, MU0>(g, kd, c.tmp, c.Wtq, c.Wxq, s);  // phi = M^dag eta
-    if (noise_on) {
-      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wtq, c.Wxq, s);
-      double2 n = c.noise[s];
-      a_md += n.x * o.x + n.y * o.y;
-    }
-  }
-  const double Smd0 = T::sum(a_md);
+  team_apply<1, MU0, T>(c, c.tmp, c.phi);  // phi = M^dag eta
+  const double Smd0 = T::sum(noise_on ? team_apply<1, MU0, T>(c, c.noise, nullptr) : 0.0);
   // leapfrog, hmc.c:708-716 (two half steps between MD steps share a pass)
   const double eps = P.tau / P.nsteps;
   const double cstep = 2.0 * (P.tau * 0.5 / P.nsteps);
@@ -545,7 +743,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     // in tmp (the same function of the same operands); otherwise apply M.
     const double2* Mx = c.tmp;
     if (P.cg.precision != TG_PREC_MIXED || o.n_ru == 0) {
-      TG_BSITES(s, V) c.Mx[s] = dslash_at<double, 0, MU0>(g, km, c.x, c.Wtq, c.Wxq, s);
+      team_apply<0, MU0, T>(c, c.x, c.Mx);
       T::sync();
       Mx = c.Mx;
     }
@@ -566,17 +764,13 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     T::sync();
   }
   // end actions, hmc.c:719-726
-  double b_pf = 0, b_mom = 0, b_g = 0, b_md = 0;
+  double b_pf = 0, b_mom = 0, b_g = 0;
+  const double b_md = noise_on ? team_apply<1, MU0, T>(c, c.noise, nullptr) : 0.0;
   TG_BSITES(s, V) {
     double2 ph = c.phi[s], xv = c.x[s], p = c.mom[s], a = c.An[s];
     b_pf += ph.x * xv.x + ph.y * xv.y;
     b_mom += p.x * p.x + p.y * p.y;
     b_g += (1. - cos(a.x)) + (1. - cos(a.y));
-    if (noise_on) {
-      double2 o = dslash_at<double, 1, MU0>(g, kd, c.noise, c.Wtq, c.Wxq, s);
-      double2 n = c.noise[s];
-      b_md += n.x * o.x + n.y * o.y;
-    }
   }
   const double Spf1 = T::sum(b_pf), Smom1 = T::sum(b_mom), Sg1 = fac * T::sum(b_g), Smd1 = T::sum(b_md);
   const double dS = Smom1 - Smom0 + Spf1 - Spf0 + Smd1 - Smd0 + Sg1 - Sg0;  // hmc.c:729-732

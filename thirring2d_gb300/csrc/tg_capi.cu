@@ -1497,12 +1497,28 @@ int batch_cfg(const tg_batch* B, const tg_batch_params& p) {
 
 int batch_launch(tg_batch* B, const tg_batch_params& p, int cfg, cudaStream_t s) {
   if (cfg < 0 || cfg >= kBatchNumCfgs) return fail(TG_E_ARG, "unknown batch kernel instance");
-  if (batch_teams(cfg, B->sms) <= 0) return fail(TG_E_CUDA, "batch kernel instance cannot launch on this GPU");
+  if (batch_teams(cfg, B->sms, p.cg.precision == TG_PREC_FP64) <= 0) return fail(TG_E_CUDA, "batch kernel instance cannot launch on this GPU");
   BatchTraj t;
   t.nsteps = p.nsteps;
   t.tau = p.tau;
   t.stochastic_term = p.stochastic_term;
-  t.cg = BatchCg{p.cg.rel_tol, p.cg.abs_tol2, p.cg.maxiter, p.cg.precision, p.cg.ru_interval};
+  t.cg = BatchCg{p.cg.rel_tol, p.cg.abs_tol2, p.cg.maxiter, p.cg.precision, p.cg.ru_interval, 0};
+  if (p.cg.precision == TG_PREC_FP64) {
+    // Room for the largest chain that fits a block's share, where such chains are
+    // most of the work; elsewhere the larger chains need the L1 (512 chains of
+    // 16^2 ... 128^2, of which 48^2 would fit: 145 ms with, 137 without).
+    const int limit = batch_smem_limit(cfg);
+    double all = 0, fits = 0;
+    int need = 0;
+    for (const tg_chain_params& c : B->P) {
+      const double V = (double)c.nt * c.nx, cost = V / std::max(fabs(c.m), 1e-3);
+      all += cost;
+      if (V * kSmallSite > limit) continue;
+      fits += cost;
+      need = std::max(need, (int)(V * kSmallSite));
+    }
+    if (fits > 0.5 * all) t.cg.smem = need;
+  }
   t.from_back = 0;
   // cluster instances with solo_sites: single blocks from the first queued chain that small
   t.solo_from = B->n;
@@ -1844,7 +1860,7 @@ int tg_batch_autotune(tg_batch* B, const tg_batch_params* p, int* best_block, do
   int best = -1;
   double bms = 1e300;
   for (int c = 0; c < kBatchNumCfgs; c++) {
-    if (batch_teams(c, B->sms) <= 0) continue;
+    if (batch_teams(c, B->sms, p->cg.precision == TG_PREC_FP64) <= 0) continue;
     double ms = 0;
     tg_batch_params q = *p;
     q.use_graph = 0;
