@@ -570,7 +570,7 @@ __device__ __noinline__ double block_reliable(const ChainCtx& ctx, const double2
 }
 
 template <bool MU0, class T>
-__device__ __noinline__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
+__device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
   const int V = c.g.V;
   OpK<float> km32{(float)c.m, (float)c.ep, (float)-c.em, MU0}, kd32{(float)c.m, (float)-c.em, (float)c.ep, MU0};
   double a = 0;
@@ -709,7 +709,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     double2 p = philox_gauss_pair(c.seed, tr, (unsigned)s, 16u);
     c.mom[s] = p;
     a_mom += p.x * p.x + p.y * p.y;
-    a_g += (1. - cos(a.x)) + (1. - cos(a.y));
+    a_g += one_minus_cos(a.x) + one_minus_cos(a.y);
     if (noise_on) c.noise[s] = philox_gauss_pair(c.seed, tr, (unsigned)s, 17u);
     c.An[s] = a;
   }
@@ -770,7 +770,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     double2 ph = c.phi[s], xv = c.x[s], p = c.mom[s], a = c.An[s];
     b_pf += ph.x * xv.x + ph.y * xv.y;
     b_mom += p.x * p.x + p.y * p.y;
-    b_g += (1. - cos(a.x)) + (1. - cos(a.y));
+    b_g += one_minus_cos(a.x) + one_minus_cos(a.y);
   }
   const double Spf1 = T::sum(b_pf), Smom1 = T::sum(b_mom), Sg1 = fac * T::sum(b_g), Smd1 = T::sum(b_md);
   const double dS = Smom1 - Smom0 + Spf1 - Spf0 + Smd1 - Smd0 + Sg1 - Sg0;  // hmc.c:729-732

@@ -8,6 +8,7 @@
 #include <math.h>
 
 #include "tg_launch.h"
+#include "tg_trig.cuh"
 
 namespace tg {
 
@@ -16,30 +17,20 @@ namespace tg {
 // eta_t(x) = (-1)^x, eta_x = 1 (hmc.c:914-921); bc_mu applies on the link that
 // leaves the last slice (hmc.c:143-148, 165-170).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void link_vals(const Geo& g, int bc_t, int bc_x, int s, double2 a, double2& wt,
-                                          double2& wx) {
+__device__ __forceinline__ void write_links(const Geo& g, int bc_t, int bc_x, int s, double2 a, const LinkOut& o) {
   int t, x;
   site_tx(g, s, t, x);
-  double ft = 0.5 * ((x & 1) ? -1.0 : 1.0) * ((t == g.nt - 1) ? (double)bc_t : 1.0);
-  double fx = 0.5 * ((x == g.nx - 1) ? (double)bc_x : 1.0);
-  double st, ct, sx, cx;
-  sincos(a.x, &st, &ct);
-  sincos(a.y, &sx, &cx);
-  wt = make_double2(ft * ct, ft * st);
-  wx = make_double2(fx * cx, fx * sx);
-}
-
-__device__ __forceinline__ void write_links(const Geo& g, int bc_t, int bc_x, int s, double2 a, const LinkOut& o) {
-  double2 wt, wx;
-  link_vals(g, bc_t, bc_x, s, a, wt, wx);
-  if (o.Wt != nullptr) {
-    o.Wt[s] = wt;
-    o.Wx[s] = wx;
-  }
-  o.Wt32[s] = make_float2((float)wt.x, (float)wt.y);
-  o.Wx32[s] = make_float2((float)wx.x, (float)wx.y);
-  o.Wtq[s] = to_fx_link(wt);
-  o.Wxq[s] = to_fx_link(wx);
+  const int ft = ((x & 1) ? -1 : 1) * ((t == g.nt - 1) ? bc_t : 1), fx = (x == g.nx - 1) ? bc_x : 1;
+  double2 w;
+  FxLink q;
+  fx_link_of(a.x, ft, w, q);
+  if (o.Wt != nullptr) o.Wt[s] = w;
+  o.Wt32[s] = make_float2((float)w.x, (float)w.y);
+  o.Wtq[s] = q;
+  fx_link_of(a.y, fx, w, q);
+  if (o.Wx != nullptr) o.Wx[s] = w;
+  o.Wx32[s] = make_float2((float)w.x, (float)w.y);
+  o.Wxq[s] = q;
 }
 
 // ---------------------------------------------------------------------------
@@ -196,10 +187,10 @@ __device__ __forceinline__ double2 philox_gauss_pair(unsigned long long seed, un
                                                      unsigned stream_id) {
   uint4 r = philox4x32(make_uint4(site, stream_id, (unsigned)tr, (unsigned)(tr >> 32)),
                        make_uint2((unsigned)seed, (unsigned)(seed >> 32)));
-  double u1 = u53(r.x, r.y), u2 = u53(r.z, r.w);
+  double u1 = u53(r.x, r.y);
   double rad = sqrt(-2.0 * log(u1));
   double sn, cs;
-  sincospi(2.0 * u2, &sn, &cs);
+  fx_sincos_turn(((unsigned long long)r.z << 21) ^ (r.w >> 11), cs, sn);  // 2 pi u53(r.z, r.w)
   return make_double2(rad * cs, rad * sn);
 }
 

@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kBlock) k_gauge_action(int n, const double2* _
   double a = 0;
   TG_SITES(s, n) {
     double2 v = A[s];
-    a += (1. - cos(v.x)) + (1. - cos(v.y));
+    a += one_minus_cos(v.x) + one_minus_cos(v.y);
   }
   double tot;
   if (grid_sum<kBlock, double>(a, red.partials, red.counter, &tot) && threadIdx.x == 0) *dst = fac * tot;
