@@ -14,6 +14,7 @@
 #include <map>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "tg_batch.h"
@@ -84,15 +85,45 @@ struct RefStream {
     if (avail == 0) twist();
     return out[--avail];
   }
-  void gauss_pairs(long n, double* dst) {  // dst[2n]
-    for (long k = 0; k < n; k++) {
-      double u1 = next(), u2 = next();
-      double r = sqrt(-2 * log(u1));
-      dst[2 * k] = r * cos(2 * M_PI * u2);
-      dst[2 * k + 1] = r * sin(2 * M_PI * u2);
+  void fill(long n, double* dst) {  // the next n uniforms
+    while (n > 0) {
+      if (avail == 0) twist();
+      const long k = n < avail ? n : avail;
+      for (long i = 0; i < k; i++) dst[i] = out[avail - 1 - i];
+      avail -= (int)k;
+      dst += k;
+      n -= k;
     }
   }
 };
+
+// Box-Muller pairs in place of n pairs of uniforms (hmc.c:423-426), by the host's
+// math library, whose results the reference's trajectories carry bit for bit:
+// 45 ns a pair against 8 for the stream, so large fields are split over threads.
+void box_muller(double* p, long n) {
+  auto some = [p](long k0, long k1) {
+    for (long k = k0; k < k1; k++) {
+      const double u1 = p[2 * k], u2 = p[2 * k + 1];
+      const double r = sqrt(-2 * log(u1));
+      p[2 * k] = r * cos(2 * M_PI * u2);
+      p[2 * k + 1] = r * sin(2 * M_PI * u2);
+    }
+  };
+  const long cores = (long)std::thread::hardware_concurrency();
+  const long parts = std::max(1L, std::min(std::min(cores, 8L), n / 4096));  // 4096 pairs: 0.2 ms
+  std::vector<std::thread> extra;
+  long begin = 0;
+  try {
+    for (long i = 0; i + 1 < parts; i++) {
+      const long end = n * (i + 1) / parts;
+      extra.emplace_back(some, begin, end);
+      begin = end;
+    }
+  } catch (const std::exception&) {  // no thread to be had: this one does the rest
+  }
+  some(begin, n);
+  for (std::thread& t : extra) t.join();
+}
 
 struct GraphEntry {
   cudaGraph_t graph = nullptr;
@@ -126,7 +157,7 @@ struct tg_lattice {
   unsigned* bar = nullptr;      // persistent solver: barrier words [kBarWords]
   double* pcg_part = nullptr;   // and its partial sums [4 * kPcgMaxGrid]
 
-  double* h_stage = nullptr;  // pinned, 2*V*kMaxPf doubles... sized at create
+  double* h_stage = nullptr;  // pinned: a trajectory's fields from the reference stream (allocated on first use)
   size_t h_stage_len = 0;
   CgState* h_st = nullptr;
   TrajStats* h_ts = nullptr;
@@ -490,18 +521,32 @@ int solver_status(int status) {
   }
 }
 
+// Copies go straight between the caller's memory and the device: on this host
+// (coherent link) 16 MB take 98-109 us from pageable memory, as from pinned, and
+// took 1150 us through a pinned buffer and memcpy.
 int upload(tg_lattice* L, void* dst, const double* src, size_t ndouble) {
-  if (ndouble > L->h_stage_len) return fail(TG_E_ARG, "field larger than staging buffer");
-  memcpy(L->h_stage, src, ndouble * sizeof(double));
-  TG_CK(cudaMemcpyAsync(dst, L->h_stage, ndouble * sizeof(double), cudaMemcpyHostToDevice, L->stream));
-  TG_CK(cudaStreamSynchronize(L->stream));  // staging buffer is reused
+  TG_CK(cudaMemcpyAsync(dst, src, ndouble * sizeof(double), cudaMemcpyHostToDevice, L->stream));
+  TG_CK(cudaStreamSynchronize(L->stream));  // the caller may reuse src
   return TG_OK;
 }
 int download(tg_lattice* L, double* dst, const void* src, size_t ndouble) {
-  if (ndouble > L->h_stage_len) return fail(TG_E_ARG, "field larger than staging buffer");
-  TG_CK(cudaMemcpyAsync(L->h_stage, src, ndouble * sizeof(double), cudaMemcpyDeviceToHost, L->stream));
+  TG_CK(cudaMemcpyAsync(dst, src, ndouble * sizeof(double), cudaMemcpyDeviceToHost, L->stream));
   TG_CK(cudaStreamSynchronize(L->stream));
-  memcpy(dst, L->h_stage, ndouble * sizeof(double));
+  return TG_OK;
+}
+
+// Pinned room for n values drawn from the reference stream.
+int ensure_stage(tg_lattice* L, size_t n) {
+  if (n <= L->h_stage_len) return TG_OK;
+  TG_CK(cudaStreamSynchronize(L->stream));
+  if (L->h_stage) cudaFreeHost(L->h_stage);
+  L->h_stage = nullptr;
+  L->h_stage_len = 0;
+  if (cudaMallocHost((void**)&L->h_stage, n * sizeof(double)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(TG_E_ALLOC, "pinned host allocation failed");
+  }
+  L->h_stage_len = n;
   return TG_OK;
 }
 
@@ -776,9 +821,7 @@ int tg_create(const tg_lattice_params* p, tg_lattice** out) {
       (rc = dmalloc(&L->pcg_part, 4 * (size_t)kPcgMaxGrid)) != TG_OK)
     return bail(rc);
   if ((rc = ensure_pf(L, 1)) != TG_OK) return bail(rc);
-  L->h_stage_len = (size_t)(kMaxPf + 2) * 2 * n;  // npf eta fields + momenta + noise
-  if (cudaMallocHost((void**)&L->h_stage, L->h_stage_len * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost((void**)&L->h_st, sizeof(CgState)) != cudaSuccess ||
+  if (cudaMallocHost((void**)&L->h_st, sizeof(CgState)) != cudaSuccess ||
       cudaMallocHost((void**)&L->h_ts, sizeof(TrajStats)) != cudaSuccess ||
       cudaMallocHost((void**)&L->h_log, sizeof(CgLog) * kMaxLog) != cudaSuccess)
     return bail(fail(TG_E_ALLOC, "pinned host allocation failed"));
@@ -1204,16 +1247,14 @@ int tg_magnetisation(tg_lattice* L, double* M) {
 int tg_fermion_phase(tg_lattice* L, int sources, const double* noise, double* phase) {
   if (!L || !phase || sources <= 0) return fail(TG_E_ARG, "bad argument");
   const size_t V = (size_t)L->V;
-  std::vector<double> draw;
-  if (!noise) {  // the reference's stream: V Gaussian pairs per source (hmc.c:802)
-    draw.resize(2 * V);
-  }
+  if (!noise) TG_TRY(ensure_stage(L, 2 * V));  // the reference's stream: V Gaussian pairs per source (hmc.c:802)
   TG_CK(cudaMemsetAsync(&L->ts->Smd1, 0, sizeof(double), L->stream));
   for (int k = 0; k < sources; k++) {
     const double* src = noise ? noise + 2 * V * k : nullptr;
     if (!noise) {
-      L->mt.gauss_pairs((long)V, draw.data());
-      src = draw.data();
+      L->mt.fill(2 * (long)V, L->h_stage);
+      box_muller(L->h_stage, (long)V);
+      src = L->h_stage;
     }
     TG_TRY(upload(L, L->vin, src, 2 * V));
     dslash64(L->stream, L->g, op_k(L, 1), 1, L->vin, L->vout, L->Wtq, L->Wxq);
@@ -1415,19 +1456,16 @@ int tg_trajectory(tg_lattice* L, const tg_hmc_params* p, tg_traj_result* r) {
   // (hmc.c:695-698), then the accept uniform (hmc.c:738)
   const size_t V = (size_t)L->V;
   TG_TRY(ensure_pf(L, p->npf > 0 ? p->npf : 1));
+  const size_t n_eta = 2 * V * p->npf, n_noise = p->stochastic_term ? 2 * V : 0;
+  TG_TRY(ensure_stage(L, n_eta + 2 * V + n_noise));
   double* h = L->h_stage;
-  size_t off = 0;
-  size_t n_eta = 2 * V * p->npf;
-  L->mt.gauss_pairs((long)V * p->npf, h);
-  off += n_eta;
-  L->mt.gauss_pairs((long)V, h + off);
-  off += 2 * V;
-  if (p->stochastic_term) L->mt.gauss_pairs((long)V, h + off);
+  L->mt.fill((long)(n_eta + 2 * V + n_noise), h);
+  box_muller(h, (long)(n_eta + 2 * V + n_noise) / 2);
   double u = L->mt.next();
   if (n_eta) TG_CK(cudaMemcpyAsync(L->eta, h, n_eta * sizeof(double), cudaMemcpyHostToDevice, L->stream));
   TG_CK(cudaMemcpyAsync(L->mom, h + n_eta, 2 * V * sizeof(double), cudaMemcpyHostToDevice, L->stream));
-  if (p->stochastic_term)
-    TG_CK(cudaMemcpyAsync(L->noise, h + n_eta + 2 * V, 2 * V * sizeof(double), cudaMemcpyHostToDevice, L->stream));
+  if (n_noise)
+    TG_CK(cudaMemcpyAsync(L->noise, h + n_eta + 2 * V, n_noise * sizeof(double), cudaMemcpyHostToDevice, L->stream));
   L->h_ts->u = u;
   TG_CK(cudaMemcpyAsync(&L->ts->u, &L->h_ts->u, sizeof(double), cudaMemcpyHostToDevice, L->stream));
   TG_CK(cudaStreamSynchronize(L->stream));
