@@ -37,7 +37,7 @@ def test_solution_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, mu, precis
     recurrences and reliable updates it shares (on a lattice of a few sites
     either restarts a CG that would have ended exactly)."""
     if precision == 0 and nt * nx > 128 * 128:
-        pytest.skip("FP64 lattices of this size run on the grid solver")
+        pytest.skip("the mixed solver's largest case")
     rng = np.random.default_rng(nt * 1000 + nx)
     A, b, m = rng.normal(0, 0.5, (nt, nx, 2)), cplx(rng, (nt, nx)), 0.3
     o = oracle_lib.Oracle(nt, nx, m, 0.5, mu, -1, 1)

@@ -793,8 +793,8 @@ int tg_create(const tg_lattice_params* p, tg_lattice** out) {
     int cap = 8 * sms;
     L->g.grid = nblocks((int)V) < cap ? nblocks((int)V) : cap;
     const char* e = getenv("TG_MARCH");
-    L->g.march = (p->nx % 32 == 0) && (p->nt % kMarchT == 0) && !(e && e[0] == '0');
-    int items = L->g.march ? (p->nx / 32) * (p->nt / kMarchT) : 0;
+    L->g.march = march_ok(p->nx) && !(e && e[0] == '0');
+    int items = L->g.march ? march_strips(p->nx) * ((p->nt + kMarchT - 1) / kMarchT) : 0;
     int mg = (items + kBlock / 32 - 1) / (kBlock / 32);
     L->g.mgrid = L->g.march ? (mg < cap ? mg : cap) : L->g.grid;
   }

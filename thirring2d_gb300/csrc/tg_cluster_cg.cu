@@ -760,9 +760,9 @@ static int ccg_max_cluster() {
 // least a row.  One site per thread in FP64, two to four in the mixed solver
 // beyond 256 sites a block, whose shorter passes gain less from more warps than the sums
 // lose (96^2 at 512 / 256 threads: FP64 7.8 / 7.7, mixed 4.0 / 3.5; 128^2 9.8 /
-// 10.3, 4.4 / 4.1).  Against the grid solver: 16^2 5.7 / 2.8, 64^2 10.9 / 7.6, 128^2
-// 11.1 (here 9.8) / 7.9 (4.1), 256^2 mixed 8.7 (7.6); the FP64 solver stops at
-// 1088 sites a block, where the two meet, the mixed one where the shared memory ends.
+// 10.3, 4.4 / 4.1).  The grid solver takes over where the two meet: FP64 (cluster /
+// grid) 96^2 7.7 / 9.2, 112^2 8.8 / 9.2, 128^2 9.8 / 9.3; mixed 128^2 4.1 / 6.3, 256x192
+// 6.5 / 7.0, 256^2 7.6 / 7.1.
 // TG_CLUSTER_CG=0 turns it off, =blocks:threads sets the shape; the overrides of
 // the grid solvers (TG_PCG_BLOCK, TG_MIXED_CG) turn it off as well.
 CcgShape ccg_shape(const Geo& g, bool mixed) {
@@ -774,7 +774,7 @@ CcgShape ccg_shape(const Geo& g, bool mixed) {
   if (e && sscanf(e, "%d:%d", &want, &threads) >= 1 && want <= 0) return none;
   // (the lattice's limits first: a large one never asks the device)
   const int blocks = std::min(std::min(want, kCcgMaxBlocks), g.nt), n = (g.V + blocks - 1) / blocks;
-  if (ccg_bytes(g, blocks, mixed) > (size_t)kCcgSmem || (!mixed && n > 1088)) return none;
+  if (ccg_bytes(g, blocks, mixed) > (size_t)kCcgSmem || n > (mixed ? 3300 : 850)) return none;
   if (blocks > ccg_max_cluster()) return none;
   const int own = mixed && n > 256 ? std::max(256, n / 4) : n;
   const int t = threads > 0 ? threads : own;

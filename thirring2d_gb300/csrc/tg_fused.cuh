@@ -31,9 +31,10 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
   const int nt = g.nt, nx = g.nx;
   const int lane = threadIdx.x & 31;
   const int x0 = xw << 5;
-  const int x = x0 + lane;
+  const int last = min(nx - x0, 32) - 1;          // the strip's last lane
+  const int x = x0 + min(lane, last);
   const int xle = (x0 == 0) ? nx - 1 : x0 - 1;    // column left of the warp
-  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;  // column right of the warp
+  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;  // column right of the warp
   auto wrap = [nt](int t) { return t < 0 ? t + nt : (t >= nt ? t - nt : t); };
   const float2 zero = make_float2(0.f, 0.f);
 
@@ -46,10 +47,10 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
                                       ld.val(t * nx + cm), Wt[s], Wt[tm * nx + c], Wx[s], Wx[t * nx + cm]);
   };
   // u = M v on one row of the warp: vc = v(t), vu = v(t+1), vd = v(t-1); the
-  // operand beyond the warp's edge pe (lanes 0 and 31) and Wx(t, x0-1) we (lane 0)
+  // operand beyond the warp's edge pe (lanes 0 and last) and Wx(t, x0-1) we (lane 0)
   auto u_row = [&](float2 vc, float2 vu, float2 vd, float2 wt, float2 wtd, float2 wx, float2 pe, float2 we) {
     float2 pr = shfl_down1<float>(vc), pl = shfl_up1<float>(vc), wl = shfl_up1<float>(wx);
-    if (lane == 31) pr = pe;
+    if (lane == last) pr = pe;
     if (lane == 0) {
       pl = pe;
       wl = we;
@@ -57,17 +58,17 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
     return dslash_vals<float, 0, MU0>(km, vc, vu, vd, pr, pl, wt, wtd, wx, wl);
   };
   // w = M^dag u on one row: uc = u(t), uu = u(t+1), ud = u(t-1); ue = u beyond
-  // the edge (lanes 0 and 31), we = Wx(t, x0-1) (lane 0)
+  // the edge (lanes 0 and last), we = Wx(t, x0-1) (lane 0)
   auto w_row = [&](float2 uc, float2 uu, float2 ud, float2 wt, float2 wtd, float2 wx, float2 ue, float2 we) {
     float2 ur = shfl_down1<float>(uc), ul = shfl_up1<float>(uc), wl = shfl_up1<float>(wx);
-    if (lane == 31) ur = ue;
+    if (lane == last) ur = ue;
     if (lane == 0) {
       ul = ue;
       wl = we;
     }
     return dslash_vals<float, 1, MU0>(kd, uc, uu, ud, ur, ul, wt, wtd, wx, wl);
   };
-  const int xe = (lane == 31) ? xre : xle;  // the edge column lanes 0 and 31 use
+  const int xe = (lane == last) ? xre : xle;  // the edge column lanes 0 and last use
 
   // ---- prologue: u(ta-1), u(ta) ----
   const int tm1 = wrap(ta - 1), tm2 = wrap(ta - 2), tp1 = wrap(ta + 1);
@@ -80,7 +81,7 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
   const float2 wx_m = Wx[tm1 * nx + x];
   float2 wx_c = Wx[ta * nx + x];
   float2 pe_m = zero, pe_c = zero, we_m = zero, we_c = zero;
-  if (lane == 0 || lane == 31) {
+  if (lane == 0 || lane == last) {
     pe_m = ld.val(tm1 * nx + xe);
     pe_c = ld.val(ta * nx + xe);
     we_m = Wx[tm1 * nx + xle];
@@ -112,13 +113,13 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
     }
 #pragma unroll
     for (int i = 0; i < kMarchT; i++) {
-      const int src = (lane == 31) ? kMarchT + i : i;
+      const int src = (lane == last) ? kMarchT + i : i;
       const float2 pe = shfl_c2<float>(er, src);
       const float2 we = shfl_c2<float>(ewl, i);
       const float2 ue = shfl_c2<float>(eu, src);
       const float2 u_n = u_row(o_n.v, on[i].v, o_c.v, wtn[i], wt_c, wxn[i], pe, we);
       const float2 w = w_row(u_c, u_n, u_m, wt_c, wt_m, wx_c, ue, we_c);
-      epi((t + i) * nx + x, w, u_c, o_c);
+      if (lane <= last) epi((t + i) * nx + x, w, u_c, o_c);
       u_m = u_c;
       u_c = u_n;
       o_c = o_n;
@@ -135,14 +136,14 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
     const Op onn = ld.own(wrap(t + 2) * nx + x);
     const float2 wtn = Wt[r1 * nx + x], wxn = Wx[r1 * nx + x];
     float2 pe = zero, we = zero, ue = zero;
-    if (lane == 0 || lane == 31) {
+    if (lane == 0 || lane == last) {
       pe = ld.val(r1 * nx + xe);
       we = Wx[r1 * nx + xle];
       ue = u_at(t, xe);
     }
     const float2 u_n = u_row(o_n.v, onn.v, o_c.v, wtn, wt_c, wxn, pe, we);
     const float2 w = w_row(u_c, u_n, u_m, wt_c, wt_m, wx_c, ue, we_c);
-    epi(t * nx + x, w, u_c, o_c);
+    if (lane <= last) epi(t * nx + x, w, u_c, o_c);
     u_m = u_c;
     u_c = u_n;
     o_c = o_n;
@@ -154,8 +155,8 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
   }
 }
 
-// M^dagger M over every site of the lattice (column-march lattices only: nx a
-// multiple of 32, nt of kMarchT), the rows split over the grid's warps.
+// M^dagger M over every site of the lattice (column-march lattices only), the rows
+// split over the grid's warps.
 template <bool MU0, class Ld, class Epi>
 __device__ __forceinline__ void stencil_mdagm(const Geo& g, const OpK<float>& km, const OpK<float>& kd, const Ld& ld,
                                               const float2* __restrict__ Wt, const float2* __restrict__ Wx, Epi& epi) {

@@ -4,8 +4,8 @@
 // warp column march of stencil_all(): a warp walks a contiguous range of rows
 // of 32 consecutive x, reusing psi(t-1), psi(t), Wt(t-1) from registers and
 // taking x neighbours from warp shuffles, with the CG vector updates and norms
-// fused into the per-site epilogue.  Lattices whose nx is not a multiple of 32 (or
-// nt of kMarchT) use one site per thread.  Streaming kernels are one site per
+// fused into the per-site epilogue.  Lattices that do not march (march_ok) use one
+// site per thread.  Streaming kernels are one site per
 // thread over the full grid.  Reductions are deterministic (fixed shuffle
 // tree per block, partials summed in index order by the last block), so
 // results do not depend on block scheduling.
@@ -113,7 +113,7 @@ template <class K> int occ_grid_smem(K kernel, int work, int smem) {
 // for the copy pipeline to reach steady state).
 bool staged_enabled(const Geo& g) {
   const char* e = getenv("TG_STAGED");
-  return g.march && e && e[0] == '1';
+  return g.march && g.nx % 32 == 0 && e && e[0] == '1';  // (bulk copies of whole 32-column rows)
 }
 
 template <typename R, int DAG, bool MU0, bool STAGED = false>

@@ -105,7 +105,7 @@ extern "C" int tg_cg_noalloc(const tg_lattice_params* p, const tg_cg_params* cp,
   g.nx = p->nx;
   g.V = p->nt * p->nx;
   g.inv_nx = 1.0f / (float)p->nx;
-  g.march = (p->nx % 32 == 0) && (p->nt % kMarchT == 0);
+  g.march = march_ok(p->nx);
   g.grid = nblocks(g.V);
   g.mgrid = g.grid;
   // carve the scratch

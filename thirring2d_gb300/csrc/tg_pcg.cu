@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgmx(PcgMxArgs a) {
 //      every load of a thread's sites issued before the first store;
 //   B  after a grid barrier, w = A r in one pass of the fused M^dag M march
 //      (tg_fused.cuh), which also forms the partials of gamma and delta.
-// Column-march lattices only (nx a multiple of 32, nt of kMarchT).
+// Column-march lattices only.
 // ---------------------------------------------------------------------------
 struct PlainOp {
   float2 v;
@@ -653,7 +653,7 @@ __device__ __forceinline__ void cgcg_update(const Geo& g, float4* __restrict__ r
                                             float4* __restrict__ s, float4* __restrict__ p, float4* __restrict__ xs,
                                             float al, float be) {
   constexpr int U = 1;
-  const int n4 = g.V >> 1;  // V is even on column-march lattices
+  const int n4 = g.V >> 1;
   const int stride = gridDim.x * blockDim.x;
   for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n4; i0 += U * stride) {
     float4 rv[U], wv[U], sv[U], pv[U], xv[U];
@@ -680,6 +680,17 @@ __device__ __forceinline__ void cgcg_update(const Geo& g, float4* __restrict__ r
         r[i] = axpy4(-al, sk, rv[u]);
       }
     }
+  }
+  if ((g.V & 1) && blockIdx.x == 0 && threadIdx.x == 0) {  // the last site of an odd number
+    const int i = g.V - 1;
+    float2 *const r2 = reinterpret_cast<float2*>(r), *const s2 = reinterpret_cast<float2*>(s),
+           *const p2 = reinterpret_cast<float2*>(p), *const x2 = reinterpret_cast<float2*>(xs);
+    const float2 rv = __ldcg(r2 + i), sk = axpy2(be, __ldcg(s2 + i), __ldcg(reinterpret_cast<const float2*>(w) + i)),
+                 pk = axpy2(be, __ldcg(p2 + i), rv);
+    s2[i] = sk;
+    p2[i] = pk;
+    x2[i] = axpy2(al, pk, __ldcg(x2 + i));
+    r2[i] = axpy2(-al, sk, rv);
   }
 }
 
@@ -922,7 +933,7 @@ cudaError_t coop_launch(K kernel, int grid, int bs, cudaStream_t s, const Args& 
 // Blocks of bs threads the stencil can use with at least `rows` rows of 32
 // columns per warp (column march) or one site per thread.
 int pcg_work(const Geo& g, int bs, int rows) {
-  return g.march ? ((g.nx >> 5) * ((g.nt + rows - 1) / rows) + bs / 32 - 1) / (bs / 32) : nblocks(g.V, bs);
+  return g.march ? (march_strips(g.nx) * ((g.nt + rows - 1) / rows) + bs / 32 - 1) / (bs / 32) : nblocks(g.V, bs);
 }
 
 int pcg_grid(const Geo& g, int resident, int bs) {
@@ -935,6 +946,14 @@ int pcg_grid(const Geo& g, int resident, int bs) {
 // fills the GPU (one 512-thread block per SM, warps beyond the lattice's rows
 // idle), so small test lattices can hold that shape to the reference's
 // outputs; TG_PCG_BLOCK=256 forces the small-lattice shape.  Unset: by size.
+// From how many sites on the persistent solvers march.  One site per thread starts
+// each pass with all its loads, a march with its first rows'; its fewer loads and
+// operations win when threads have three sites and more.  us per iteration, march /
+// site by site: FP64 256^2 13.2 / 11.9, 384^2 17.1 / 16.3, 448^2 19.4 / 20.2, 512^2
+// 21.8 / 24.5, 1000^2 60.3 / 64.3, 2048^2 167 / 266; mixed 256^2 8.3 / 7.1, 512^2 10.4 / 10.4,
+// 768^2 14.6 / 14.7, 1024^2 18.9 / 21.4, 1000^2 19.3 / 20.8.
+constexpr int kPcgMarch64 = 200000, kPcgMarchMx = 550000;
+
 int pcg_block_override() {
   const char* e = getenv("TG_PCG_BLOCK");
   if (e == nullptr) return 0;
@@ -942,13 +961,12 @@ int pcg_block_override() {
   return (v == 512 || v == 256) ? v : 0;
 }
 
-// The 512-thread kernel when its blocks fill every SM with a row per warp,
-// else the 256-thread one.  A small lattice spreads to one row per warp: its
-// passes are bound by each warp's own latency, and more blocks cost the grid
-// sums little (us per iteration at four rows / one row per warp: FP64 64^2 16.5
-// / 11.0, 128^2 17.3 / 11.1, 256^2 17.4 / 13.5; mixed 64^2 8.5 / 7.7, 256^2 9.4 /
-// 8.6; two rows lie between; blocks of 128 and 64 threads gain 0.1-0.8 us
-// up to 128^2 and lose up to 8 us from 256^2 on).  A lattice whose work fits
+// The 512-thread kernel when its blocks fill every SM with a row per warp (or a
+// site per thread), else the 256-thread one.  A marching lattice spreads to one row
+// per warp: its passes are bound by each warp's own latency, and more blocks cost
+// the grid sums little (us per iteration at four rows / one row per warp: FP64 128^2
+// 17.3 / 11.1, 256^2 17.4 / 13.5; mixed 256^2 9.4 / 8.6; blocks of 128 and 64 threads
+// lose up to 8 us from 256^2 on).  A lattice whose work fits
 // one 256-thread block at one_rows rows per warp runs the one-block instance
 // (k1; L1-cached loads, block totals kept on chip): FP32 sums gain more from
 // that than from four blocks (32^2 4.7 against 6.9 us), FP64 less (12.2, 10.1).
@@ -956,7 +974,7 @@ template <class K512, class K256, class K1, class Args>
 cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, cudaStream_t s, const Args& a,
                        int warp_smem = 0) {
   const int r512 = pcg_resident(k512, 512, 16 * warp_smem);
-  const int force = pcg_block_override();
+  const int force = pcg_block_override();  // (keeps the march: small lattices on the large ones' path)
   if (force == 512) return coop_launch(k512, std::min(r512, kPcgMaxGrid), 512, s, a, 16 * warp_smem);
   if (force == 0 && pcg_work(g, 512, 1) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a, 16 * warp_smem);
   if (one_rows > 0 && pcg_work(g, 256, one_rows) == 1) return coop_launch(k1, 1, 256, s, a);
@@ -964,6 +982,7 @@ cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, 
 }
 
 cudaError_t pcg64(cudaStream_t s, bool mu0, Pcg64Args a) {
+  if (a.g.V < kPcgMarch64 && pcg_block_override() == 0) a.g.march = 0;
   if (mu0) return pcg_launch(a.g, k_pcg64<512, true>, k_pcg64<256, true>, k_pcg64<256, true, true>, 1, s, a, kRingWarp);
   return pcg_launch(a.g, k_pcg64<512, false>, k_pcg64<256, false>, k_pcg64<256, false, true>, 1, s, a, kRingWarp);
 }
@@ -982,6 +1001,7 @@ cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, lon
 }
 
 cudaError_t pcgmx(cudaStream_t s, bool mu0, PcgMxArgs a) {
+  if (a.g.V < kPcgMarchMx && pcg_block_override() == 0) a.g.march = 0;
   if (mu0) return pcg_launch(a.g, k_pcgmx<512, true>, k_pcgmx<256, true>, k_pcgmx<256, true, true>, kMarchT, s, a);
   return pcg_launch(a.g, k_pcgmx<512, false>, k_pcgmx<256, false>, k_pcgmx<256, false, true>, kMarchT, s, a);
 }

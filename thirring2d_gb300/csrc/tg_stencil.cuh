@@ -11,22 +11,23 @@
 
 namespace tg {
 
-// One row t of a warp's FP32 march: the operator at the 32 sites (t, x0 + lane)
-// from psi(t-1) = pm, psi(t) = pc, psi(t+1) = pp and the links, with the
-// operand across the warp's edge pe (used by lanes 0 and 31) and the x link
+// One row t of a warp's FP32 march: the operator at the sites (t, x0 + lane), lane
+// <= last, from psi(t-1) = pm, psi(t) = pc, psi(t+1) = pp and the links, with the
+// operand across the warp's edge pe (used by lanes 0 and last) and the x link
 // entering column x0 we (used by lane 0).  Rotates pm, pc, wtm for row t+1.
 template <typename R, int DAG, bool MU0, class Epi>
-__device__ __forceinline__ void march_row(const OpK<R>& k, int s, int lane, C2<R>& pm, C2<R>& pc, C2<R>& wtm,
+__device__ __forceinline__ void march_row(const OpK<R>& k, int s, int lane, int last, C2<R>& pm, C2<R>& pc, C2<R>& wtm,
                                           C2<R> pp, C2<R> wt, C2<R> wx, C2<R> pe, C2<R> we, Epi& epi) {
   C2<R> pr = shfl_down1<R>(pc);
   C2<R> pl = shfl_up1<R>(pc);
   C2<R> wl = shfl_up1<R>(wx);
-  if (lane == 31) pr = pe;
+  if (lane == last) pr = pe;
   if (lane == 0) {
     pl = pe;
     wl = we;
   }
-  epi(s, dslash_vals<R, DAG, MU0>(k, pc, pp, pm, pr, pl, wt, wtm, wx, wl), pc);
+  const C2<R> o = dslash_vals<R, DAG, MU0>(k, pc, pp, pm, pr, pl, wt, wtm, wx, wl);
+  if (lane <= last) epi(s, o, pc);
   pm = pc;
   pc = pp;
   wtm = wt;
@@ -71,9 +72,10 @@ __device__ __forceinline__ void march_segment32(const Geo& g, const OpK<float>& 
   const int nx = g.nx;
   const int lane = threadIdx.x & 31;
   const int x0 = xw << 5;
-  const int x = x0 + lane;
+  const int last = min(nx - x0, 32) - 1;             // the strip's last lane
+  const int x = x0 + min(lane, last);
   const int xle = (x0 == 0) ? nx - 1 : x0 - 1;       // column left of the warp
-  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;     // column right of the warp
+  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;  // column right of the warp
   const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
   C2<R> pm = ld(tm * nx + x);
   C2<R> wtm = Wt[tm * nx + x];
@@ -93,14 +95,14 @@ __device__ __forceinline__ void march_segment32(const Geo& g, const OpK<float>& 
     }
 #pragma unroll
     for (int i = 0; i < kMarchT; i++)
-      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, pm, pc, wtm, pp[i], wt[i], wx[i],
-                             shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
+      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, last, pm, pc, wtm, pp[i], wt[i], wx[i],
+                             shfl_c2<R>(ep, (lane == last) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
   }
-  for (; t < tb; t++) {  // the last rows of the segment: lanes 0 and 31 fetch their own
-    const int xe = (lane == 31) ? xre : xle;
+  for (; t < tb; t++) {  // the last rows of the segment: lanes 0 and last fetch their own
+    const int xe = (lane == last) ? xre : xle;
     const int tp = (t + 1 == g.nt) ? 0 : t + 1;
     const int s = t * nx + x;
-    march_row<R, DAG, MU0>(k, s, lane, pm, pc, wtm, ld(tp * nx + x), Wt[s], Wx[s], ld(t * nx + xe), Wx[t * nx + xle],
+    march_row<R, DAG, MU0>(k, s, lane, last, pm, pc, wtm, ld(tp * nx + x), Wt[s], Wx[s], ld(t * nx + xe), Wx[t * nx + xle],
                            epi);
   }
 }
@@ -135,18 +137,19 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
   const int nx = g.nx;
   const int lane = threadIdx.x & 31;
   const int x0 = xw << 5;
-  const int x = x0 + lane;
+  const int last = min(nx - x0, 32) - 1;
+  const int x = x0 + min(lane, last);
   const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
-  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;
+  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;
   const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
   FxC pm = to_fx(ld(tm * nx + x));
   FxLink wtm = Wt[tm * nx + x];
   double2 own = ld(ta * nx + x);
   FxC pc = to_fx(own);
-  // row t: in(t+1) = pp, in beyond the warp's edge pe (lanes 0 and 31), the x link entering x0 we (lane 0)
+  // row t: in(t+1) = pp, in beyond the warp's edge pe (lanes 0 and last), the x link entering x0 we (lane 0)
   auto row = [&](int t, double2 pp, FxLink wt, FxLink wx, const FxC& pe, FxLink we) {
     const int s = t * nx + x;
-    const FxC pr = sel_fx(lane == 31, pe, shfl_fx(pc, lane + 1));
+    const FxC pr = sel_fx(lane == last, pe, shfl_fx(pc, lane + 1));
     const FxC pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
     FxLink wl = shfl_lk(wx, lane - 1);
     if (lane == 0) wl = we;
@@ -157,7 +160,7 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
       o = dslash_vals<double, DAG, MU0>(k, ld(s), ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), fx_link_value(wt),
                                         fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
     }
-    epi(s, o, own);
+    if (lane <= last) epi(s, o, own);
     pm = pc;
     pc = pn;
     own = pp;
@@ -188,12 +191,12 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
       }
 #pragma unroll
       for (int i = 0; i < kChunk64; i++)
-        row(t + h + i, pp[i], wt[i], wx[i], shfl_fx(ef, (lane == 31) ? kMarchT + h + i : h + i), shfl_lk(ew, h + i));
+        row(t + h + i, pp[i], wt[i], wx[i], shfl_fx(ef, (lane == last) ? kMarchT + h + i : h + i), shfl_lk(ew, h + i));
     }
   }
   for (; t < tb; t++) {
     const int tp = (t + 1 == g.nt) ? 0 : t + 1;
-    row(t, ld(tp * nx + x), Wt[t * nx + x], Wx[t * nx + x], to_fx(ld(t * nx + ((lane == 31) ? xre : xle))),
+    row(t, ld(tp * nx + x), Wt[t * nx + x], Wx[t * nx + x], to_fx(ld(t * nx + ((lane == last) ? xre : xle))),
         Wx[t * nx + xle]);
   }
 }
@@ -230,9 +233,9 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
   constexpr int NA = NS + 2 + NE, EL = 2 * kMarchT;
   const int nx = g.nx, n = tb - ta;
   const int lane = threadIdx.x & 31;
-  const int x0 = xw << 5, x = x0 + lane;
+  const int x0 = xw << 5, last = min(nx - x0, 32) - 1, x = x0 + min(lane, last);
   const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
-  const int xre = (x0 + 32 == nx) ? 0 : x0 + 32;
+  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;
   double2* const rows = reinterpret_cast<double2*>(ring) + lane;
   double2* const edges = reinterpret_cast<double2*>(ring + D * NA * 512) + (lane & (EL - 1));
   const unsigned rows_a = smem_addr(rows), edges_a = smem_addr(edges);
@@ -297,8 +300,8 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
       const FxLink wt = *reinterpret_cast<const FxLink*>(rw + NS * 32);
       const FxLink wx = *reinterpret_cast<const FxLink*>(rw + (NS + 1) * 32);
       const double2 pp = comb(v);
-      const FxC pe = shfl_fx(ef, (lane == 31) ? kMarchT + ic : ic);
-      const FxC pr = sel_fx(lane == 31, pe, shfl_fx(pc, lane + 1));
+      const FxC pe = shfl_fx(ef, (lane == last) ? kMarchT + ic : ic);
+      const FxC pr = sel_fx(lane == last, pe, shfl_fx(pc, lane + 1));
       const FxC pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
       const FxLink we = shfl_lk(ew, ic);
       FxLink wl = shfl_lk(wx, lane - 1);
@@ -311,7 +314,7 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
         o = dslash_vals<double, DAG, MU0>(k, own, at(nb.tp), at(nb.tm), at(nb.xp), at(nb.xm), fx_link_value(wt),
                                           fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
       }
-      epi(s, o, own, rw + (NS + 2) * 32);
+      if (lane <= last) epi(s, o, own, rw + (NS + 2) * 32);
       pm = pc;
       pc = pn;
       own = pp;
@@ -334,7 +337,7 @@ __device__ __forceinline__ void march_segment(const Geo& g, const OpK<R>& k, Ld&
 // f(xw, ta, tb) for each strip segment of this warp's range.
 template <class F> __device__ __forceinline__ void for_warp_rows(const Geo& g, F&& f) {
   const int wpb = (int)(blockDim.x >> 5);
-  const long long rows = (long long)(g.nx >> 5) * g.nt;
+  const long long rows = (long long)march_strips(g.nx) * g.nt;
   const long long nw = (long long)gridDim.x * wpb;
   const long long gw = (long long)blockIdx.x * wpb + (threadIdx.x >> 5);
   long long r = rows * gw / nw;
@@ -377,15 +380,14 @@ __device__ __forceinline__ void stencil_all(const Geo& g, const OpK<R>& k, const
 // batched-chain kernel: one block, or the blocks of a cluster).  T gives the
 // block's rank in the team and the team's size.  The team's warps split the
 // lattice's (strip, t) rows into one contiguous range each, as for_warp_rows
-// splits them over a grid; lattices whose nx is not a multiple of 32 go one
-// site per thread.
+// splits them over a grid; lattices that do not march go one site per thread.
 template <class T, typename R, int DAG, bool MU0, class Ld, class Epi>
 __device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& ld, const Lk<R>* __restrict__ Wt,
                                              const Lk<R>* __restrict__ Wx, Epi& epi) {
   const int wpb = blockDim.x >> 5;
-  if ((g.nx & 31) == 0) {
+  if (march_ok(g.nx)) {
     const int nw = T::nblocks() * wpb, w = T::rank() * wpb + (threadIdx.x >> 5);
-    const int rows = (g.nx >> 5) * g.nt;
+    const int rows = march_strips(g.nx) * g.nt;
     int r = (int)((long long)rows * w / nw);
     const int r1 = (int)((long long)rows * (w + 1) / nw);
     while (r < r1) {
@@ -409,7 +411,7 @@ __device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& 
 // Blocks of work of a stencil kernel (march: at least one row per warp, so that
 // a small lattice spreads over more SMs).
 inline int stencil_work(const Geo& g) {
-  return g.march ? ((g.nx >> 5) * g.nt + kBlock / 32 - 1) / (kBlock / 32) : nblocks(g.V);
+  return g.march ? (march_strips(g.nx) * g.nt + kBlock / 32 - 1) / (kBlock / 32) : nblocks(g.V);
 }
 
 // ---------------------------------------------------------------------------
@@ -554,7 +556,7 @@ __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>&
       C2<R> v[Src::n];
 #pragma unroll
       for (int j = 0; j < Src::n; j++) v[j] = sv[(j * kMarchT + i) * 32 + lane];
-      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, pm, pc, wtm, src.combine(v),
+      march_row<R, DAG, MU0>(k, (t + i) * nx + x, lane, 31, pm, pc, wtm, src.combine(v),
                                    sv[(Src::n * kMarchT + i) * 32 + lane], sv[((Src::n + 1) * kMarchT + i) * 32 + lane],
                                    shfl_c2<R>(ep, (lane == 31) ? kMarchT + i : i), shfl_c2<R>(ew, i), epi);
     }
@@ -568,7 +570,7 @@ __device__ __forceinline__ void march_segment_staged(const Geo& g, const OpK<R>&
     const int tp = (t + 1 == g.nt) ? 0 : t + 1;
     const int s = t * nx + x;
     const int xe = (lane == 31) ? xre : xle;
-    march_row<R, DAG, MU0>(k, s, lane, pm, pc, wtm, src(tp * nx + x), Wt[s], Wx[s], src(t * nx + xe),
+    march_row<R, DAG, MU0>(k, s, lane, 31, pm, pc, wtm, src(tp * nx + x), Wt[s], Wx[s], src(t * nx + xe),
                                  Wx[t * nx + xle], epi);
   }
 }
