@@ -125,3 +125,17 @@ def test_grid_solver_on_small_lattices(tg, oracle_lib, monkeypatch, nt, nx, prec
     """The grid solver stays what runs when the cluster one is turned off."""
     monkeypatch.setenv("TG_CLUSTER_CG", "0")
     test_solution_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, 0.0, precision)
+
+
+@pytest.mark.parametrize("scale", [1e-8, 3e-9, 1e-9, 3e-10])
+def test_mixed_residuals_whose_squares_are_denormal(tg, oracle_lib, scale):
+    """r^2 per site falls below 2^-126 in FP32 near the end of the solve."""
+    nt, nx, m = 24, 40, 0.3
+    rng = np.random.default_rng(2)
+    A, b = rng.normal(0, 0.5, (nt, nx, 2)), cplx(rng, (nt, nx)) * scale
+    o = oracle_lib.Oracle(nt, nx, m, 0.5, 0.0, -1, 1)
+    with tg.Lattice(nt, nx, m, 0.5, 0.0, -1, 1) as L:
+        L.set_gauge(A)
+        x, res = L.fmdm_invert_cg(b, tg.cg_params(rel_tol=1e-11, abs_tol2=0, precision=1))
+    assert res.status == 0
+    assert np.linalg.norm(b - o.Mdag(A, o.M(A, x))) <= 1.5e-11 * np.linalg.norm(b)

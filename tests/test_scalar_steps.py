@@ -126,3 +126,14 @@ def test_sums_that_are_refused(harness, kind):
         v = np.ones(32)
         v[7] = bad
         assert harness(np.array([kind, 32, last, 0.0]).tobytes() + v.tobytes())[0, 1] == 0
+
+
+@pytest.mark.parametrize("scale", [1e-37, 1e-38, 1e-40, 1e-43])
+def test_integer_sums_of_denormal_floats(harness, scale):
+    """FP32 terms below 2^-126 are whole multiples of 2^-149 and keep their value: the
+    bound of test_integer_sums at growth 1."""
+    rng = np.random.default_rng(3)
+    v = (rng.exponential(size=500) * scale).astype(np.float32).astype(np.float64)
+    exact = sum(Fraction(float(x)) for x in v)
+    t, ok = harness(np.array([2, len(v), float(exact), 0.0]).tobytes() + v.tobytes())[0]
+    assert ok and abs(Fraction(float(t)) - exact) <= exact * (Fraction(len(v), 2 ** 61) + Fraction(1, 2 ** 51))

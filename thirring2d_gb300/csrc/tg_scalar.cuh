@@ -81,10 +81,10 @@ TG_HD FxTerm fx_term(float v, int ref) {
   union { float f; unsigned u; } b;
   b.f = v;
   const int e = (int)((b.u >> 23) & 0xffu);
-  const int sh = e + 934 - ref;
-  // zero and denormal terms count as 0
-  const unsigned long long m = e == 0 ? 0ull : (unsigned long long)((b.u & 0x7fffffu) | 0x800000u);
-  return fx_split(fx_shift(m, sh), ref == 0 || e == 255 || (e != 0 && sh > 39));
+  // a denormal has exponent 1 and no leading one (a sum of r^2 in FP32 may lie below 2^-126)
+  const int sh = (e == 0 ? 1 : e) + 934 - ref;
+  const unsigned long long m = (unsigned long long)((b.u & 0x7fffffu) | (e == 0 ? 0u : 0x800000u));
+  return fx_split(fx_shift(m, sh), ref == 0 || e == 255 || (sh > 39 && (m >> (sh < 63 ? 63 - sh : 0)) != 0));
 }
 // The total as FP64 from its three limbs: low + mid 2^26 + top 2^52 (low, mid < 2^32).
 TG_HD bool fx_total_value(unsigned low, unsigned mid, unsigned top, int ref, double& total) {
