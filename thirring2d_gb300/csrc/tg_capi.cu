@@ -311,10 +311,13 @@ bool use_single_reduction(const tg_lattice* L) {
 int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const double2* b, double2* x, int log_index) {
   const Links lk = links(L);
   const GridBar bar{L->bar, reinterpret_cast<unsigned long long*>(L->bar + 2)};
-  const CcgShape small = ccg_shape(L->g, cp.precision == TG_PREC_MIXED);
+  const bool mixed = cp.precision == TG_PREC_MIXED;
+  CcgShape small = ccg_shape(L->g, mixed);
+  const CcgShape middle = gcg_shape(L->g, mixed, small);
+  if (middle.blocks > 0) small.blocks = 0;
   if (small.blocks == 0) TG_CK(cudaMemsetAsync(L->bar, 0, kBarWords * sizeof(unsigned), s));
   cudaError_t e;
-  if (cp.precision == TG_PREC_MIXED) {
+  if (mixed) {
     PcgMxArgs a{};
     a.g = L->g;
     a.km32 = op_k32(L, 0);
@@ -344,6 +347,8 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.ru_interval = cp.ru_interval;
     if (small.blocks > 0) {
       e = ccgmx(s, L->P.mu == 0.0, a, small);
+    } else if (middle.blocks > 0) {
+      e = gcgmx(s, L->P.mu == 0.0, a, middle);
     } else if (use_single_reduction(L)) {
       a.w0 = L->wmx.Mps;
       a.s0 = L->wmx.ss;
@@ -372,7 +377,9 @@ int enqueue_pcg(tg_lattice* L, cudaStream_t s, const tg_cg_params& cp, const dou
     a.rel_tol = cp.rel_tol;
     a.abs_tol2 = cp.abs_tol2;
     a.maxiter = cp.maxiter;
-    e = small.blocks > 0 ? ccg64(s, L->P.mu == 0.0, a, small) : pcg64(s, L->P.mu == 0.0, a);
+    if (small.blocks > 0) e = ccg64(s, L->P.mu == 0.0, a, small);
+    else if (middle.blocks > 0) e = gcg64(s, L->P.mu == 0.0, a, middle);
+    else e = pcg64(s, L->P.mu == 0.0, a);
   }
   if (e != cudaSuccess) return fail(TG_E_CUDA, std::string("persistent CG launch: ") + cudaGetErrorString(e));
   return TG_OK;

@@ -38,35 +38,14 @@
 #include <mutex>
 #include <unordered_map>
 
-#include "tg_device.cuh"
-#include "tg_scalar.cuh"
+#include "tg_onchip.cuh"
 
 namespace tg {
 
 namespace cg = cooperative_groups;
 
-constexpr int kCcgThreads = 512;               // most site threads of a block (one more warp does the scalars)
 constexpr int kCcgMaxBlocks = 16;              // largest cluster
-constexpr int kCcgSmem = 224 * 1024;           // dynamic shared memory a block may use
 constexpr int kCcgPart = kCcgMaxBlocks * (kCcgThreads / 32 + 1);
-
-// The block's share of the lattice.
-struct CcgPart {
-  int nblocks, c, b0, n;  // own sites b0 .. b0 + n - 1
-  int prev, next, nprev;  // the neighbouring blocks, the previous one's site count
-};
-__device__ __forceinline__ CcgPart ccg_part(int V) {
-  CcgPart p;
-  p.nblocks = (int)gridDim.x;
-  p.c = (int)blockIdx.x;
-  auto at = [&](int c) { return (int)((long long)V * c / p.nblocks); };
-  p.b0 = at(p.c);
-  p.n = at(p.c + 1) - p.b0;
-  p.prev = p.c == 0 ? p.nblocks - 1 : p.c - 1;
-  p.next = p.c == p.nblocks - 1 ? 0 : p.c + 1;
-  p.nprev = at(p.prev + 1) - at(p.prev);
-  return p;
-}
 
 template <typename T> __device__ __forceinline__ T* ccg_remote(T* p, int block) {
   return cg::this_cluster().map_shared_rank(p, (unsigned)block);
@@ -145,12 +124,6 @@ __device__ __forceinline__ void ccg_bar_wait(unsigned bar, unsigned parity, int*
   *fail = 1;
 }
 
-template <typename T> __device__ __forceinline__ T ccg_warp_allsum(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // The cluster's total of the threads' partials in FP64 (fixed order), handed to
 // f, which runs in thread 0 of every block; every thread gets f's result.  The
 // cluster barrier also orders every store made before the call.  `part` holds
@@ -193,83 +166,6 @@ __device__ __forceinline__ void ccg_leave(bool failed) {
   const int k = failed ? 8 : 1;
   for (int i = 0; i < k; i++) cg::this_cluster().sync();
 }
-
-__device__ __forceinline__ void ccg_report(CgState* st, CgLog* log, int log_index, double rr, double rr0, double stop,
-                                           int iter, int n_ru, int status) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  st->rr = rr;
-  st->rr0 = rr0;
-  st->rr_true = rr;
-  st->stop = stop;
-  st->iter = iter;
-  st->n_ru = n_ru;
-  st->status = status;
-  st->done = 1;
-  st->need_ru = 0;
-  st->restart = 0;
-  st->log_index = log_index;
-  if (log != nullptr && log_index >= 0) {
-    CgLog& l = log[log_index];
-    l.iter = iter;
-    l.status = status;
-    l.n_ru = n_ru;
-    l.rr = rr;
-    l.rr0 = rr0;
-  }
-}
-
-__device__ __forceinline__ double ccg_stop(double rr0, double rel_tol, double abs_tol2) {
-  double stop = abs_tol2;
-  if (rel_tol > 0 && rel_tol * rel_tol * rr0 > stop) stop = rel_tol * rel_tol * rr0;
-  return stop;
-}
-
-// Offsets from a site to its x neighbours in the t-major order.
-__device__ __forceinline__ void ccg_x_offsets(const Geo& g, int s, int& xp, int& xm) {
-  int t, x;
-  site_tx(g, s, t, x);
-  xp = (x == g.nx - 1) ? 1 - g.nx : 1;
-  xm = (x == 0) ? g.nx - 1 : -1;
-}
-
-// Block-floating operands (tg_fixed.cuh) in shared memory.
-struct FxArr {
-  longlong2* m;
-  int* e;
-  __device__ __forceinline__ FxC get(int i) const {
-    const longlong2 v = m[i];
-    return FxC{v.x, v.y, e[i]};
-  }
-};
-
-template <int DAG, bool MU0>
-__device__ __forceinline__ double2 ccg_op64(const OpK<double>& k, const FxArr& v, const FxLink* wt, const FxLink* wx,
-                                            int j, int nx, int xp, int xm) {
-  const FxC c = v.get(j), tu = v.get(j + nx), td = v.get(j - nx), xu = v.get(j + xp), xd = v.get(j + xm);
-  const FxLink a = wt[j], b = wt[j - nx], p = wx[j], q = wx[j + xm];
-  double2 o;
-  if (!fx_dslash<DAG, MU0>(k, c, tu, td, xu, xd, a, b, p, q, o))
-    o = dslash_vals<double, DAG, MU0>(k, fx_value(c), fx_value(tu), fx_value(td), fx_value(xu), fx_value(xd),
-                                      fx_link_value(a), fx_link_value(b), fx_link_value(p), fx_link_value(q));
-  return o;
-}
-
-// bytes of shared memory per window site and per own site
-constexpr int kCcg64Window = 6 * 16 + 2 * 4, kCcg64Own = 16;
-constexpr int kCcg32Window = 5 * 8, kCcg32Own = 8;
-
-// What the scalar warp hands to the block after the sums: the first sum's step
-// length, the second's beta and verdict (FP64: a status or -1 to go on; mixed:
-// whether a reliable update is due), and the scales of the next sums.
-struct CcgScalars {
-  double alpha, beta;
-  float af, bf;
-  int okA, refA, okB, refB, verdict, fail;
-  double rr, rn;  // |r|^2 before and after the iteration, for a sum that is taken again
-};
-
-// The bits of a non-negative double, which compare as it does (NaN above all).
-__device__ __forceinline__ long long ord(double v) { return __double_as_longlong(v); }
 
 // FP64: the iteration of k_pcg64
 template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_ccg64(Pcg64Args a, int wmax, int nmax) {
@@ -461,13 +357,6 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_ccg
   ccg_leave(status == TG_E_TIMEOUT);
   for (int i = tid; i < n; i += blockDim.x) a.x[P.b0 + i] = x[i];
   ccg_report(a.st, a.log, a.log_index, iter > 0 ? sc.rn : rr, rr0, stop, iter, 0, status);
-}
-
-template <int DAG, bool MU0>
-__device__ __forceinline__ float2 ccg_op32(const OpK<float>& k, const float2* v, const float2* wt, const float2* wx,
-                                           int j, int nx, int xp, int xm) {
-  return dslash_vals<float, DAG, MU0>(k, v[j], v[j + nx], v[j - nx], v[j + xp], v[j + xm], wt[j], wt[j - nx], wx[j],
-                                      wx[j + xm]);
 }
 
 // Mixed: the iteration and the FP64 reliable update of k_pcgmx.  The FP64 x, its

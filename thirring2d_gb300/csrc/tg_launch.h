@@ -177,6 +177,11 @@ struct CcgShape {
 CcgShape ccg_shape(const Geo& g, bool mixed);
 cudaError_t ccg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& sh);
 cudaError_t ccgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh);
+// The same on the whole grid's shared memory (tg_grid_cg.cu), for middle sizes;
+// cluster: ccg_shape's answer.
+CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster);
+cudaError_t gcg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& sh);
+cudaError_t gcgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh);
 // one grid barrier (4 blocks, cooperative) that also waits for `phantom` absent
 // blocks, giving up after `limit` polls: *status = TG_OK or TG_E_TIMEOUT
 cudaError_t barrier_check(cudaStream_t s, unsigned* count, unsigned phantom, long long limit, int* status);
