@@ -53,8 +53,18 @@ def test_shapes_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, shape, mu, p
     solve(tg, oracle_lib, nt, nx, 0.3, mu, precision)
 
 
+@pytest.mark.parametrize("nt,nx,shape,mu", [
+    (2, 64, "1:32:1", 0.0), (3, 6, "1:480:1", 0.2), (2, 2, "1:32:1", 0.0), (16, 16, "3:32:1", 0.2), (12, 200, "37:64:1", 0.2), (33, 24, "5:96:1", 0.0),
+    (100, 60, "7:256:1", 0.0), (64, 64, "4:480:1", 0.2), (96, 100, "3:480:1", 0.0), (131, 190, "152:480:1", 0.2)])
+def test_links_from_global_memory_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, shape, mu):
+    monkeypatch.setenv("TG_CLUSTER_CG", "0")
+    monkeypatch.setenv("TG_GRID_CG", shape)
+    solve(tg, oracle_lib, nt, nx, 0.3, mu, 1)
+
+
 @pytest.mark.parametrize("nt,nx,mu,precision", [(128, 256, 0.0, 0), (131, 190, 0.2, 0), (256, 256, 0.2, 0), (400, 400, 0.0, 0),
-                                                (256, 300, 0.0, 1), (512, 512, 0.2, 1), (700, 701, 0.0, 1)])
+                                                (256, 300, 0.0, 1), (512, 512, 0.2, 1), (700, 701, 0.0, 1),
+                                                (1001, 902, 0.2, 1), (1024, 1024, 0.0, 1)])
 def test_middle_sizes_against_oracle(tg, oracle_lib, nt, nx, mu, precision):
     solve(tg, oracle_lib, nt, nx, 0.3, mu, precision)
 

@@ -15,6 +15,8 @@
 // the window's upkeep (at 256^2 a block keeps 431 sites and 512 neighbours) and the
 // operator's integer instructions.  us per iteration before and after: FP64 128^2 9.3 -> 6.3, 256^2
 // 12.1 -> 8.7, 400^2 19.9 -> 13.5; mixed 256^2 7.2 -> 6.3, 512^2 10.4 -> 8.1, 700^2 13.3 -> 9.8.
+// Mixed lattices whose links no longer fit keep p, M p and r on chip and stream the
+// links from L2, ahead of their use: 800^2 15.1 -> 12.0, 1000^2 19.5 -> 15.3, 1024^2 18.9 -> 16.1.
 //
 // The barrier's wait is bounded as in tg_pcg.cu: a block that gives up ends the solve with
 // TG_E_TIMEOUT, and every other one times out at its next barrier.
@@ -24,6 +26,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "tg_gridbar.cuh"
@@ -314,13 +317,35 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
 }
 
 // Mixed: the iteration and the FP64 reliable update of k_pcgmx.  The FP64 x, its
-// image M x and the FP64 links stay in global memory.
-template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
+// image M x and the FP64 links stay in global memory.  STREAM: the FP32 links and xs
+// do too, for lattices of which only p, M p and r fit; a thread takes two sites of a row
+// at a time (nx is even) and has its next kGcgAhead pairs' links in registers, at a
+// pass's end those of the next pass.  Single sites, four ahead, took 18.3 us at 1000^2
+// (pairs: 15.3) and no gain at 1024^2; 448, 416, 384 or 320 site threads 15.7, 15.6, 16.0, 17.1.
+constexpr int kGcgAhead = 2;
+constexpr int kGcgStreamThreads = 480;  // with the scalar warp 16 warps: 128 registers instead of 96
+struct GcgLinks {
+  float4 t, td, x;  // of the pair: to t+1, from t-1, to x+1
+  float2 xl;        // from x-1 into the first
+};
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ float4 pair_of(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
+__device__ __forceinline__ float4& as4(float2* p) { return *reinterpret_cast<float4*>(p); }
+__device__ __forceinline__ float4 as4(const float2* p) { return *reinterpret_cast<const float4*>(p); }
+
+template <bool MU0, bool STREAM>
+__global__ void __launch_bounds__(STREAM ? kGcgStreamThreads + 32 : kCcgThreads + 32, 1)
+k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
   extern __shared__ __align__(16) unsigned char gcg_smem[];
   __shared__ CcgScalars sc;
   __shared__ longlong2 warp_part[kCcgThreads / 32];
   const Geo& g = a.g;
-  const CcgPart P = ccg_part(g.V);
+  CcgPart P = ccg_part(STREAM ? g.V / 2 : g.V);
+  if (STREAM) {
+    P.b0 *= 2;
+    P.n *= 2;
+  }
   const int nx = g.nx, n = P.n, win = n + 2 * nx, T = blockDim.x - 32, tid = threadIdx.x, nb = gridDim.x;
   const bool site = tid < T;  // else: the scalar warp
   const GcgExchange ex{a.bar, warp_part, &sc.fail, T};
@@ -333,7 +358,8 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
   float2* r = q + wmax;
   float2* wt = r + wmax;
   float2* wx = wt + wmax;
-  float2* xs = wx + wmax;
+  float2* const xs = STREAM ? a.xs + P.b0 : wx + wmax;
+  constexpr int U = STREAM ? kGcgAhead : 1;
 
   if (tid == T) {
     barrier_epoch() = 0;
@@ -347,16 +373,21 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
     const float2 rb = make_float2((float)bb.x, (float)bb.y);
     r[j] = rb;
     p[j] = rb;
-    wt[j] = a.Wt32[s];
-    wx[j] = a.Wx32[s];
+    if (!STREAM) {
+      wt[j] = a.Wt32[s];
+      wx[j] = a.Wx32[s];
+    }
     if (j >= nx && j < nx + n) {
-      xs[j - nx] = make_float2(0.f, 0.f);
+      if (!STREAM) xs[j - nx] = make_float2(0.f, 0.f);
       v = fma(bb.x, bb.x, v);
       v = fma(bb.y, bb.y, v);
     }
   }
   if (site)
-    for (int i = tid; i < n; i += T) a.x[P.b0 + i] = make_double2(0.0, 0.0);
+    for (int i = tid; i < n; i += T) {
+      a.x[P.b0 + i] = make_double2(0.0, 0.0);
+      if (STREAM) xs[i] = make_float2(0.f, 0.f);
+    }
   double rr = ex.sum64(v, part0);
   const double rr0 = rr, stop = ccg_stop(rr0, a.rel_tol, a.abs_tol2), limit = 1e10 * rr0;
   double drop = kRuDrop * rr;  // |r|^2 below which a reliable update is due
@@ -375,40 +406,121 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
     xm = xm0;
     if (i != tid) ccg_x_offsets(g, P.b0 + i, xp, xm);
   };
+  // STREAM: the links of the pair at site i
+  auto links = [&](int i) {
+    const int s = P.b0 + i;
+    int xp, xm;
+    ccg_x_offsets(g, s, xp, xm);
+    return GcgLinks{__ldg(reinterpret_cast<const float4*>(a.Wt32 + s)),
+                    __ldg(reinterpret_cast<const float4*>(a.Wt32 + (s < nx ? s - nx + g.V : s - nx))),
+                    __ldg(reinterpret_cast<const float4*>(a.Wx32 + s)), __ldg(a.Wx32 + s + xm)};
+  };
+  GcgLinks w[U];
+  if (STREAM && site) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (2 * (tid + u * T) < n) w[u] = links(2 * (tid + u * T));
+  }
+  // f(i, u) for the thread's pairs; w[u] holds the links of the pair at i
+  auto pairs = [&](auto f) {
+    for (int i0 = 2 * tid; i0 < n; i0 += 2 * U * T) {
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + 2 * u * T;
+        if (i < n) {
+          f(i, u);
+          w[u] = links(i + 2 * U * T < n ? i + 2 * U * T : 2 * (tid + u * T));
+        }
+      }
+    }
+  };
+  auto op2 = [&](auto dag, const OpK<float>& k, const float2* v, int i, const GcgLinks& l) {
+    int t, x;
+    site_tx(g, P.b0 + i, t, x);
+    const int j = nx + i, jl = x == 0 ? j + nx - 1 : j - 1, jr = x + 2 == nx ? j + 2 - nx : j + 2;
+    const float4 c = as4(v + j), tu = as4(v + j + nx), td = as4(v + j - nx);
+    const float2 left = v[jl], right = v[jr];
+    return pair_of(dslash_vals<float, decltype(dag)::value, MU0>(k, lo2(c), lo2(tu), lo2(td), hi2(c), left, lo2(l.t),
+                                                                 lo2(l.td), lo2(l.x), l.xl),
+                   dslash_vals<float, decltype(dag)::value, MU0>(k, hi2(c), hi2(tu), hi2(td), right, lo2(c), hi2(l.t),
+                                                                 hi2(l.td), hi2(l.x), lo2(l.x)));
+  };
+  auto halo = [&](float2* v, const float2* src) {
+    if constexpr (STREAM) {
+      for (int h = 2 * tid; h < 2 * nx; h += 2 * T) {
+        const int j = h < nx ? h : n + h;
+        int s = P.b0 - nx + j;
+        s += (s < 0) ? g.V : (s >= g.V ? -g.V : 0);
+        as4(v + j) = __ldcg(reinterpret_cast<const float4*>(src + s));
+      }
+    } else {
+      gcg_halo(P, nx, g.V, T, [&](int j, int s) { v[j] = __ldcg(src + s); });
+    }
+  };
+  float4 xa[U];  // STREAM: xs of the thread's next U pairs
   float bf = 0.f;
   while (status < 0) {
     double inv_rr = 0;
     if (site) {
-      for (int j = tid; j < win; j += T) {
-        const float2 rv = r[j], pv = p[j];
-        p[j] = make_float2(fmaf(bf, pv.x, rv.x), fmaf(bf, pv.y, rv.y));
+      if constexpr (STREAM) {
+        for (int j = 2 * tid; j < win; j += 2 * T) {
+          const float4 rv = as4(r + j), pv = as4(p + j);
+          as4(p + j) = make_float4(fmaf(bf, pv.x, rv.x), fmaf(bf, pv.y, rv.y), fmaf(bf, pv.z, rv.z), fmaf(bf, pv.w, rv.w));
+        }
+      } else {
+        for (int j = tid; j < win; j += T) {
+          const float2 rv = r[j], pv = p[j];
+          p[j] = make_float2(fmaf(bf, pv.x, rv.x), fmaf(bf, pv.y, rv.y));
+        }
       }
       ex.sites_sync();
     } else {
       inv_rr = 1.0 / rr;
     }
     float va = 0;
-    if (site)
-      for (int i = tid; i < n; i += T) {
-        int xp, xm;
-        offsets(i, xp, xm);
-        const float2 o = ccg_op32<0, MU0>(a.km32, p, wt, wx, nx + i, nx, xp, xm);
-        va = fmaf(o.x, o.x, va);
-        va = fmaf(o.y, o.y, va);
-        q[nx + i] = o;
-        if (gcg_edge(P, nx, i)) a.Mp[P.b0 + i] = o;
+    if (site) {
+      if constexpr (STREAM) {
+        pairs([&](int i, int u) {
+          const float4 o = op2(std::integral_constant<int, 0>{}, a.km32, p, i, w[u]);
+          va = fmaf(o.x, o.x, va);
+          va = fmaf(o.y, o.y, va);
+          va = fmaf(o.z, o.z, va);
+          va = fmaf(o.w, o.w, va);
+          as4(q + nx + i) = o;
+          if (gcg_edge(P, nx, i)) as4(a.Mp + P.b0 + i) = o;
+        });
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (2 * (tid + u * T) < n) xa[u] = as4(xs + 2 * (tid + u * T));
+      } else {
+        for (int i = tid; i < n; i += T) {
+          int xp, xm;
+          offsets(i, xp, xm);
+          const float2 o = ccg_op32<0, MU0>(a.km32, p, wt, wx, nx + i, nx, xp, xm);
+          va = fmaf(o.x, o.x, va);
+          va = fmaf(o.y, o.y, va);
+          q[nx + i] = o;
+          if (gcg_edge(P, nx, i)) a.Mp[P.b0 + i] = o;
+        }
       }
+    }
     ex.post(va, refA, postA);
     auto apply = [&](int i) {
       int xp, xm;
       offsets(i, xp, xm);
       return ccg_op32<1, MU0>(a.kd32, q, wt, wx, nx + i, nx, xp, xm);
     };
+    auto apply2 = [&](int i, int u) { return op2(std::integral_constant<int, 1>{}, a.kd32, q, i, w[u]); };
+    float4 ap2 = make_float4(0.f, 0.f, 0.f, 0.f);  // STREAM: of the thread's first pair
     float2 ap = make_float2(0.f, 0.f);  // the thread's first site, before alpha is known
     if (site) {
-      gcg_halo(P, nx, g.V, T, [&](int j, int s) { q[j] = __ldcg(a.Mp + s); });
+      halo(q, a.Mp);
       ex.sites_sync();
-      if (tid < n) ap = apply(tid);
+      if constexpr (STREAM) {
+        if (2 * tid < n) ap2 = apply2(2 * tid, 0);
+      } else if (tid < n) {
+        ap = apply(tid);
+      }
     } else {
       double pap;
       const bool ok = ex.total(postA, refA, pap);
@@ -432,24 +544,49 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
       break;
     }
     float vb = 0;
-    if (site)
-      for (int i = tid; i < n; i += T) {
-        if (i != tid) ap = apply(i);
-        float2 xv = xs[i], rv = r[nx + i];
-        const float2 pv = p[nx + i];
-        rv.x = fmaf(-af, ap.x, rv.x);
-        rv.y = fmaf(-af, ap.y, rv.y);
-        r[nx + i] = rv;
-        if (gcg_edge(P, nx, i)) a.r[P.b0 + i] = rv;
-        vb = fmaf(rv.x, rv.x, vb);
-        vb = fmaf(rv.y, rv.y, vb);
-        xv.x = fmaf(af, pv.x, xv.x);
-        xv.y = fmaf(af, pv.y, xv.y);
-        xs[i] = xv;
+    if (site) {
+      if constexpr (STREAM) {
+        pairs([&](int i, int u) {
+          if (i != 2 * tid) ap2 = apply2(i, u);
+          float4 xv = xa[u], rv = as4(r + nx + i);
+          const float4 pv = as4(p + nx + i);
+          rv.x = fmaf(-af, ap2.x, rv.x);
+          rv.y = fmaf(-af, ap2.y, rv.y);
+          rv.z = fmaf(-af, ap2.z, rv.z);
+          rv.w = fmaf(-af, ap2.w, rv.w);
+          as4(r + nx + i) = rv;
+          if (gcg_edge(P, nx, i)) as4(a.r + P.b0 + i) = rv;
+          vb = fmaf(rv.x, rv.x, vb);
+          vb = fmaf(rv.y, rv.y, vb);
+          vb = fmaf(rv.z, rv.z, vb);
+          vb = fmaf(rv.w, rv.w, vb);
+          xv.x = fmaf(af, pv.x, xv.x);
+          xv.y = fmaf(af, pv.y, xv.y);
+          xv.z = fmaf(af, pv.z, xv.z);
+          xv.w = fmaf(af, pv.w, xv.w);
+          as4(xs + i) = xv;
+          if (i + 2 * U * T < n) xa[u] = as4(xs + i + 2 * U * T);
+        });
+      } else {
+        for (int i = tid; i < n; i += T) {
+          if (i != tid) ap = apply(i);
+          float2 xv = xs[i], rv = r[nx + i];
+          const float2 pv = p[nx + i];
+          rv.x = fmaf(-af, ap.x, rv.x);
+          rv.y = fmaf(-af, ap.y, rv.y);
+          r[nx + i] = rv;
+          if (gcg_edge(P, nx, i)) a.r[P.b0 + i] = rv;
+          vb = fmaf(rv.x, rv.x, vb);
+          vb = fmaf(rv.y, rv.y, vb);
+          xv.x = fmaf(af, pv.x, xv.x);
+          xv.y = fmaf(af, pv.y, xv.y);
+          xs[i] = xv;
+        }
       }
+    }
     ex.post(vb, refB, postB);
     if (site) {
-      gcg_halo(P, nx, g.V, T, [&](int j, int s) { r[j] = __ldcg(a.r + s); });
+      halo(r, a.r);
     } else {
       double rn;
       const bool ok = ex.total(postB, refB, rn);
@@ -521,7 +658,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
       status = TG_E_TIMEOUT;
       break;
     }
-    if (site) gcg_halo(P, nx, g.V, T, [&](int j, int s) { r[j] = __ldcg(a.r + s); });
+    if (site) halo(r, a.r);
     __syncthreads();
     if (rt > kRuRestart * rr) bf = 0.f;  // the recursive residual was far too optimistic: restart p from r
     drop = kRuDrop * rt;
@@ -539,8 +676,13 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
 // ---------------------------------------------------------------------------
 // Launch
 // ---------------------------------------------------------------------------
-static size_t gcg_bytes(const Geo& g, int nblocks, bool mixed) {
-  const size_t nmax = (g.V + nblocks - 1) / nblocks, win = nmax + 2 * (size_t)g.nx;
+// sites of the largest block
+static int gcg_most_sites(int V, int nblocks, bool stream) {
+  return stream ? (V / 2 + nblocks - 1) / nblocks * 2 : (V + nblocks - 1) / nblocks;
+}
+static size_t gcg_bytes(const Geo& g, int nblocks, bool mixed, bool stream) {
+  const size_t nmax = gcg_most_sites(g.V, nblocks, stream), win = nmax + 2 * (size_t)g.nx;
+  if (stream) return win * 3 * sizeof(float2);
   return win * (mixed ? kCcg32Window : kCcg64Window) + nmax * (mixed ? kCcg32Own : kCcg64Own);
 }
 
@@ -555,12 +697,14 @@ static int gcg_resident() {
   auto it = cache.find(dev);
   if (it != cache.end()) return it->second;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
-  const void* kernels[] = {(const void*)k_gcg64<true>, (const void*)k_gcg64<false>, (const void*)k_gcgmx<true>,
-                           (const void*)k_gcgmx<false>};
+  const void* kernels[] = {(const void*)k_gcg64<true>,         (const void*)k_gcg64<false>,
+                           (const void*)k_gcgmx<true, false>,  (const void*)k_gcgmx<false, false>,
+                           (const void*)k_gcgmx<true, true>,   (const void*)k_gcgmx<false, true>};
   for (const void* k : kernels) {
     int n = 0;
+    const int threads = k == kernels[4] || k == kernels[5] ? kGcgStreamThreads : kCcgThreads;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCcgSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kCcgThreads + 32, kCcgSmem) != cudaSuccess || n < 1)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads + 32, kCcgSmem) != cudaSuccess || n < 1)
       sms = 0;
   }
   (void)cudaGetLastError();
@@ -577,7 +721,9 @@ static int gcg_resident() {
 // In FP64 a cluster of 16 blocks is faster while each of its threads has one site
 // (512 a block), mixed up to 2400 sites a block.  Beyond, this solver takes what its
 // shared memory holds: about 170 000 sites in FP64 and 650 000 mixed, less the
-// window.  Mixed lattices whose rows span more than three blocks lose to the
+// window; mixed lattices of even rows up to about 1.1 million sites stream their links
+// (this solver / the grid solver: 600x1300 14.0 / 17.3, 3000x300 13.8 / 18.9, 10000x80 12.7 / 17.3,
+// 250x2600 15.0 / 15.8, 1056x1040 16.7 / 20.1).  Mixed lattices whose rows span more than three blocks lose to the
 // window's upkeep (40x1500 7.4 / - / 7.2, 20x2000 7.2 / - / 6.6; 50x1000 7.0 / - / 7.2).
 // One block per SM: half of them cost 8.7 -> 11.3 at 256^2.  Threads: a site each, and
 // no fewer than half the window (16x1000 12.0 -> 8.9 with 544 instead of 128); 256 or 384
@@ -585,11 +731,11 @@ static int gcg_resident() {
 constexpr int kGcgSites64 = 512, kGcgSitesMx = 2400;
 
 CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
-  const CcgShape none{0, 0};
+  const CcgShape none{0, 0, 0};
   if (getenv("TG_PCG_BLOCK") != nullptr || getenv("TG_MIXED_CG") != nullptr) return none;
   const char *e = getenv("TG_GRID_CG"), *cl = getenv("TG_CLUSTER_CG");
-  int want = 1 << 20, threads = 0;
-  if (e && sscanf(e, "%d:%d", &want, &threads) >= 1 && want <= 0) return none;
+  int want = 1 << 20, threads = 0, stream = 0;
+  if (e && sscanf(e, "%d:%d:%d", &want, &threads, &stream) >= 1 && want <= 0) return none;
   if (cluster.blocks > 0) {
     const int n = (g.V + cluster.blocks - 1) / cluster.blocks;
     if (cl || n <= (mixed ? kGcgSitesMx : kGcgSites64)) return none;
@@ -600,19 +746,22 @@ CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
   if (sms <= 0) return none;
   const int blocks = std::max(1, std::min(std::min(want, sms), g.V / 64));
   const int n = (g.V + blocks - 1) / blocks;
-  if (gcg_bytes(g, blocks, mixed) > (size_t)kCcgSmem) return none;
+  if (mixed && gcg_bytes(g, blocks, true, false) > (size_t)kCcgSmem) stream = 1;
+  if (!mixed) stream = 0;
+  if (stream && g.nx % 2 != 0) return none;
+  if (gcg_bytes(g, blocks, mixed, stream != 0) > (size_t)kCcgSmem) return none;
   if (!e && mixed && g.nx > 3 * n) return none;
-  const int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx);
-  return CcgShape{blocks, std::min(kCcgThreads, (t + 31) / 32 * 32)};
+  const int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx) / (stream ? 2 : 1);
+  return CcgShape{blocks, std::min(stream ? kGcgStreamThreads : kCcgThreads, (t + 31) / 32 * 32), stream};
 }
 
 template <class K, class Args>
 static cudaError_t gcg_launch(K kernel, cudaStream_t s, const Args& a, bool mixed, const CcgShape& sh) {
-  const int nmax = (a.g.V + sh.blocks - 1) / sh.blocks;
+  const int nmax = gcg_most_sites(a.g.V, sh.blocks, sh.stream != 0);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)sh.blocks);
   cfg.blockDim = dim3((unsigned)sh.threads + 32);  // and the scalar warp
-  cfg.dynamicSmemBytes = gcg_bytes(a.g, sh.blocks, mixed);
+  cfg.dynamicSmemBytes = gcg_bytes(a.g, sh.blocks, mixed, sh.stream != 0);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -626,7 +775,9 @@ cudaError_t gcg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& 
   return mu0 ? gcg_launch(k_gcg64<true>, s, a, false, sh) : gcg_launch(k_gcg64<false>, s, a, false, sh);
 }
 cudaError_t gcgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh) {
-  return mu0 ? gcg_launch(k_gcgmx<true>, s, a, true, sh) : gcg_launch(k_gcgmx<false>, s, a, true, sh);
+  if (sh.stream)
+    return mu0 ? gcg_launch(k_gcgmx<true, true>, s, a, true, sh) : gcg_launch(k_gcgmx<false, true>, s, a, true, sh);
+  return mu0 ? gcg_launch(k_gcgmx<true, false>, s, a, true, sh) : gcg_launch(k_gcgmx<false, false>, s, a, true, sh);
 }
 
 }  // namespace tg
