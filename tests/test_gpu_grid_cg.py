@@ -62,6 +62,15 @@ def test_links_from_global_memory_against_oracle(tg, oracle_lib, monkeypatch, nt
     solve(tg, oracle_lib, nt, nx, 0.3, mu, 1)
 
 
+@pytest.mark.parametrize("nt,nx,shape,mu", [
+    (2, 64, "1:32:2", 0.0), (2, 2, "1:32:2", 0.0), (12, 200, "37:64:2", 0.2), (33, 24, "5:96:2", 0.0), (100, 60, "7:256:2", 0.0),
+    (64, 64, "4:512:2", 0.2), (131, 190, "152:512:2", 0.2)])
+def test_pairs_of_sites_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, shape, mu):
+    monkeypatch.setenv("TG_CLUSTER_CG", "0")
+    monkeypatch.setenv("TG_GRID_CG", shape)
+    solve(tg, oracle_lib, nt, nx, 0.3, mu, 1)
+
+
 @pytest.mark.parametrize("nt,nx,mu,precision", [(128, 256, 0.0, 0), (131, 190, 0.2, 0), (256, 256, 0.2, 0), (400, 400, 0.0, 0),
                                                 (256, 300, 0.0, 1), (512, 512, 0.2, 1), (700, 701, 0.0, 1),
                                                 (1001, 902, 0.2, 1), (1024, 1024, 0.0, 1)])

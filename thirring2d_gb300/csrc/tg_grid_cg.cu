@@ -14,7 +14,7 @@
 // Bound: two grid barriers and sums, about 2.5 us of the 6.3 us at 128^2; above,
 // the window's upkeep (at 256^2 a block keeps 431 sites and 512 neighbours) and the
 // operator's integer instructions.  us per iteration before and after: FP64 128^2 9.3 -> 6.3, 256^2
-// 12.1 -> 8.7, 400^2 19.9 -> 13.5; mixed 256^2 7.2 -> 6.3, 512^2 10.4 -> 8.1, 700^2 13.3 -> 9.8.
+// 12.1 -> 8.7, 400^2 19.9 -> 13.5; mixed 256^2 7.2 -> 6.1, 512^2 10.4 -> 7.8, 700^2 13.7 -> 9.8.
 // Mixed lattices whose links no longer fit keep p, M p and r on chip and stream the
 // links from L2, ahead of their use: 800^2 15.1 -> 12.0, 1000^2 19.5 -> 15.3, 1024^2 18.9 -> 16.1.
 //
@@ -317,11 +317,17 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
 }
 
 // Mixed: the iteration and the FP64 reliable update of k_pcgmx.  The FP64 x, its
-// image M x and the FP64 links stay in global memory.  STREAM: the FP32 links and xs
-// do too, for lattices of which only p, M p and r fit; a thread takes two sites of a row
-// at a time (nx is even) and has its next kGcgAhead pairs' links in registers, at a
-// pass's end those of the next pass.  Single sites, four ahead, took 18.3 us at 1000^2
-// (pairs: 15.3) and no gain at 1024^2; 448, 416, 384 or 320 site threads 15.7, 15.6, 16.0, 17.1.
+// image M x and the FP64 links stay in global memory.  FORM:
+//   kGcgSites   one site of a thread at a time
+//   kGcgPairs   two sites of a row (nx is even), with half the loads: us per iteration
+//               228^2 6.4 -> 6.1, 256^2 6.6 -> 6.1, 400^2 7.7 -> 7.3, 512^2 8.3 -> 7.8,
+//               700^2 10.1 -> 9.8, 1000x200 7.5 -> 7.4, 50x1000 7.2 -> 6.7
+//   kGcgStream  pairs, with the FP32 links and xs in global memory, for lattices of
+//               which only p, M p and r fit; a thread has its next kGcgAhead pairs'
+//               links in registers, at a pass's end those of the next pass.
+//               Single sites, four ahead, took 18.3 us at 1000^2 (pairs: 15.3) and gained nothing
+//               at 1024^2; 448, 416, 384 or 320 site threads 15.7, 15.6, 16.0, 17.1.
+constexpr int kGcgSites = 0, kGcgStream = 1, kGcgPairs = 2;
 constexpr int kGcgAhead = 2;
 constexpr int kGcgStreamThreads = 480;  // with the scalar warp 16 warps: 128 registers instead of 96
 struct GcgLinks {
@@ -334,15 +340,16 @@ __device__ __forceinline__ float4 pair_of(float2 a, float2 b) { return make_floa
 __device__ __forceinline__ float4& as4(float2* p) { return *reinterpret_cast<float4*>(p); }
 __device__ __forceinline__ float4 as4(const float2* p) { return *reinterpret_cast<const float4*>(p); }
 
-template <bool MU0, bool STREAM>
-__global__ void __launch_bounds__(STREAM ? kGcgStreamThreads + 32 : kCcgThreads + 32, 1)
+template <bool MU0, int FORM>
+__global__ void __launch_bounds__(FORM == kGcgStream ? kGcgStreamThreads + 32 : kCcgThreads + 32, 1)
 k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
   extern __shared__ __align__(16) unsigned char gcg_smem[];
   __shared__ CcgScalars sc;
   __shared__ longlong2 warp_part[kCcgThreads / 32];
   const Geo& g = a.g;
-  CcgPart P = ccg_part(STREAM ? g.V / 2 : g.V);
-  if (STREAM) {
+  constexpr bool STREAM = FORM == kGcgStream, PAIRS = FORM != kGcgSites;
+  CcgPart P = ccg_part(PAIRS ? g.V / 2 : g.V);
+  if (PAIRS) {
     P.b0 *= 2;
     P.n *= 2;
   }
@@ -429,24 +436,25 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
         const int i = i0 + 2 * u * T;
         if (i < n) {
           f(i, u);
-          w[u] = links(i + 2 * U * T < n ? i + 2 * U * T : 2 * (tid + u * T));
+          if (STREAM) w[u] = links(i + 2 * U * T < n ? i + 2 * U * T : 2 * (tid + u * T));
         }
       }
     }
   };
-  auto op2 = [&](auto dag, const OpK<float>& k, const float2* v, int i, const GcgLinks& l) {
+  auto op2 = [&](auto dag, const OpK<float>& k, const float2* v, int i, int u) {
     int t, x;
     site_tx(g, P.b0 + i, t, x);
     const int j = nx + i, jl = x == 0 ? j + nx - 1 : j - 1, jr = x + 2 == nx ? j + 2 - nx : j + 2;
     const float4 c = as4(v + j), tu = as4(v + j + nx), td = as4(v + j - nx);
     const float2 left = v[jl], right = v[jr];
+    const GcgLinks l = STREAM ? w[u] : GcgLinks{as4(wt + j), as4(wt + j - nx), as4(wx + j), wx[jl]};
     return pair_of(dslash_vals<float, decltype(dag)::value, MU0>(k, lo2(c), lo2(tu), lo2(td), hi2(c), left, lo2(l.t),
                                                                  lo2(l.td), lo2(l.x), l.xl),
                    dslash_vals<float, decltype(dag)::value, MU0>(k, hi2(c), hi2(tu), hi2(td), right, lo2(c), hi2(l.t),
                                                                  hi2(l.td), hi2(l.x), lo2(l.x)));
   };
   auto halo = [&](float2* v, const float2* src) {
-    if constexpr (STREAM) {
+    if constexpr (PAIRS) {
       for (int h = 2 * tid; h < 2 * nx; h += 2 * T) {
         const int j = h < nx ? h : n + h;
         int s = P.b0 - nx + j;
@@ -462,7 +470,7 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
   while (status < 0) {
     double inv_rr = 0;
     if (site) {
-      if constexpr (STREAM) {
+      if constexpr (PAIRS) {
         for (int j = 2 * tid; j < win; j += 2 * T) {
           const float4 rv = as4(r + j), pv = as4(p + j);
           as4(p + j) = make_float4(fmaf(bf, pv.x, rv.x), fmaf(bf, pv.y, rv.y), fmaf(bf, pv.z, rv.z), fmaf(bf, pv.w, rv.w));
@@ -479,9 +487,9 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
     }
     float va = 0;
     if (site) {
-      if constexpr (STREAM) {
+      if constexpr (PAIRS) {
         pairs([&](int i, int u) {
-          const float4 o = op2(std::integral_constant<int, 0>{}, a.km32, p, i, w[u]);
+          const float4 o = op2(std::integral_constant<int, 0>{}, a.km32, p, i, u);
           va = fmaf(o.x, o.x, va);
           va = fmaf(o.y, o.y, va);
           va = fmaf(o.z, o.z, va);
@@ -491,7 +499,7 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
         });
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (2 * (tid + u * T) < n) xa[u] = as4(xs + 2 * (tid + u * T));
+          if (STREAM && 2 * (tid + u * T) < n) xa[u] = as4(xs + 2 * (tid + u * T));
       } else {
         for (int i = tid; i < n; i += T) {
           int xp, xm;
@@ -510,13 +518,13 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
       offsets(i, xp, xm);
       return ccg_op32<1, MU0>(a.kd32, q, wt, wx, nx + i, nx, xp, xm);
     };
-    auto apply2 = [&](int i, int u) { return op2(std::integral_constant<int, 1>{}, a.kd32, q, i, w[u]); };
-    float4 ap2 = make_float4(0.f, 0.f, 0.f, 0.f);  // STREAM: of the thread's first pair
+    auto apply2 = [&](int i, int u) { return op2(std::integral_constant<int, 1>{}, a.kd32, q, i, u); };
+    float4 ap2 = make_float4(0.f, 0.f, 0.f, 0.f);  // of the thread's first pair
     float2 ap = make_float2(0.f, 0.f);  // the thread's first site, before alpha is known
     if (site) {
       halo(q, a.Mp);
       ex.sites_sync();
-      if constexpr (STREAM) {
+      if constexpr (PAIRS) {
         if (2 * tid < n) ap2 = apply2(2 * tid, 0);
       } else if (tid < n) {
         ap = apply(tid);
@@ -545,10 +553,10 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
     }
     float vb = 0;
     if (site) {
-      if constexpr (STREAM) {
+      if constexpr (PAIRS) {
         pairs([&](int i, int u) {
           if (i != 2 * tid) ap2 = apply2(i, u);
-          float4 xv = xa[u], rv = as4(r + nx + i);
+          float4 xv = STREAM ? xa[u] : as4(xs + i), rv = as4(r + nx + i);
           const float4 pv = as4(p + nx + i);
           rv.x = fmaf(-af, ap2.x, rv.x);
           rv.y = fmaf(-af, ap2.y, rv.y);
@@ -565,7 +573,7 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
           xv.z = fmaf(af, pv.z, xv.z);
           xv.w = fmaf(af, pv.w, xv.w);
           as4(xs + i) = xv;
-          if (i + 2 * U * T < n) xa[u] = as4(xs + i + 2 * U * T);
+          if (STREAM && i + 2 * U * T < n) xa[u] = as4(xs + i + 2 * U * T);
         });
       } else {
         for (int i = tid; i < n; i += T) {
@@ -677,12 +685,12 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
 // Launch
 // ---------------------------------------------------------------------------
 // sites of the largest block
-static int gcg_most_sites(int V, int nblocks, bool stream) {
-  return stream ? (V / 2 + nblocks - 1) / nblocks * 2 : (V + nblocks - 1) / nblocks;
+static int gcg_most_sites(int V, int nblocks, int form) {
+  return form != kGcgSites ? (V / 2 + nblocks - 1) / nblocks * 2 : (V + nblocks - 1) / nblocks;
 }
-static size_t gcg_bytes(const Geo& g, int nblocks, bool mixed, bool stream) {
-  const size_t nmax = gcg_most_sites(g.V, nblocks, stream), win = nmax + 2 * (size_t)g.nx;
-  if (stream) return win * 3 * sizeof(float2);
+static size_t gcg_bytes(const Geo& g, int nblocks, bool mixed, int form) {
+  const size_t nmax = gcg_most_sites(g.V, nblocks, form), win = nmax + 2 * (size_t)g.nx;
+  if (form == kGcgStream) return win * 3 * sizeof(float2);
   return win * (mixed ? kCcg32Window : kCcg64Window) + nmax * (mixed ? kCcg32Own : kCcg64Own);
 }
 
@@ -698,11 +706,12 @@ static int gcg_resident() {
   if (it != cache.end()) return it->second;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
   const void* kernels[] = {(const void*)k_gcg64<true>,         (const void*)k_gcg64<false>,
-                           (const void*)k_gcgmx<true, false>,  (const void*)k_gcgmx<false, false>,
-                           (const void*)k_gcgmx<true, true>,   (const void*)k_gcgmx<false, true>};
+                           (const void*)k_gcgmx<true, kGcgSites>,  (const void*)k_gcgmx<false, kGcgSites>,
+                           (const void*)k_gcgmx<true, kGcgPairs>,  (const void*)k_gcgmx<false, kGcgPairs>,
+                           (const void*)k_gcgmx<true, kGcgStream>, (const void*)k_gcgmx<false, kGcgStream>};
   for (const void* k : kernels) {
     int n = 0;
-    const int threads = k == kernels[4] || k == kernels[5] ? kGcgStreamThreads : kCcgThreads;
+    const int threads = k == kernels[6] || k == kernels[7] ? kGcgStreamThreads : kCcgThreads;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCcgSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads + 32, kCcgSmem) != cudaSuccess || n < 1)
       sms = 0;
@@ -717,7 +726,7 @@ static int gcg_resident() {
 //   FP64   64^2 5.8 / 4.3 / 9.3   90^2 6.2 / 6.3 / 9.3   128^2 6.3 / - / 9.3
 //          256^2 8.7 / - / 12.1   400^2 13.5 / - / 19.9  16x1000 8.9 / - / 9.3
 //   mixed  128^2 5.6 / 4.1 / 6.3  190^2 6.0 / 5.9 / 6.5  228^2 6.1 / 6.8 / 7.0
-//          256^2 6.3 / - / 7.2    512^2 8.1 / - / 10.4   700^2 9.8 / - / 13.3
+//          256^2 6.1 / - / 7.2    512^2 7.8 / - / 10.4   700^2 9.8 / - / 13.7
 // In FP64 a cluster of 16 blocks is faster while each of its threads has one site
 // (512 a block), mixed up to 2400 sites a block.  Beyond, this solver takes what its
 // shared memory holds: about 170 000 sites in FP64 and 650 000 mixed, less the
@@ -734,8 +743,8 @@ CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
   const CcgShape none{0, 0, 0};
   if (getenv("TG_PCG_BLOCK") != nullptr || getenv("TG_MIXED_CG") != nullptr) return none;
   const char *e = getenv("TG_GRID_CG"), *cl = getenv("TG_CLUSTER_CG");
-  int want = 1 << 20, threads = 0, stream = 0;
-  if (e && sscanf(e, "%d:%d:%d", &want, &threads, &stream) >= 1 && want <= 0) return none;
+  int want = 1 << 20, threads = 0, form = e ? kGcgSites : kGcgPairs;
+  if (e && sscanf(e, "%d:%d:%d", &want, &threads, &form) >= 1 && want <= 0) return none;
   if (cluster.blocks > 0) {
     const int n = (g.V + cluster.blocks - 1) / cluster.blocks;
     if (cl || n <= (mixed ? kGcgSitesMx : kGcgSites64)) return none;
@@ -746,22 +755,22 @@ CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
   if (sms <= 0) return none;
   const int blocks = std::max(1, std::min(std::min(want, sms), g.V / 64));
   const int n = (g.V + blocks - 1) / blocks;
-  if (mixed && gcg_bytes(g, blocks, true, false) > (size_t)kCcgSmem) stream = 1;
-  if (!mixed) stream = 0;
-  if (stream && g.nx % 2 != 0) return none;
-  if (gcg_bytes(g, blocks, mixed, stream != 0) > (size_t)kCcgSmem) return none;
+  if (!mixed || (form == kGcgPairs && g.nx % 2 != 0)) form = kGcgSites;
+  if (mixed && gcg_bytes(g, blocks, true, form) > (size_t)kCcgSmem) form = kGcgStream;
+  if (form == kGcgStream && g.nx % 2 != 0) return none;
+  if (gcg_bytes(g, blocks, mixed, form) > (size_t)kCcgSmem) return none;
   if (!e && mixed && g.nx > 3 * n) return none;
-  const int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx) / (stream ? 2 : 1);
-  return CcgShape{blocks, std::min(stream ? kGcgStreamThreads : kCcgThreads, (t + 31) / 32 * 32), stream};
+  const int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx) / (form != kGcgSites ? 2 : 1);
+  return CcgShape{blocks, std::min(form == kGcgStream ? kGcgStreamThreads : kCcgThreads, (t + 31) / 32 * 32), form};
 }
 
 template <class K, class Args>
 static cudaError_t gcg_launch(K kernel, cudaStream_t s, const Args& a, bool mixed, const CcgShape& sh) {
-  const int nmax = gcg_most_sites(a.g.V, sh.blocks, sh.stream != 0);
+  const int nmax = gcg_most_sites(a.g.V, sh.blocks, sh.form);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)sh.blocks);
   cfg.blockDim = dim3((unsigned)sh.threads + 32);  // and the scalar warp
-  cfg.dynamicSmemBytes = gcg_bytes(a.g, sh.blocks, mixed, sh.stream != 0);
+  cfg.dynamicSmemBytes = gcg_bytes(a.g, sh.blocks, mixed, sh.form);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -775,9 +784,14 @@ cudaError_t gcg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& 
   return mu0 ? gcg_launch(k_gcg64<true>, s, a, false, sh) : gcg_launch(k_gcg64<false>, s, a, false, sh);
 }
 cudaError_t gcgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh) {
-  if (sh.stream)
-    return mu0 ? gcg_launch(k_gcgmx<true, true>, s, a, true, sh) : gcg_launch(k_gcgmx<false, true>, s, a, true, sh);
-  return mu0 ? gcg_launch(k_gcgmx<true, false>, s, a, true, sh) : gcg_launch(k_gcgmx<false, false>, s, a, true, sh);
+  switch (sh.form) {
+    case kGcgStream:
+      return mu0 ? gcg_launch(k_gcgmx<true, kGcgStream>, s, a, true, sh) : gcg_launch(k_gcgmx<false, kGcgStream>, s, a, true, sh);
+    case kGcgPairs:
+      return mu0 ? gcg_launch(k_gcgmx<true, kGcgPairs>, s, a, true, sh) : gcg_launch(k_gcgmx<false, kGcgPairs>, s, a, true, sh);
+    default:
+      return mu0 ? gcg_launch(k_gcgmx<true, kGcgSites>, s, a, true, sh) : gcg_launch(k_gcgmx<false, kGcgSites>, s, a, true, sh);
+  }
 }
 
 }  // namespace tg
