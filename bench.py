@@ -67,7 +67,7 @@ def peaks():
 # DRAM bytes (read + write) of one FP64 CG iteration of the persistent solver
 # (k_pcg64, 100 iterations in one launch) at 1024^2, from one ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum over the launch / 100).
-CG_ITER_DRAM_BYTES = 116.4e6
+CG_ITER_DRAM_BYTES = 102.4e6
 # FP64 work of one CG iteration per site, in flops (FMA = 2): two operator
 # applies (16 FMA + 2 MUL each), p' = r + beta p, x/r updates, two norms.
 CG_ITER_FP64_FLOPS_PER_SITE = 2 * 34 + 4 + 8 + 4 + 4
@@ -546,15 +546,16 @@ def run_ours(args, ws, rank, local):
                      "ms_per_iteration": t_iter_ms,
                      "traffic": CG_ITER_DRAM_BYTES,
                      "traffic_source": "ncu, one capture of k_pcg64 at 1024^2, DRAM read + write per iteration",
-                     "note": "the FP64 CG is bound by the FP64 pipe, not HBM: at 88 flops per 208 B "
-                             "and the measured FP64 rate, the pipe caps this HBM fraction at "
-                             f"{fp64_peak_for_cap(hbm):.2f}; fp64_alu.frac is the fraction of the measured "
-                             "FP64 FMA rate; dslash.at_2048.fp32_frac is the HBM-bound FP32 stencil's"},
+                     "note": "the FP64 operator runs on the integer pipes; an iteration is bound by instruction "
+                             "latency at 16 warps per SM (issue 42%, FP64 pipe 50%, ncu), not HBM; an operator "
+                             "on the FP64 pipe alone would cap this HBM fraction at "
+                             f"{fp64_peak_for_cap(hbm):.2f}; dslash.at_2048.fp32_frac is the HBM-bound FP32 stencil's"},
         "fp64_alu": {"achieved_tflops": fp64_achieved, "peak_tflops": fp64_peak, "peak_source": fp64_peak_kind,
                      "frac": fp64_achieved / fp64_peak, "flops_per_site": CG_ITER_FP64_FLOPS_PER_SITE,
                      "issue_rate_tflops": issue_tflops, "frac_of_issue_rate": fp64_achieved / issue_tflops,
                      "issue_rate_source": "2 DFMA per SM per clock x SMs x the sampled maximum SM clock",
-                     "note": "the FP64 CG keeps the FP64 pipe busy most of the time (ncu); it is FP64-ALU-bound"},
+                     "note": "the reference's FP64 operation count over time; above the pipe's rate because the "
+                             "operator's products are integer limb products (ncu: FP64 pipe 50% busy)"},
         "dslash": {"fp64_gbs": dslash_gbs, "fp64_ms_M": t_M, "fp64_ms_Mdag": t_Md, "fp64_frac": dslash_gbs / hbm,
                    "fp32_gbs": dslash32_gbs, "fp32_ms": t_M32, "bytes_per_site_fp64": 64, "bytes_per_site_fp32": 32,
                    "at_2048": dict(dslash_2048, fp64_frac=dslash_2048["fp64_gbs"] / hbm,

@@ -21,9 +21,9 @@
 // than it does to FP64 addition, and the result is a function of the site's
 // operands alone: every path that computes a site returns the same bits.
 //
-// Measured on GB300: the FP64 apply at 1024^2 32 -> 24.5 us and at 2048^2 135 ->
-// 84 us, the FP64 CG iteration at 1024^2 86.8 -> 58.7 us; error against exact
-// arithmetic 1.1e-16 relative (FP64 FMA order: 1.4e-16).
+// Measured on GB300: the FP64 apply at 1024^2 32 -> 18.8 us and at 2048^2 135 ->
+// 78.5 us, the FP64 CG iteration at 1024^2 86.8 -> 58.7 us (52.5 with the rows
+// prefetched, tg_stencil.cuh); error against exact arithmetic 1.1e-16 relative (FP64 FMA order: 1.4e-16).
 //
 // Exponents outside [kFxEmin, kFxEmax] (operands all zero, denormal, huge, Inf
 // or NaN), operator constants that are not finite, and links that are not
