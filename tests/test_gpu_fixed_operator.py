@@ -73,3 +73,25 @@ def test_gauge_field_that_is_not_finite(tg):
                 assert np.array_equal(np.isnan(out), bad)
             x, res = L.fmdm_invert_cg(psi)
             assert res.status == tg.native.TG_E_NAN
+
+
+@pytest.mark.parametrize("nt,nx,mu", [(8, 32, 0.0), (6, 10, 0.0), (40, 70, 0.2), (64, 64, 0.0)])
+@pytest.mark.parametrize("value", [1.0, 0.0, -0.0, 1e-310])
+def test_vectors_that_are_zero_but_for_one_site(tg, oracle_lib, nt, nx, mu, value):
+    """M and M^dagger of a point source: the five sites it reaches, to rounding (18 of 2^-53
+    and the integer form's 5, of the value; denormals have steps of 2^-1074 instead), and zeros;
+    the solve's residual meets the tolerance 1e-11 (and rounding) where there is one."""
+    rng = np.random.default_rng(7)
+    A = rng.normal(0, 0.7, (nt, nx, 2))
+    psi = np.zeros((nt, nx), complex)
+    psi[nt // 2, nx - 1] = complex(value, 0.0)
+    o = oracle_lib.Oracle(nt, nx, 0.3, 0.5, mu, -1, 1)
+    with tg.Lattice(nt, nx, 0.3, 0.5, mu, -1, 1) as L:
+        L.set_gauge(A)
+        for got, want in ((L.fm_mul(psi), o.M(A, psi)), (L.fm_conjugate_mul(psi), o.Mdag(A, psi))):
+            assert np.array_equal(got == 0, want == 0)
+            assert np.abs(got - want).max() <= 50 * 2.0 ** -53 * abs(value) + 20 * 2.0 ** -1074
+        if value == 1.0:
+            x, res = L.fmdm_invert_cg(psi, tg.cg_params(rel_tol=1e-11, abs_tol2=0))
+            assert res.status == 0
+            assert np.linalg.norm(psi - o.Mdag(A, o.M(A, x))) <= 1.5e-11

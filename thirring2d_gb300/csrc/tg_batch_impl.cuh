@@ -489,8 +489,7 @@ __device__ __noinline__ CgOut block_cg64_small(const ChainCtx& ctx, const BatchC
       double2 o;
       if (!fx_dslash<0, MU0>(c.km, get(pm, pe, s), get(pm, pe, n.tp), get(pm, pe, n.tm), get(pm, pe, n.xp),
                              get(pm, pe, n.xm), wt, wtd, wx, wxd, o))
-        o = dslash_vals<double, 0, MU0>(c.km, p[s], p[n.tp], p[n.tm], p[n.xp], p[n.xm], fx_link_value(wt),
-                                        fx_link_value(wtd), fx_link_value(wx), fx_link_value(wxd));
+        o = dslash_wide<0, MU0>(c.km, p[s], p[n.tp], p[n.tm], p[n.xp], p[n.xm], wt, wtd, wx, wxd);
       const FxC f = to_fx(o);
       qm[s] = make_longlong2(f.re, f.im);
       qe[s] = f.e;
@@ -508,10 +507,9 @@ __device__ __noinline__ CgOut block_cg64_small(const ChainCtx& ctx, const BatchC
       double2 o;
       if (!fx_dslash<1, MU0>(c.kd, get(qm, qe, s), get(qm, qe, n.tp), get(qm, qe, n.tm), get(qm, qe, n.xp),
                              get(qm, qe, n.xm), wt, wtd, wx, wxd, o))
-        o = dslash_vals<double, 1, MU0>(c.kd, fx_value(get(qm, qe, s)), fx_value(get(qm, qe, n.tp)),
-                                        fx_value(get(qm, qe, n.tm)), fx_value(get(qm, qe, n.xp)),
-                                        fx_value(get(qm, qe, n.xm)), fx_link_value(wt), fx_link_value(wtd),
-                                        fx_link_value(wx), fx_link_value(wxd));
+        o = dslash_wide<1, MU0>(c.kd, fx_value(get(qm, qe, s)), fx_value(get(qm, qe, n.tp)),
+                                fx_value(get(qm, qe, n.tm)), fx_value(get(qm, qe, n.xp)), fx_value(get(qm, qe, n.xm)),
+                                wt, wtd, wx, wxd);
       double2 xv = x[s], rv = r[s];
       const double2 pv = p[s];
       xv.x += alpha * pv.x;

@@ -157,8 +157,7 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
     double2 o;
     if (!fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o)) {
       const Nbr n = neighbours(g, s, t, x);
-      o = dslash_vals<double, DAG, MU0>(k, ld(s), ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), fx_link_value(wt),
-                                        fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
+      o = dslash_wide<DAG, MU0>(k, ld(s), ld(n.tp), ld(n.tm), ld(n.xp), ld(n.xm), wt, wtm, wx, wl);
     }
     if (lane <= last) epi(s, o, own);
     pm = pc;
@@ -311,6 +310,7 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
       double2 o;
       if (!fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o)) {
         const Nbr nb = neighbours(g, s, t, x);
+        // (not dslash_wide: its test for zeros costs this march 2%, 183 -> 187 ms a 1024^2 trajectory)
         o = dslash_vals<double, DAG, MU0>(k, own, at(nb.tp), at(nb.tm), at(nb.xp), at(nb.xm), fx_link_value(wt),
                                           fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
       }
