@@ -823,7 +823,7 @@ int tg_create(const tg_lattice_params* p, tg_lattice** out) {
   for (auto pp : f2)
     if ((rc = dmalloc(pp, n)) != TG_OK) return bail(rc);
   if ((rc = dmalloc(&L->st, 1)) != TG_OK || (rc = dmalloc(&L->log, kMaxLog)) != TG_OK ||
-      (rc = dmalloc(&L->ts, 1)) != TG_OK || (rc = dmalloc(&L->red.partials, (size_t)nblocks((int)V) + 32)) != TG_OK ||
+      (rc = dmalloc(&L->ts, 1)) != TG_OK || (rc = dmalloc(&L->red.partials, (size_t)reduction_blocks(L->g))) != TG_OK ||
       (rc = dmalloc(&L->red.counter, 1)) != TG_OK || (rc = dmalloc(&L->bar, kBarWords)) != TG_OK ||
       (rc = dmalloc(&L->pcg_part, 4 * (size_t)kPcgMaxGrid)) != TG_OK)
     return bail(rc);

@@ -169,6 +169,18 @@ __device__ __forceinline__ bool grid_sum(T v, double* partials, unsigned* counte
 
 inline int nblocks(int n, int bs = kBlock) { return (n + bs - 1) / bs; }
 inline int grid_of(const Geo& g) { return g.grid; }
+// Blocks of work of a stencil kernel (march: at least one row per warp, so that
+// a small lattice spreads over more SMs).
+inline int stencil_work(const Geo& g) {
+  return g.march ? nblocks(march_strips(g.nx) * g.nt, kBlock / 32) : nblocks(g.V);
+}
+// The most blocks a kernel with a grid_sum is launched with, each of which stores
+// a partial: the site kernels' or the stencil's.  A march whose last strip is not full
+// has more warp rows than V / 32 (720 x 144: 450 blocks, one site per thread 405).
+inline int reduction_blocks(const Geo& g) {
+  const int sites = nblocks(g.V), stencil = stencil_work(g);
+  return sites > stencil ? sites : stencil;
+}
 inline int stream_grid(int n) { return nblocks(n); }  // streaming kernels without reductions
 
 // grid-stride loop over the sites of a kernel

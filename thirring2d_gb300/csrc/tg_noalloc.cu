@@ -26,7 +26,9 @@ constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 constexpr size_t kVec64 = align_up(sizeof(double2) * kNoAllocMaxSites);
 constexpr size_t kVec32 = align_up(sizeof(float2) * kNoAllocMaxSites);
+// (reduction_blocks of any lattice it takes: a march has at most 10 / 288 of a warp row per site)
 constexpr size_t kPartials = align_up(sizeof(double) * (kNoAllocMaxSites / kBlock + 64));
+static_assert(kPartials / sizeof(double) > (size_t)kNoAllocMaxSites * 10 / 288 / (kBlock / 32) + 1, "partials");
 constexpr size_t kStateBytes = align_up(sizeof(CgState));
 constexpr size_t kCounterBytes = align_up(sizeof(unsigned));
 // Wtq, Wxq, r, p0, p1, Mp (16 bytes a site) + Wt32, Wx32 (FP32 links the link kernel also

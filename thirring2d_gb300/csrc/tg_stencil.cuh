@@ -408,12 +408,6 @@ __device__ __forceinline__ void stencil_team(const Geo& g, const OpK<R>& k, Ld& 
   }
 }
 
-// Blocks of work of a stencil kernel (march: at least one row per warp, so that
-// a small lattice spreads over more SMs).
-inline int stencil_work(const Geo& g) {
-  return g.march ? (march_strips(g.nx) * g.nt + kBlock / 32 - 1) / (kBlock / 32) : nblocks(g.V);
-}
-
 // ---------------------------------------------------------------------------
 // TMA-staged march.  Each warp owns kStages stage buffers in dynamic shared
 // memory, each holding one chunk (kMarchT rows) of its 32 columns: the
