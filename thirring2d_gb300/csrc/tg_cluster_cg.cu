@@ -225,12 +225,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_ccg
   int status = -1, iter = 0, refA = fx_total_ref(rr0), refB = refA;
   if (isnan(rr)) status = TG_E_NAN;
   else if (!(rr >= stop) || rr == 0.0) status = TG_OK;
-  auto tests = [&](double rn) -> int {
-    const long long b = ord(rn);
-    if (b < ord(stop)) return TG_OK;                                              // hmc.c:381
-    if (b > ord(limit)) return b > ord(INFINITY) ? TG_E_NAN : TG_E_DIVERGED;      // hmc.c:383-386
-    return iter + 1 >= a.maxiter ? TG_E_NOCONV : -1;
-  };
+  auto tests = [&](double rn) { return cg_verdict(rn, stop, limit, iter + 1 >= a.maxiter); };
   if (tid == 0) sc.rr = rr;
   int xp0, xm0;  // of the thread's first site
   ccg_x_offsets(g, min(P.b0 + tid, g.V - 1), xp0, xm0);
@@ -419,8 +414,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_ccg
   if (isnan(rr)) status = TG_E_NAN;
   else if (!(rr >= stop) || rr == 0.0) status = TG_OK;
   auto due = [&](double rn) -> int {  // a reliable update
-    const long long b = ord(rn);
-    return since_ru + 1 >= a.ru_interval || iter + 1 >= a.maxiter || b < ord(stop) || b < ord(drop) || b > ord(limit);
+    return since_ru + 1 >= a.ru_interval || iter + 1 >= a.maxiter || cg_update_due(rn, stop, drop, limit);
   };
   if (tid == 0) sc.rr = rr;
   int xp0, xm0;  // of the thread's first site

@@ -117,7 +117,4 @@ struct CcgScalars {
   double rr, rn;  // |r|^2 before and after the iteration, for a sum that is taken again
 };
 
-// The bits of a non-negative double, which compare as it does (NaN above all).
-__device__ __forceinline__ long long ord(double v) { return __double_as_longlong(v); }
-
 }  // namespace tg

@@ -94,6 +94,27 @@ TG_HD bool fx_total_value(unsigned low, unsigned mid, unsigned top, int ref, dou
   return q >= (1ull << 52) && top < kFxTopRefused - 64 && ref != 0;
 }
 
+// The bits of a double that is not negative (a norm, a stopping threshold), which
+// compare as it does, NaN above all: a NaN may have its sign set (an invalid operation's has).
+TG_HD long long norm_bits(double v) {
+  return (long long)(((unsigned long long)((unsigned)dbl_hi(v) & 0x7fffffffu) << 32) | dbl_lo(v));
+}
+
+// The verdict on |r|^2 = rn after a CG iteration: a status, or -1 to go on
+// (hmc.c:381-386).
+TG_HD int cg_verdict(double rn, double stop, double limit, bool last) {
+  const long long b = norm_bits(rn);
+  if (b > norm_bits(INFINITY)) return TG_E_NAN;
+  if (b < norm_bits(stop)) return TG_OK;
+  if (b > norm_bits(limit)) return TG_E_DIVERGED;
+  return last ? TG_E_NOCONV : -1;
+}
+// The mixed solvers' test for a reliable update, besides the count of iterations
+TG_HD bool cg_update_due(double rn, double stop, double drop, double limit) {
+  const long long b = norm_bits(rn);
+  return b < norm_bits(stop) || b < norm_bits(drop) || b > norm_bits(limit);
+}
+
 #ifdef __CUDACC__
 // A warp's partial: low + mid 2^26 in x, the top limbs in y.
 __device__ __forceinline__ longlong2 fx_warp_partial(FxTerm t) {
