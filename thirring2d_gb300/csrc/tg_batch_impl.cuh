@@ -344,11 +344,12 @@ template <class F> __device__ __forceinline__ auto block_sum_int(double v, int& 
   }
   __syncthreads();
   if (s_ref < 0) {
-    return BlockTeam::sum_then(v, [&](double t) {
-      ref = 0;
+    const S r = BlockTeam::sum_then(v, [&](double t) {
       if (threadIdx.x == 0) s_ref = fx_total_ref(t);
       return f(t);
     });
+    ref = s_ref;  // every thread: written behind sum_then's barriers, next behind the next sum's first one
+    return r;
   }
   ref = s_ref;
   return *reinterpret_cast<const S*>(sc.out);
