@@ -12,9 +12,11 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
+#include "tg_resident.h"
 #include "tg_stencil.cuh"
 
 namespace tg {
@@ -79,30 +81,9 @@ template <class K> int occ_grid(K kernel, int work) {
   return grid < work ? grid : (work > 0 ? work : 1);
 }
 
-// The same with dynamic shared memory (staged kernels); the kernel's dynamic
-// shared memory limit is raised to smem on first use.
+// The same with dynamic shared memory (staged kernels).
 template <class K> int occ_grid_smem(K kernel, int work, int smem) {
-  static int sms = 0;
-  static std::mutex mu;
-  static std::unordered_map<const void*, int> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  }
-  auto it = cache.find((const void*)kernel);
-  int per_sm;
-  if (it == cache.end()) {
-    per_sm = 0;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, smem) != cudaSuccess || per_sm <= 0)
-      per_sm = 1;
-    cache.emplace((const void*)kernel, per_sm);
-  } else {
-    per_sm = it->second;
-  }
-  int grid = per_sm * sms;
+  const int grid = std::max(1, resident_blocks((const void*)kernel, kBlock, smem));
   return grid < work ? grid : (work > 0 ? work : 1);
 }
 

@@ -21,11 +21,9 @@
 
 #include <algorithm>
 
-#include <mutex>
-#include <unordered_map>
-
 #include "tg_fused.cuh"
 #include "tg_gridbar.cuh"
+#include "tg_resident.h"
 #include "tg_scalar.cuh"
 
 namespace tg {
@@ -844,23 +842,6 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcgcg(PcgMxArgs a) {
 // stencil's work; cooperative launch so the barrier cannot wait on a block
 // that is not running.
 // ---------------------------------------------------------------------------
-template <class K> int pcg_resident(K kernel, int bs, int smem = 0) {
-  static std::mutex mu;
-  static std::unordered_map<const void*, int> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find((const void*)kernel);
-  if (it != cache.end()) return it->second;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, bs, smem) != cudaSuccess || per_sm <= 0)
-    per_sm = 1;
-  const int n = per_sm * sms;
-  cache.emplace((const void*)kernel, n);
-  return n;
-}
-
 template <class K, class Args>
 cudaError_t coop_launch(K kernel, int grid, int bs, cudaStream_t s, const Args& a, int smem = 0) {
   cudaLaunchConfig_t cfg = {};
@@ -919,12 +900,14 @@ int pcg_block_override() {
 template <class K512, class K256, class K1, class Args>
 cudaError_t pcg_launch(const Geo& g, K512 k512, K256 k256, K1 k1, int one_rows, cudaStream_t s, const Args& a,
                        int warp_smem = 0) {
-  const int r512 = pcg_resident(k512, 512, 16 * warp_smem);
+  const int r512 = resident_blocks((const void*)k512, 512, 16 * warp_smem);
+  const int r256 = resident_blocks((const void*)k256, 256, 8 * warp_smem);
+  if (r512 <= 0 || r256 <= 0) return cudaErrorLaunchOutOfResources;
   const int force = pcg_block_override();  // (keeps the march: small lattices on the large ones' path)
   if (force == 512) return coop_launch(k512, std::min(r512, kPcgMaxGrid), 512, s, a, 16 * warp_smem);
   if (force == 0 && pcg_work(g, 512, 1) >= r512) return coop_launch(k512, pcg_grid(g, r512, 512), 512, s, a, 16 * warp_smem);
   if (one_rows > 0 && pcg_work(g, 256, one_rows) == 1) return coop_launch(k1, 1, 256, s, a);
-  return coop_launch(k256, pcg_grid(g, pcg_resident(k256, 256, 8 * warp_smem), 256), 256, s, a, 8 * warp_smem);
+  return coop_launch(k256, pcg_grid(g, r256, 256), 256, s, a, 8 * warp_smem);
 }
 
 cudaError_t pcg64(cudaStream_t s, bool mu0, Pcg64Args a) {
