@@ -64,11 +64,19 @@ int batch_smem_limit(int cfg) {
   return std::min(per_block - 1024, 227 * 1024) - kBatchStaticSmem;
 }
 
+// Let kernel k of instance cfg have up to the instance's share.  The limit belongs to
+// the kernel, not to a launch: one that followed the launch's own need would be lowered by
+// another batch's thread between the two.  (All instances that run one kernel have
+// the same share.)
+void batch_allow_smem(const void* k, int cfg) {
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem_limit(cfg));
+}
+
 static void launch_blocks(cudaStream_t s, int cfg, int grid, const BatchChain* chains, const int* order, int n,
                           const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
   const void* k = batch_kernel_of(cfg, P.cg.precision == TG_PREC_FP64);
   const int sm = P.cg.smem;
-  if (sm > 0) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (sm > 0) batch_allow_smem(k, cfg);
   BatchFields f = F;
   BatchTraj p = P;
   void* args[] = {&chains, &order, &n, &f, &p, &results, &queue};
@@ -99,9 +107,7 @@ void batch_filler_launch(cudaStream_t s, int cfg, int blocks, const BatchChain* 
   // run the same code, so a chain's result does not depend on which block ran it
   const bool wide = kBatchCfgs[cfg].block == 512;
   const int sm = P.cg.smem;
-  if (sm > 0)
-    cudaFuncSetAttribute(wide ? batch_kernel<512, 1>() : batch_kernel<256, 1>(),
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (sm > 0) batch_allow_smem(wide ? batch_kernel<512, 1>() : batch_kernel<256, 1>(), cfg);
   if (wide) k_batch_trajectory<512, 1><<<blocks, 512, sm, s>>>(chains, order, n, F, f, results, queue);
   else k_batch_trajectory<256, 1><<<blocks, 256, sm, s>>>(chains, order, n, F, f, results, queue);
 }
@@ -110,7 +116,7 @@ void batch_trajectory(cudaStream_t s, int cfg, int sms, const BatchChain* chains
                       const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
   const int teams = std::min(n, std::max(1, batch_teams(cfg, sms, P.cg.precision == TG_PREC_FP64)));
   if (kBatchCfgs[cfg].cluster > 1)
-    batch_cluster_launch(s, cluster_kernel_of(cfg), teams, chains, order, n, F, P, results, queue);
+    batch_cluster_launch(s, cfg, cluster_kernel_of(cfg), teams, chains, order, n, F, P, results, queue);
   else launch_blocks(s, cfg, teams, chains, order, n, F, P, results, queue);
 }
 

@@ -86,6 +86,7 @@ void batch_filler_launch(cudaStream_t s, int cfg, int blocks, const BatchChain* 
 // and what instance cfg has for it per block.
 constexpr int kSmallSite = 5 * 16 + 2 * 4, kBatchStaticSmem = 1536;
 int batch_smem_limit(int cfg);
+void batch_allow_smem(const void* kernel, int cfg);
 // teams (blocks or clusters) of instance cfg that can be resident at once (0: cannot launch)
 int batch_teams(int cfg, int sms, bool fp64);
 // the tuned instance as reported to callers: block * 100 + 10 * cluster (if > 1)
@@ -98,8 +99,8 @@ inline int batch_cfg_id(const BatchCfg& c) {
 // tg_batch_cluster.cu: instance `which` (0: 512 x 2 blocks, 1: 512 x 4, 2: 256 x 4,
 // 3: 512 x 4 with pairs)
 int batch_cluster_max(int which);
-void batch_cluster_launch(cudaStream_t s, int which, int clusters, const BatchChain* chains, const int* order, int n,
-                          const BatchFields& F, const BatchTraj& P, ChainResult* results,
+void batch_cluster_launch(cudaStream_t s, int cfg, int which, int clusters, const BatchChain* chains, const int* order,
+                          int n, const BatchFields& F, const BatchTraj& P, ChainResult* results,
                           unsigned long long* queue);
 
 }  // namespace tg

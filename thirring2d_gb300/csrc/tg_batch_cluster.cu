@@ -37,21 +37,21 @@ int batch_cluster_max(int which) {
 }
 
 template <int BS, int CL, bool PAIRS = false>
-static void launch_cluster(cudaStream_t s, int clusters, const BatchChain* chains, const int* order, int n,
+static void launch_cluster(cudaStream_t s, int cfg, int clusters, const BatchChain* chains, const int* order, int n,
                            const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
   const int sm = P.cg.smem;
-  if (sm > 0)
-    cudaFuncSetAttribute(k_batch_cluster<BS, CL, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (sm > 0) batch_allow_smem((const void*)k_batch_cluster<BS, CL, PAIRS>, cfg);
   k_batch_cluster<BS, CL, PAIRS><<<clusters * CL, BS, sm, s>>>(chains, order, n, F, P, results, queue);
 }
 
-void batch_cluster_launch(cudaStream_t s, int which, int clusters, const BatchChain* chains, const int* order, int n,
-                          const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
+void batch_cluster_launch(cudaStream_t s, int cfg, int which, int clusters, const BatchChain* chains, const int* order,
+                          int n, const BatchFields& F, const BatchTraj& P, ChainResult* results,
+                          unsigned long long* queue) {
   switch (which) {
-    case 0: launch_cluster<512, 2>(s, clusters, chains, order, n, F, P, results, queue); break;
-    case 1: launch_cluster<512, 4>(s, clusters, chains, order, n, F, P, results, queue); break;
-    case 3: launch_cluster<512, 4, true>(s, clusters, chains, order, n, F, P, results, queue); break;
-    default: launch_cluster<256, 4>(s, clusters, chains, order, n, F, P, results, queue); break;
+    case 0: launch_cluster<512, 2>(s, cfg, clusters, chains, order, n, F, P, results, queue); break;
+    case 1: launch_cluster<512, 4>(s, cfg, clusters, chains, order, n, F, P, results, queue); break;
+    case 3: launch_cluster<512, 4, true>(s, cfg, clusters, chains, order, n, F, P, results, queue); break;
+    default: launch_cluster<256, 4>(s, cfg, clusters, chains, order, n, F, P, results, queue); break;
   }
 }
 
