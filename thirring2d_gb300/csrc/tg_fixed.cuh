@@ -27,8 +27,8 @@
 //
 // Exponents outside [kFxEmin, kFxEmax] (operands all zero, denormal, huge, Inf
 // or NaN), operator constants that are not finite, and links that are not
-// finite (marked by bit 0 of the real low limb) take the FP64 form: fx_dslash
-// returns false and the caller computes the site in FP64.
+// finite or lie across an open boundary (marked by bit 0 of the real low limb) take
+// the FP64 form: fx_dslash returns false and the caller computes the site in FP64.
 #pragma once
 
 #include <math.h>
@@ -148,13 +148,22 @@ TG_HD FxLink to_fx_link(double2 w) {
   l.w = i.lo;
   return l;
 }
+// A link across an open boundary, W = 0: marked too, because the operand behind it does
+// not contribute and must not set the scale of the site's sum (beside one 2^60 times the
+// others nothing would be left of them).  Bit 0 of both low limbs.
+TG_HD FxLink fx_open_link() {
+  FxLink l;
+  l.x = l.z = 0;
+  l.y = l.w = 1;
+  return l;
+}
 // ... and back, for the FP64 form
 TG_HD double2 fx_link_value(FxLink l) {
   const double s = 1.0 / 1152921504606846976.0;  // 2^-60
   double2 w;
   w.x = (double)((long long)l.x * 4294967296LL + l.y) * s;
   w.y = (double)((long long)l.z * 4294967296LL + l.w) * s;
-  if (l.y & 1) w.x = w.y = dbl_of(0x7ff8000000000000ull);
+  if (l.y & 1) w.x = w.y = (l.w & 1) ? 0.0 : dbl_of(0x7ff8000000000000ull);
   return w;
 }
 

@@ -144,7 +144,7 @@ TG_HD void fx_link_of(double a, int sgn, double2& w, FxLink& q) {
   const double f = 0.5 * (double)sgn;
   w.x = f * cs;
   w.y = f * sn;
-  q = to_fx_link(w);
+  q = (sgn == 0 && w.x == 0 && w.y == 0) ? fx_open_link() : to_fx_link(w);
 }
 
 // 1 - cos a
