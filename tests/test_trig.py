@@ -143,3 +143,26 @@ def test_turns(harness):
         es, ec = sincos(2 * PI * (2 * int(x) + 1) / 2 ** 54)
         for got, want in ((c, ec), (s, es)):
             assert abs(Fraction(float(got)) - want) <= Fraction(8, 2 ** 64) + Fraction(math.ulp(float(got)))
+
+
+def test_links_near_the_axes_keep_their_relative_accuracy(harness):
+    """Near the multiples of pi/2 the small part of W is within 2 ulp (4 of 2^-53) of itself."""
+    rng = np.random.default_rng(5)
+    k = np.concatenate((np.arange(-40, 41), rng.integers(-600000, 600000, 150)))
+    near = np.concatenate([k * (math.pi / 2), k * (math.pi / 2) + rng.normal(size=len(k)) * 2.0 ** rng.integers(-45, -6, len(k))])
+    near = near[np.abs(near) < 2.0 ** 20]
+    for x, (wc, ws, _, _) in zip(near, harness(0, near)):
+        s, c = sincos(Fraction(float(x)))
+        for got, want in ((wc, c / 2), (ws, s / 2)):
+            assert abs(Fraction(float(got)) - want) <= Fraction(4, 2 ** 53) * abs(want)
+
+
+def test_turns_near_the_axes_keep_their_relative_accuracy(harness):
+    rng = np.random.default_rng(6)
+    v = np.concatenate([q * 2 ** 51 + s * rng.integers(0, 2 ** int(b), 20) for q in range(5) for b in (1, 5, 20, 40, 44, 45, 46, 50)
+                        for s in (1, -1)])
+    v = v[(v >= 0) & (v < 2 ** 53)].astype(float)
+    for x, (c, s, _, _) in zip(v, harness(3, v)):
+        es, ec = sincos(2 * PI * (2 * int(x) + 1) / 2 ** 54)
+        for got, want in ((c, ec), (s, es)):
+            assert abs(Fraction(float(got)) - want) <= Fraction(4, 2 ** 53) * abs(want)

@@ -9,9 +9,11 @@
 // Series: sum (-z)^n / (2n+1)!, n <= 9, and sum (-z)^n / (2n)!, n <= 10, z = r^2 <=
 // 0.617; the first terms left out are below 2^-72.  A product drops its low*low
 // limbs and is at most 2 units of 2^-64 low; each factor z shrinks what came before,
-// so the results are within 8 * 2^-64 absolute.  Where no multiple of pi/2 was taken out, sin is
-// formed as a * (sin(r)/r) in FP64, which keeps its relative accuracy at small
-// angles (1 ulp).  |a| >= 2^20, Inf and NaN: fx_trig returns false.
+// so the results are within 8 * 2^-64 absolute.  Relative accuracy (2 ulp) too:
+//   * where no multiple of pi/2 was taken out, sin is formed as a * (sin(r)/r) in FP64;
+//   * near the other multiples a part of a link below 2^-8 is left to the library, and
+//     one of a Gaussian's angle, which is exact there, is formed as r * (sin(r)/r).
+// |a| >= 2^20, Inf and NaN: fx_trig returns false.
 #pragma once
 
 #include "tg_fixed.cuh"
@@ -109,10 +111,13 @@ TG_HD bool fx_trig(double a, FxTrig& out) {
   return true;
 }
 
+// Results below 2^(kTrigSmall - 64) have less than FP64's relative accuracy.
+constexpr int kTrigSmall = 56;
+
 // half * sgn * (cos a, sin a) in FP64 and as limbs: one link (sgn = -1, 0 or 1).
 TG_HD void fx_link_of(double a, int sgn, double2& w, FxLink& q) {
   FxTrig t;
-  if (sgn != 0 && fx_trig(a, t)) {
+  if (sgn != 0 && fx_trig(a, t) && !(t.reduced && ((t.sn < t.cs ? t.sn : t.cs) >> kTrigSmall) == 0)) {
     const bool flip = sgn < 0;
     const double wc = u64_scaled(t.cs, 65);
     w.x = (t.neg_cs != flip) ? -wc : wc;
@@ -164,6 +169,11 @@ TG_HD void fx_sincos_turn(u64 v, double& cs, double& sn) {
   const FxTrig t = fx_trig_reduced(mulhi_exact(f << 1, 0xc90fdaa22168c234ull), neg, k, true);
   cs = u64_scaled(t.cs, 64);
   sn = u64_scaled(t.sn, 64);
+  if ((f >> kTrigSmall) == 0) {  // f has 44 bits
+    const double s = u64_scaled(f, 64) * 1.5707963267948966 * u64_scaled(t.ratio, 64);
+    if (k & 1u) cs = s;
+    else sn = s;
+  }
   if (t.neg_cs) cs = -cs;
   if (t.neg_sn) sn = -sn;
 }
