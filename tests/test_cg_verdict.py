@@ -1,8 +1,10 @@
 """How a CG iteration ends (cg_verdict in csrc/tg_scalar.cuh): on the CPU against the
 plain comparisons, NaNs of either sign and payload among them; and on the GPU,
 solves that meet a NaN inside the iteration in every solver."""
+import math
 import os
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -60,3 +62,53 @@ def test_nan_inside_a_solve(nt, nx, precision):
         L.set_gauge(rng.normal(0, 0.5, (nt, nx, 2)))
         b = 1e160 * (rng.normal(size=(nt, nx)) + 1j * rng.normal(size=(nt, nx)))
         assert L.fmdm_invert_cg(b, cp)[1].status == tg.native.TG_E_NAN
+
+
+QUOTIENTS = r"""
+#include <cstdio>
+#include "tg_scalar.cuh"
+int main() {  // records a, b -> a / b with 1 / b known
+  double r[2];
+  while (fread(r, sizeof r, 1, stdin) == 1) {
+    const double q = tg::div_prepared(r[0], r[1], 1.0 / r[1]);
+    fwrite(&q, sizeof q, 1, stdout);
+  }
+}
+"""
+
+
+def test_quotients_from_a_reciprocal(tmp_path):
+    """(1/2 + 2^-40) ulp, 0.75 allowed, as of the other quotients; down to sums that are denormal,
+    whose reciprocal overflows."""
+    (tmp_path / "h.cu").write_text(QUOTIENTS)
+    subprocess.run([os.environ.get("NVCC", "nvcc"), "-std=c++17", "-O1", "-gencode", "arch=compute_103a,code=sm_103a",
+                    f"-I{ROOT}/thirring2d_gb300/csrc", f"-I{ROOT}/include", "-o", str(tmp_path / "h"), str(tmp_path / "h.cu")],
+                   check=True, capture_output=True)
+    rng = np.random.default_rng(2)
+    e = rng.integers(-1074, 900, 4000)
+    e[:200] = rng.integers(-1074, -1000, 200)
+    b = rng.uniform(1, 2, 4000) * np.exp2(e.astype(float))
+    b = b[b > 0]
+    a = b * rng.uniform(1e-3, 4, len(b))
+    got = np.frombuffer(subprocess.run([str(tmp_path / "h")], input=np.stack([a, b], 1).tobytes(), capture_output=True,
+                                       check=True).stdout)
+    for x, y, v in zip(a, b, got):
+        q = Fraction(x) / Fraction(y)
+        assert abs(Fraction(float(v)) - q) <= Fraction(3, 4) * Fraction(math.ulp(float(v)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nt,nx", [(8, 8), (48, 64), (128, 128), (256, 256), (512, 640)])
+def test_tiny_sources(nt, nx):
+    """|b|^2 of 1e-295 to 1e-300 and a residual whose square ends below the normal range."""
+    import thirring2d_gb300 as tg
+    rng = np.random.default_rng(3)
+    with tg.Lattice(nt, nx, 0.3, 0.5, 0.0, -1, 1) as L:
+        L.set_gauge(rng.normal(0, 0.5, (nt, nx, 2)))
+        b = rng.normal(size=(nt, nx)) + 1j * rng.normal(size=(nt, nx))
+        cp = tg.cg_params(rel_tol=1e-8, abs_tol2=0, maxiter=2000)
+        x, res = L.fmdm_invert_cg(b, cp)
+        y, tiny = L.fmdm_invert_cg(1e-150 * b, cp)
+    assert res.status == tiny.status == 0
+    assert abs(tiny.iterations - res.iterations) <= 2
+    assert np.linalg.norm(y / 1e-150 - x) <= 4e-8 / 0.3 * np.linalg.norm(x)

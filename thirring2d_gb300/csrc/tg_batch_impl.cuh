@@ -419,7 +419,7 @@ __device__ __noinline__ CgOut block_cg64(const ChainCtx& ctx, const BatchCg& P, 
     };
     stencil_team<T, double, 1, MU0>(c.g, kd, ld2, c.Wtq, c.Wxq, epi2);
     const CgTail64 e = T::sum_then(v, [&](double rn) {
-      return CgTail64{rn, rn * st.inv_rr, tests(rn, out.iter + 1)};
+      return CgTail64{rn, div_prepared(rn, rr, st.inv_rr), tests(rn, out.iter + 1)};
     });
     half ^= 1;
     out.iter++;
@@ -523,7 +523,7 @@ __device__ __noinline__ CgOut block_cg64_small(const ChainCtx& ctx, const BatchC
       v = fma(rv.y, rv.y, v);
     }
     const CgTail64 e = block_sum_int(v, refB, [&](double rn) {
-      return CgTail64{rn, rn * st.inv_rr, tests(rn, out.iter + 1)};
+      return CgTail64{rn, div_prepared(rn, rr, st.inv_rr), tests(rn, out.iter + 1)};
     });
     out.iter++;
     beta = e.beta;

@@ -317,7 +317,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_ccg
       double rn;
       const bool ok = fx_partials_total(postB, P.nblocks * nsw, refB, rn);
       if (tid == T) {
-        sc.beta = rn * inv_rr;
+        sc.beta = div_prepared(rn, rr, inv_rr);
         sc.verdict = tests(rn);
         sc.okB = ok;
         sc.refB = fx_total_ref(rn);

@@ -282,7 +282,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
       double rn;
       const bool ok = ex.total(postB, refB, rn);
       if (tid == T) {
-        sc.beta = rn * inv_rr;
+        sc.beta = div_prepared(rn, rr, inv_rr);
         sc.verdict = tests(rn);
         sc.okB = ok;
         sc.refB = fx_total_ref(rn);

@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(BS, pcg_min_blocks(BS)) k_pcg64(Pcg64Args a) {
     PcgTail64 e;
     double inv_rr = 0;  // thread 0's
     if (!grid_total_then<BS>(vb, partB, a.bar, [&](double rn) {
-          PcgTail64 o{rn, rn * inv_rr, -1};
+          PcgTail64 o{rn, div_prepared(rn, rr, inv_rr), -1};
           if (isnan(rn)) o.status = TG_E_NAN;
           else if (rn < stop) o.status = TG_OK;           // hmc.c:381
           else if (rn > limit) o.status = TG_E_DIVERGED;  // hmc.c:383-386

@@ -22,6 +22,12 @@ TG_HD double div_corrected(double a, double b, double inv) {
   return fma(fma(-b, q, a), inv, q);
 }
 
+// a / b, b > 0, given inv = 1 / b rounded: the same, where inv has not overflowed or
+// come near it (b < 2^-1000: plain division).
+TG_HD double div_prepared(double a, double b, double inv) {
+  return inv < 1.0715086071862673e301 ? div_corrected(a, b, inv) : a / b;  // 2^1000
+}
+
 // a / b by Newton's iteration on the reciprocal (x' = x + x (1 - b x), which
 // doubles the correct bits) from an FP32 reciprocal of b's mantissa, then the
 // residual correction (without CORRECT, for a quotient that is rounded to FP32,
