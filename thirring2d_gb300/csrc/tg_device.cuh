@@ -87,7 +87,7 @@ __device__ __forceinline__ double2 dslash_wide(const OpK<double>& k, double2 pc,
   const bool zero = pc.x == 0 && pc.y == 0 && ptu.x == 0 && ptu.y == 0 && ptd.x == 0 && ptd.y == 0 && pxu.x == 0 &&
                     pxu.y == 0 && pxd.x == 0 && pxd.y == 0;
   // (a constant or a link that is not finite makes it NaN)
-  if (zero && k.emin == kFxEmin && !((wt.y | wtd.y | wx.y | wxd.y) & 1)) return make_double2(0.0, 0.0);
+  if (zero && fx_finite(k, wt, wtd, wx, wxd)) return make_double2(0.0, 0.0);
   return dslash_vals<double, DAG, MU0>(k, pc, ptu, ptd, pxu, pxd, fx_link_value(wt), fx_link_value(wtd),
                                        fx_link_value(wx), fx_link_value(wxd));
 }

@@ -167,6 +167,9 @@ TG_HD double2 fx_link_value(FxLink l) {
   return w;
 }
 
+// Not finite (bit 0)
+TG_HD int fx_link_bad(FxLink l) { return l.y & ~l.w; }
+
 // Operator constants.  out = m in + cf Wt in(+t) + cb conj(Wt(-t)) in(-t) + ...;
 // besides the FP64 values, m as 60-bit limbs at the scale 2^60 with its
 // exponent me, and |cf|, |cb| as 62-bit limbs (values in [1/2, 1)) with theirs.
@@ -287,6 +290,15 @@ TG_HD bool fx_dslash(const OpK<double>& k, const FxC& pc, const FxC& ptu, const 
   out.x = fx_round(x, E);
   out.y = fx_round(y, E);
   return ok;
+}
+
+// For a site that fx_dslash refused: nothing makes the products of zeros NaN.
+TG_HD bool fx_finite(const OpK<double>& k, FxLink wt, FxLink wtd, FxLink wx, FxLink wxd) {
+  return k.emin == kFxEmin && !((fx_link_bad(wt) | fx_link_bad(wtd) | fx_link_bad(wx) | fx_link_bad(wxd)) & 1);
+}
+// Zero of either sign: exponent 0 and only the stray bit (a denormal has mantissa bits besides it).
+TG_HD bool fx_zero(const FxC& f) {
+  return f.e == 0 && (((f.re ^ (f.re >> 63)) | (f.im ^ (f.im >> 63))) ^ (1LL << 59)) == 0;
 }
 
 }  // namespace tg

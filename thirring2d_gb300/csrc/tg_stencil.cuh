@@ -243,12 +243,14 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
     const int t = ta + i, tp = (t + 1 == g.nt) ? 0 : t + 1;
     const unsigned d = rows_a + slot * (NA * 512);
     const int so = t * nx + x, sp = tp * nx + x;
+    if (lane <= last) {  // (the spare lanes' copies of one address took a ragged strip's warps 17% longer)
 #pragma unroll
-    for (int j = 0; j < NS; j++) cp_async16(d + j * 512, src[j] + sp);
-    cp_async16(d + NS * 512, Wt + so);
-    cp_async16(d + (NS + 1) * 512, Wx + so);
+      for (int j = 0; j < NS; j++) cp_async16(d + j * 512, src[j] + sp);
+      cp_async16(d + NS * 512, Wt + so);
+      cp_async16(d + (NS + 1) * 512, Wx + so);
 #pragma unroll
-    for (int j = 0; j < NE; j++) cp_async16(d + (NS + 2 + j) * 512, ext[j] + so);
+      for (int j = 0; j < NE; j++) cp_async16(d + (NS + 2 + j) * 512, ext[j] + so);
+    }
     if ((i & (kMarchT - 1)) == 0 && lane < EL) {
       const int rr = min(t + (lane & (kMarchT - 1)), tb - 1);
       const int c = rr * nx + (lane < kMarchT ? xle : xre);
@@ -299,20 +301,38 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
       const FxLink wt = *reinterpret_cast<const FxLink*>(rw + NS * 32);
       const FxLink wx = *reinterpret_cast<const FxLink*>(rw + (NS + 1) * 32);
       const double2 pp = comb(v);
-      const FxC pe = shfl_fx(ef, (lane == last) ? kMarchT + ic : ic);
-      const FxC pr = sel_fx(lane == last, pe, shfl_fx(pc, lane + 1));
-      const FxC pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
-      const FxLink we = shfl_lk(ew, ic);
-      FxLink wl = shfl_lk(wx, lane - 1);
-      if (lane == 0) wl = we;
+      // the x neighbours and the link from x - 1, out of the lanes beside this one
+      auto beside = [&](FxC& pr, FxC& pl, FxLink& wl) {
+        const FxC pe = shfl_fx(ef, (lane == last) ? kMarchT + ic : ic);
+        pr = sel_fx(lane == last, pe, shfl_fx(pc, lane + 1));
+        pl = sel_fx(lane == 0, pe, shfl_fx(pc, lane - 1));
+        const FxLink we = shfl_lk(ew, ic);
+        wl = shfl_lk(wx, lane - 1);
+        if (lane == 0) wl = we;
+      };
+      FxC pr, pl;
+      FxLink wl;
+      beside(pr, pl, wl);
       const FxC pn = to_fx(pp);
       const int t = ta + i, s = t * nx + x;
       double2 o;
-      if (!fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o)) {
-        const Nbr nb = neighbours(g, s, t, x);
-        // (not dslash_wide: its test for zeros costs this march 2%, 183 -> 187 ms a 1024^2 trajectory)
-        o = dslash_vals<double, DAG, MU0>(k, own, at(nb.tp), at(nb.tm), at(nb.xp), at(nb.xm), fx_link_value(wt),
-                                          fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
+      // (what the lanes beyond the strip's last hold is arbitrary, and of no use)
+      const bool ok = fx_dslash<DAG, MU0>(k, pc, pn, pm, pr, pl, wt, wtm, wx, wl, o) || lane > last;
+      // A vector that is zero in places has whole rows of refused sites, which are not worth
+      // a reload and the FP64 form (1024^2 iteration on a point source 58 us, 192 with it).
+      // The whole warp comes here, so that the neighbours can be shuffled again
+      // instead of being kept in registers past the operator (a dense solve 52 us so, 53 kept).
+      if (__any_sync(0xffffffffu, !ok)) {
+        beside(pr, pl, wl);
+        if (!ok) {
+          if (fx_zero(pc) && fx_zero(pn) && fx_zero(pm) && fx_zero(pr) && fx_zero(pl) && fx_finite(k, wt, wtm, wx, wl)) {
+            o = make_double2(0.0, 0.0);
+          } else {
+            const Nbr nb = neighbours(g, s, t, x);
+            o = dslash_vals<double, DAG, MU0>(k, own, at(nb.tp), at(nb.tm), at(nb.xp), at(nb.xm), fx_link_value(wt),
+                                              fx_link_value(wtm), fx_link_value(wx), fx_link_value(wl));
+          }
+        }
       }
       if (lane <= last) epi(s, o, own, rw + (NS + 2) * 32);
       pm = pc;
