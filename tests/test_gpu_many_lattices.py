@@ -1,0 +1,89 @@
+"""Several lattices at once, each with its own thread and stream, at the sizes whose solves
+take a block on every SM (csrc/tg_grid_cg.cu): they run beside one another, to the
+same bits as alone; and the shapes that let them, at the edges of their rules, against
+the oracle."""
+import ctypes
+import threading
+import time
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tg():
+    import thirring2d_gb300 as tg
+    tg.native.load()
+    return tg
+
+
+def cplx(rng, shape):
+    return rng.normal(size=shape) + 1j * rng.normal(size=shape)
+
+
+@pytest.mark.parametrize("nt,nx,precision", [(93, 100, 0), (128, 128, 0), (40, 330, 0), (161, 160, 0), (190, 204, 0), (197, 198, 0),
+                                             (64, 210, 0), (256, 256, 0), (278, 279, 0), (197, 198, 1), (260, 260, 1),
+                                             (278, 280, 1), (282, 276, 1), (80, 600, 1)])
+@pytest.mark.parametrize("mu", [0.0, 0.2])
+def test_shapes_against_oracle(tg, oracle_lib, nt, nx, precision, mu):
+    """Both residuals are 1e-11 of b: 2e-11 / m of |x|, doubled for the rounding of sums."""
+    rng = np.random.default_rng(nt * 1000 + nx)
+    A, b, m = rng.normal(0, 0.5, (nt, nx, 2)), cplx(rng, (nt, nx)), 0.3
+    o = oracle_lib.Oracle(nt, nx, m, 0.5, mu, -1, 1)
+    xo, st, it = o.cg(A, b, rel_tol=1e-11, abs_tol2=0)
+    with tg.Lattice(nt, nx, m, 0.5, mu, -1, 1) as L:
+        L.set_gauge(A)
+        x, res = L.fmdm_invert_cg(b, tg.cg_params(rel_tol=1e-11, abs_tol2=0, precision=precision))
+    assert res.status == 0 and st == 0
+    assert np.linalg.norm(x - xo) <= 4e-11 / m * np.linalg.norm(xo)
+    if precision == 0:
+        assert abs(res.iterations - it) <= max(2, it // 20)
+
+
+# the share of k lattices one after another that k at once may take (measured 0.29, 0.45, 0.59, 0.29;
+# where only one lattice's blocks fit an SM, 0.5 to 1)
+@pytest.mark.parametrize("n,precision,share", [(128, 0, 0.45), (192, 0, 0.65), (256, 0, 0.78), (256, 1, 0.42)])
+def test_at_once(tg, n, precision, share):
+    k, runs = 8, 12
+    cp = tg.cg_params(rel_tol=1e-10, abs_tol2=0, precision=precision)
+    rng = np.random.default_rng(n)
+    lattices, b, x = [], [], []
+    for _ in range(k):
+        L = tg.Lattice(n, n, 0.05, 0.6, 0.0, -1, 1)
+        L.set_gauge(rng.normal(0, 0.3, (n, n, 2)))
+        lattices.append(L)
+        b.append(torch.from_numpy(cplx(rng, (n, n))).cuda())
+        x.append(torch.empty_like(b[-1]))
+    torch.cuda.synchronize()
+
+    def work(i):
+        res = tg.native.CgResult()
+        for _ in range(runs):
+            rc = lattices[i].lib.tg_cg_dev(lattices[i].h, ctypes.byref(cp), ctypes.c_void_p(b[i].data_ptr()),
+                                           ctypes.c_void_p(x[i].data_ptr()), ctypes.byref(res))
+            assert rc == 0 and res.status == 0
+    alone, best = [], [1e9, 1e9]
+    for _ in range(3):
+        t0 = time.perf_counter()
+        for i in range(k):
+            work(i)
+        best[0] = min(best[0], time.perf_counter() - t0)
+        alone = [v.cpu() for v in x]
+        for v in x:
+            v.zero_()
+        torch.cuda.synchronize()
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(k)]
+        t0 = time.perf_counter()
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        best[1] = min(best[1], time.perf_counter() - t0)
+        for v, w in zip(x, alone):
+            assert torch.equal(v.cpu(), w)
+    for L in lattices:
+        L.close()
+    assert best[1] <= share * best[0]

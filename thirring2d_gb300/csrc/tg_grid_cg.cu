@@ -135,8 +135,12 @@ template <class F> __device__ __forceinline__ void gcg_halo(const CcgPart& P, in
 }
 __device__ __forceinline__ bool gcg_edge(const CcgPart& P, int nx, int i) { return i < nx || i >= P.n - nx; }
 
-// FP64: the iteration of k_pcg64
-template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg64(Pcg64Args a, int wmax, int nmax) {
+// FP64: the iteration of k_pcg64.  THREE: in 72 registers and at most 256 site threads, for
+// lattices of which an SM holds three blocks (gcg_shape).
+constexpr int kGcgThreeThreads = 256;
+template <bool MU0, bool THREE>
+__global__ void __launch_bounds__(THREE ? kGcgThreeThreads + 32 : kCcgThreads + 32, THREE ? 3 : 1)
+k_gcg64(Pcg64Args a, int wmax, int nmax) {
   extern __shared__ __align__(16) unsigned char gcg_smem[];
   __shared__ CcgScalars sc;
   __shared__ longlong2 warp_part[kCcgThreads / 32];
@@ -322,7 +326,7 @@ template <bool MU0> __global__ void __launch_bounds__(kCcgThreads + 32, 1) k_gcg
 //               links in registers, at a pass's end those of the next pass.
 //               Single sites, four ahead, took 18.3 us at 1000^2 (pairs: 15.3) and gained nothing
 //               at 1024^2; 448, 416, 384 or 320 site threads 15.7, 15.6, 16.0, 17.1.
-constexpr int kGcgSites = 0, kGcgStream = 1, kGcgPairs = 2;
+constexpr int kGcgSites = 0, kGcgStream = 1, kGcgPairs = 2, kGcgThree = 3;
 constexpr int kGcgAhead = 2;
 constexpr int kGcgStreamThreads = 480;  // with the scalar warp 16 warps: 128 registers instead of 96
 struct GcgLinks {
@@ -680,7 +684,7 @@ k_gcgmx(PcgMxArgs a, int wmax, int nmax) {
 // ---------------------------------------------------------------------------
 // sites of the largest block
 static int gcg_most_sites(int V, int nblocks, int form) {
-  return form != kGcgSites ? (V / 2 + nblocks - 1) / nblocks * 2 : (V + nblocks - 1) / nblocks;
+  return form == kGcgPairs || form == kGcgStream ? (V / 2 + nblocks - 1) / nblocks * 2 : (V + nblocks - 1) / nblocks;
 }
 static size_t gcg_bytes(const Geo& g, int nblocks, bool mixed, int form) {
   const size_t nmax = gcg_most_sites(g.V, nblocks, form), win = nmax + 2 * (size_t)g.nx;
@@ -699,15 +703,23 @@ static int gcg_resident() {
   auto it = cache.find(dev);
   if (it != cache.end()) return it->second;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
-  const void* kernels[] = {(const void*)k_gcg64<true>,         (const void*)k_gcg64<false>,
-                           (const void*)k_gcgmx<true, kGcgSites>,  (const void*)k_gcgmx<false, kGcgSites>,
-                           (const void*)k_gcgmx<true, kGcgPairs>,  (const void*)k_gcgmx<false, kGcgPairs>,
-                           (const void*)k_gcgmx<true, kGcgStream>, (const void*)k_gcgmx<false, kGcgStream>};
-  for (const void* k : kernels) {
+  const struct {
+    const void* k;
+    int threads;
+  } kernels[] = {{(const void*)k_gcg64<true, false>, kCcgThreads},
+                 {(const void*)k_gcg64<false, false>, kCcgThreads},
+                 {(const void*)k_gcg64<true, true>, kGcgThreeThreads},
+                 {(const void*)k_gcg64<false, true>, kGcgThreeThreads},
+                 {(const void*)k_gcgmx<true, kGcgSites>, kCcgThreads},
+                 {(const void*)k_gcgmx<false, kGcgSites>, kCcgThreads},
+                 {(const void*)k_gcgmx<true, kGcgPairs>, kCcgThreads},
+                 {(const void*)k_gcgmx<false, kGcgPairs>, kCcgThreads},
+                 {(const void*)k_gcgmx<true, kGcgStream>, kGcgStreamThreads},
+                 {(const void*)k_gcgmx<false, kGcgStream>, kGcgStreamThreads}};
+  for (const auto& q : kernels) {
     int n = 0;
-    const int threads = k == kernels[6] || k == kernels[7] ? kGcgStreamThreads : kCcgThreads;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCcgSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads + 32, kCcgSmem) != cudaSuccess || n < 1)
+    if (cudaFuncSetAttribute(q.k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCcgSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, q.k, q.threads + 32, kCcgSmem) != cudaSuccess || n < 1)
       sms = 0;
   }
   (void)cudaGetLastError();
@@ -729,9 +741,20 @@ static int gcg_resident() {
 // 250x2600 15.0 / 15.8, 1056x1040 16.7 / 20.1).  Mixed lattices whose rows span more than three blocks lose to the
 // window's upkeep (40x1500 7.4 / - / 7.2, 20x2000 7.2 / - / 6.6; 50x1000 7.0 / - / 7.2).
 // One block per SM: half of them cost 8.7 -> 11.3 at 256^2.  Threads: a site each, and
-// no fewer than half the window (16x1000 12.0 -> 8.9 with 544 instead of 128); 256 or 384
-// of them are no faster (256^2 9.0 and 9.5).
+// no fewer than half the window (16x1000 12.0 -> 8.9 with 544 instead of 128).
+//
+// Several lattices at once, each on its own stream and thread, share the SMs: a lattice of up to
+// a few hundred sites a block therefore takes no more threads and registers
+// than let an SM hold the blocks of two to four (an SM's quarter holds 5 warps of 96 registers, 7 of
+// 72).  us per iteration and lattice, 1 / 4 / 8 / 16 lattices, with the threads of one site each, and so:
+//   FP64   128^2 6.4 / 3.6 / 3.5 / 3.5 -> 6.8 / 2.3 / 1.9 / 1.9    192^2 7.3 / 7.2 / 7.2 / 7.2 -> 7.6 / 3.4 / 3.4 / 3.3
+//          256^2 8.9 / 8.8 / 8.8 / 8.8 -> 9.0 / 5.2 / 5.2 / 5.2    40x330 7.3 / 7.1 / 7.0 -> 7.1 / 3.9 / 3.8
+//   mixed  256^2 6.2 / 3.2 / 3.2 / 3.2 -> 5.8 / 1.8 / 1.8 / 1.8    278^2 6.3 / 3.3 / 3.3 / 3.2 -> 6.3 / 1.9 / 1.9 / 1.9
+// FP64, up to 256 sites a block where three fit the shared memory: the 72-register instance, a site a
+// thread, and no fewer than a third of the window; up to 512 where two fit: 256 threads.  Mixed,
+// up to 512 sites a block where four fit: two pairs a thread.
 constexpr int kGcgSites64 = 512, kGcgSitesMx = 2400;
+constexpr size_t kSmSmem = 228 * 1024, kBlockSmem = 1024 + 512;  // an SM's, and a block's besides its dynamic
 
 CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
   const CcgShape none{0, 0, 0};
@@ -754,8 +777,20 @@ CcgShape gcg_shape(const Geo& g, bool mixed, const CcgShape& cluster) {
   if (form == kGcgStream && g.nx % 2 != 0) return none;
   if (gcg_bytes(g, blocks, mixed, form) > (size_t)kCcgSmem) return none;
   if (!e && mixed && g.nx > 3 * n) return none;
-  const int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx) / (form != kGcgSites ? 2 : 1);
-  return CcgShape{blocks, std::min(form == kGcgStream ? kGcgStreamThreads : kCcgThreads, (t + 31) / 32 * 32), form};
+  auto fit = [&](size_t k) { return k * (gcg_bytes(g, blocks, mixed, form) + kBlockSmem) <= kSmSmem; };
+  int t = threads > 0 ? threads : std::max(n, n / 2 + g.nx) / (form != kGcgSites ? 2 : 1), most = kCcgThreads;
+  if (form == kGcgStream) {
+    most = kGcgStreamThreads;
+  } else if (!mixed && n <= 256 && (threads <= 0 || t <= kGcgThreeThreads) && fit(3)) {
+    form = kGcgThree;
+    most = kGcgThreeThreads;
+    if (threads <= 0) t = std::max(n, (n + 2 * g.nx + 2) / 3);
+  } else if (!mixed && threads <= 0 && n <= 512 && fit(2)) {
+    most = 256;
+  } else if (form == kGcgPairs && threads <= 0 && n <= 512 && fit(4)) {
+    most = 128;
+  }
+  return CcgShape{blocks, std::min(most, (t + 31) / 32 * 32), form};
 }
 
 template <class K, class Args>
@@ -775,7 +810,9 @@ static cudaError_t gcg_launch(K kernel, cudaStream_t s, const Args& a, bool mixe
 }
 
 cudaError_t gcg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& sh) {
-  return mu0 ? gcg_launch(k_gcg64<true>, s, a, false, sh) : gcg_launch(k_gcg64<false>, s, a, false, sh);
+  if (sh.form == kGcgThree)
+    return mu0 ? gcg_launch(k_gcg64<true, true>, s, a, false, sh) : gcg_launch(k_gcg64<false, true>, s, a, false, sh);
+  return mu0 ? gcg_launch(k_gcg64<true, false>, s, a, false, sh) : gcg_launch(k_gcg64<false, false>, s, a, false, sh);
 }
 cudaError_t gcgmx(cudaStream_t s, bool mu0, const PcgMxArgs& a, const CcgShape& sh) {
   switch (sh.form) {

@@ -173,7 +173,7 @@ cudaError_t pcgcg(cudaStream_t s, bool mu0, PcgMxArgs a);
 // blocks and threads per block, 0 blocks where the grid solvers are to be used.
 struct CcgShape {
   int blocks, threads;
-  int form = 0;  // grid solver, mixed: kGcgSites, kGcgPairs or kGcgStream (tg_grid_cg.cu)
+  int form = 0;  // grid solver, mixed: kGcgSites, kGcgPairs or kGcgStream; FP64: kGcgSites or kGcgThree (tg_grid_cg.cu)
 };
 CcgShape ccg_shape(const Geo& g, bool mixed);
 cudaError_t ccg64(cudaStream_t s, bool mu0, const Pcg64Args& a, const CcgShape& sh);
