@@ -34,6 +34,12 @@ __device__ __forceinline__ double warp_allsum(double v) {
   return v;
 }
 
+// a + Re(conj(u) v), the roundings spelled out: a chain has the same bits in every kernel,
+// and the compiler contracts u.x * v.x + u.y * v.y one way in one and another in the next.
+__device__ __forceinline__ double add_dot(double a, double2 u, double2 v) {
+  return fma(u.y, v.y, fma(u.x, v.x, a));
+}
+
 // Shared scratch of the team sums: the warps' partials, the block's total (read
 // by the other blocks of a cluster) and the result of the step that follows a
 // sum.
@@ -372,7 +378,7 @@ __device__ __noinline__ CgOut block_cg64(const ChainCtx& ctx, const BatchCg& P, 
     x[s] = make_double2(0, 0);
     c.r64[s] = bb;
     c.p64[s] = bb;
-    a += bb.x * bb.x + bb.y * bb.y;
+    a = add_dot(a, bb, bb);
   }
   const double rr0 = T::sum(a);
   double stop = P.abs_tol2;
@@ -459,7 +465,7 @@ __device__ __noinline__ CgOut block_cg64_small(const ChainCtx& ctx, const BatchC
     x[s] = make_double2(0, 0);
     r[s] = bb;
     p[s] = bb;
-    a += bb.x * bb.x + bb.y * bb.y;
+    a = add_dot(a, bb, bb);
   }
   const double rr0 = BlockTeam::sum(a);
   double stop = P.abs_tol2;
@@ -580,7 +586,7 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
     c.rs[s] = rb;
     c.ps[s] = rb;
     c.xs[s] = make_float2(0.f, 0.f);
-    a += bb.x * bb.x + bb.y * bb.y;
+    a = add_dot(a, bb, bb);
   }
   const double rr0 = T::sum(a);
   double stop = P.abs_tol2;
@@ -685,7 +691,7 @@ __device__ __noinline__ double team_apply(const ChainCtx& ctx, const double2* in
   TG_BSITES(s, c.g.V) {
     const double2 o = dslash_at<double, DAG, MU0>(c.g, DAG ? c.kd : c.km, in, c.Wtq, c.Wxq, s), n = in[s];
     if (out != nullptr) out[s] = o;
-    a += n.x * o.x + n.y * o.y;
+    a = add_dot(a, n, o);
   }
   return a;
 }
@@ -704,10 +710,10 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
     write_links(g, c.bc_t, c.bc_x, s, a, LinkOut{c.Wt, c.Wx, c.Wt32, c.Wx32, c.Wtq, c.Wxq});
     double2 e = philox_gauss_pair(c.seed, tr, (unsigned)s, 0u);
     c.tmp[s] = e;
-    a_pf += e.x * e.x + e.y * e.y;
+    a_pf = add_dot(a_pf, e, e);
     double2 p = philox_gauss_pair(c.seed, tr, (unsigned)s, 16u);
     c.mom[s] = p;
-    a_mom += p.x * p.x + p.y * p.y;
+    a_mom = add_dot(a_mom, p, p);
     a_g += one_minus_cos(a.x) + one_minus_cos(a.y);
     if (noise_on) c.noise[s] = philox_gauss_pair(c.seed, tr, (unsigned)s, 17u);
     c.An[s] = a;
@@ -767,8 +773,8 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
   const double b_md = noise_on ? team_apply<1, MU0, T>(c, c.noise, nullptr) : 0.0;
   TG_BSITES(s, V) {
     double2 ph = c.phi[s], xv = c.x[s], p = c.mom[s], a = c.An[s];
-    b_pf += ph.x * xv.x + ph.y * xv.y;
-    b_mom += p.x * p.x + p.y * p.y;
+    b_pf = add_dot(b_pf, ph, xv);
+    b_mom = add_dot(b_mom, p, p);
     b_g += one_minus_cos(a.x) + one_minus_cos(a.y);
   }
   const double Spf1 = T::sum(b_pf), Smom1 = T::sum(b_mom), Sg1 = fac * T::sum(b_g), Smd1 = T::sum(b_md);
