@@ -41,3 +41,25 @@ def test_chains_match_single_lattices(tg, instance, sizes):
                 assert abs(b.cg_iterations - r.cg_iterations) <= 2 * r.cg_solves
             assert np.abs(B.get_gauge(i) - L.get_gauge()).max() < 1e-9
     B.close()
+
+
+@pytest.mark.parametrize("instance", [12808, 25604])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_instances_with_a_kernel_per_precision(tg, instance, precision):
+    """The 64-register instances run mixed solves, and FP64 ones on other kernels: both
+    follow the 512-thread instance (dH to 1e-7 with solves to 1e-11, the same decisions)."""
+    rng = np.random.default_rng(18)
+    chains = [dict(nt=t, nx=x, m=0.3, g=0.7, mu=0.1 * (k % 2), bc_t=-1, bc_x=1, seed=60 + k)
+              for k, (t, x) in enumerate([(8, 8), (16, 16), (17, 15), (32, 32), (30, 64), (64, 64)])]
+    A0 = [rng.normal(0, 0.2, (c["nt"], c["nx"], 2)) for c in chains]
+    out = []
+    for inst in (51201, instance):
+        B = tg.Batch(chains)
+        for i, A in enumerate(A0):
+            B.set_gauge(i, A)
+        out.append(B.trajectory(tg.batch_params(nsteps=4, tau=0.1, block=inst,
+                                                cg=tg.cg_params(rel_tol=1e-11, abs_tol2=0.0, precision=precision))))
+        B.close()
+    for a, b in zip(*out):
+        assert a.status == b.status == 0 and a.accepted == b.accepted
+        assert abs(a.dH - b.dH) <= 1e-7 * max(1.0, abs(a.dH))

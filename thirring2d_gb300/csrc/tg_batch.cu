@@ -7,12 +7,12 @@
 
 namespace tg {
 
-template <int BS, int MINB>
+template <int BS, int MINB, BatchSolves S>
 __global__ void __launch_bounds__(BS, MINB) k_batch_trajectory(const BatchChain* __restrict__ chains,
                                                                const int* __restrict__ order, int n,
                                                                BatchFields F, BatchTraj P, ChainResult* results,
                                                                unsigned long long* queue) {
-  batch_trajectory_body<BS, MINB, BlockTeam>(chains, order, n, F, P, results, queue);
+  batch_trajectory_body<BlockTeam, S>(chains, order, n, F, P, results, queue);
 }
 
 // The kernel instances the autotuner chooses from: (threads per block,
@@ -36,7 +36,9 @@ static int cluster_kernel_of(int cfg) {
   return c.cluster == 2 ? 0 : (c.block == 512 ? 1 : 2);
 }
 
-template <int BS, int MINB> const void* batch_kernel() { return (const void*)k_batch_trajectory<BS, MINB>; }
+template <int BS, int MINB, BatchSolves S = kSolvesBoth> const void* batch_kernel() {
+  return (const void*)k_batch_trajectory<BS, MINB, S>;
+}
 
 // The kernel that runs instance cfg.  The 64-register ones (8 blocks of 128 or 4 of
 // 256 threads per SM) run FP64 trajectories at 128 registers and half the
@@ -45,8 +47,8 @@ template <int BS, int MINB> const void* batch_kernel() { return (const void*)k_b
 // 296 ms so, 549 at 64 registers; 512 chains of 16^2 at 8 blocks of 128: 5.3, 7.6.
 static const void* batch_kernel_of(int cfg, bool fp64) {
   switch (cfg) {
-    case 0: return fp64 ? batch_kernel<128, 4>() : batch_kernel<128, 8>();
-    case 1: return fp64 ? batch_kernel<256, 2>() : batch_kernel<256, 4>();
+    case 0: return fp64 ? batch_kernel<128, 4, kSolvesFp64>() : batch_kernel<128, 8, kSolvesMixed>();
+    case 1: return fp64 ? batch_kernel<256, 2>() : batch_kernel<256, 4, kSolvesMixed>();
     case 2: return batch_kernel<256, 2>();
     case 3: return batch_kernel<256, 1>();
     case 4: return batch_kernel<384, 1>();
@@ -72,15 +74,15 @@ void batch_allow_smem(const void* k, int cfg) {
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem_limit(cfg));
 }
 
-static void launch_blocks(cudaStream_t s, int cfg, int grid, const BatchChain* chains, const int* order, int n,
-                          const BatchFields& F, const BatchTraj& P, ChainResult* results, unsigned long long* queue) {
-  const void* k = batch_kernel_of(cfg, P.cg.precision == TG_PREC_FP64);
+static void launch_kernel(cudaStream_t s, const void* k, int cfg, int grid, int block, const BatchChain* chains,
+                          const int* order, int n, const BatchFields& F, const BatchTraj& P, ChainResult* results,
+                          unsigned long long* queue) {
   const int sm = P.cg.smem;
   if (sm > 0) batch_allow_smem(k, cfg);
   BatchFields f = F;
   BatchTraj p = P;
   void* args[] = {&chains, &order, &n, &f, &p, &results, &queue};
-  cudaLaunchKernel(k, dim3((unsigned)grid), dim3((unsigned)kBatchCfgs[cfg].block), args, (size_t)sm, s);
+  cudaLaunchKernel(k, dim3((unsigned)grid), dim3((unsigned)block), args, (size_t)sm, s);
 }
 
 int batch_teams(int cfg, int sms, bool fp64) {
@@ -105,11 +107,9 @@ void batch_filler_launch(cudaStream_t s, int cfg, int blocks, const BatchChain* 
   f.from_back = 1;
   // the one-block instance of the cluster kernel's block size: its solo chains
   // run the same code, so a chain's result does not depend on which block ran it
-  const bool wide = kBatchCfgs[cfg].block == 512;
-  const int sm = P.cg.smem;
-  if (sm > 0) batch_allow_smem(wide ? batch_kernel<512, 1>() : batch_kernel<256, 1>(), cfg);
-  if (wide) k_batch_trajectory<512, 1><<<blocks, 512, sm, s>>>(chains, order, n, F, f, results, queue);
-  else k_batch_trajectory<256, 1><<<blocks, 256, sm, s>>>(chains, order, n, F, f, results, queue);
+  const int bs = kBatchCfgs[cfg].block;
+  launch_kernel(s, bs == 512 ? batch_kernel<512, 1>() : batch_kernel<256, 1>(), cfg, blocks, bs, chains, order, n, F, f, results,
+                queue);
 }
 
 void batch_trajectory(cudaStream_t s, int cfg, int sms, const BatchChain* chains, const int* order, int n,
@@ -117,7 +117,9 @@ void batch_trajectory(cudaStream_t s, int cfg, int sms, const BatchChain* chains
   const int teams = std::min(n, std::max(1, batch_teams(cfg, sms, P.cg.precision == TG_PREC_FP64)));
   if (kBatchCfgs[cfg].cluster > 1)
     batch_cluster_launch(s, cfg, cluster_kernel_of(cfg), teams, chains, order, n, F, P, results, queue);
-  else launch_blocks(s, cfg, teams, chains, order, n, F, P, results, queue);
+  else
+    launch_kernel(s, batch_kernel_of(cfg, P.cg.precision == TG_PREC_FP64), cfg, teams, kBatchCfgs[cfg].block, chains, order, n, F,
+                  P, results, queue);
 }
 
 }  // namespace tg

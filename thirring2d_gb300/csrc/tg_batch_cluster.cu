@@ -11,7 +11,7 @@ template <int BS, int CL, bool PAIRS = false>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(BS, 1)
     k_batch_cluster(const BatchChain* __restrict__ chains, const int* __restrict__ order, int n, BatchFields F,
                     BatchTraj P, ChainResult* results, unsigned long long* queue) {
-  batch_trajectory_body<BS, 1, ClusterTeam<CL>, PAIRS>(chains, order, n, F, P, results, queue);
+  batch_trajectory_body<ClusterTeam<CL>, kSolvesBoth, PAIRS>(chains, order, n, F, P, results, queue);
 }
 
 template <int BS, int CL, bool PAIRS = false> int max_clusters_of() {

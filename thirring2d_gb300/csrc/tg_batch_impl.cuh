@@ -669,14 +669,22 @@ __device__ CgOut block_cg_mixed(const ChainCtx& c, const BatchCg& P, const doubl
   return out;
 }
 
-template <bool MU0, class T>
+// The solvers a kernel holds: an instance that only ever runs one precision leaves the
+// other's out.
+enum BatchSolves { kSolvesBoth, kSolvesMixed, kSolvesFp64 };
+
+template <bool MU0, class T, BatchSolves S>
 __device__ __forceinline__ CgOut block_cg(const ChainCtx& c, const BatchCg& P, const double2* b, double2* x) {
-  if (P.precision == TG_PREC_MIXED) return block_cg_mixed<MU0, T>(c, P, b, x);
-  if constexpr (T::nblocks_const == 1) {
-    // (8^2 chains: 1.8 ms per 512-chain trajectory here, 1.6 on the global path)
-    if (c.g.V >= 128 && c.g.V * kSmallSite <= P.smem) return block_cg64_small<MU0>(c, P, b, x);
+  if constexpr (S != kSolvesFp64) {
+    if (S == kSolvesMixed || P.precision == TG_PREC_MIXED) return block_cg_mixed<MU0, T>(c, P, b, x);
   }
-  return block_cg64<MU0, T>(c, P, b, x);
+  if constexpr (S != kSolvesMixed) {
+    if constexpr (T::nblocks_const == 1) {
+      // (8^2 chains: 1.8 ms per 512-chain trajectory here, 1.6 on the global path)
+      if (c.g.V >= 128 && c.g.V * kSmallSite <= P.smem) return block_cg64_small<MU0>(c, P, b, x);
+    }
+    return block_cg64<MU0, T>(c, P, b, x);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -696,7 +704,7 @@ __device__ __noinline__ double team_apply(const ChainCtx& ctx, const double2* in
   return a;
 }
 
-template <bool MU0, class T>
+template <bool MU0, class T, BatchSolves S>
 __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainResult* res) {
   const int V = c.g.V;
   const Geo& g = c.g;
@@ -738,7 +746,7 @@ __device__ void chain_trajectory(const ChainCtx& c, const BatchTraj& P, ChainRes
       write_links(g, c.bc_t, c.bc_x, s, a, LinkOut{c.Wt, c.Wx, c.Wt32, c.Wx32, c.Wtq, c.Wxq});
     }
     T::sync();
-    CgOut o = block_cg<MU0, T>(c, P.cg, c.phi, c.x);
+    CgOut o = block_cg<MU0, T, S>(c, P.cg, c.phi, c.x);
     iters += o.iter;
     maxit = max(maxit, o.iter);
     n_ru += o.n_ru;
@@ -844,7 +852,7 @@ __device__ __forceinline__ int queue_back(unsigned long long* queue, int n, int 
   return n;
 }
 
-template <int BS, int MINB, class T, bool PAIRS = false>
+template <class T, BatchSolves S = kSolvesBoth, bool PAIRS = false>
 __device__ __forceinline__ void batch_trajectory_body(const BatchChain* __restrict__ chains,
                                                       const int* __restrict__ order, int n, const BatchFields& F,
                                                       const BatchTraj& P, ChainResult* results,
@@ -867,8 +875,8 @@ __device__ __forceinline__ void batch_trajectory_body(const BatchChain* __restri
     const int ci = order[q];
     if (threadIdx.x == 0) fill_ctx(c, chains[ci], F);
     __syncthreads();
-    if (c.mu == 0.0) chain_trajectory<true, T>(c, P, &results[ci]);
-    else chain_trajectory<false, T>(c, P, &results[ci]);
+    if (c.mu == 0.0) chain_trajectory<true, T, S>(c, P, &results[ci]);
+    else chain_trajectory<false, T, S>(c, P, &results[ci]);
   }
   if constexpr (T::kCluster) {
     int carry = -1;  // a ticket past pair_end that this block runs alone
@@ -898,8 +906,8 @@ __device__ __forceinline__ void batch_trajectory_body(const BatchChain* __restri
             pair_timeouts() = 0;
           }
           __syncthreads();
-          if (c.mu == 0.0) chain_trajectory<true, PairTeam>(c, P, &results[ci]);
-          else chain_trajectory<false, PairTeam>(c, P, &results[ci]);
+          if (c.mu == 0.0) chain_trajectory<true, PairTeam, S>(c, P, &results[ci]);
+          else chain_trajectory<false, PairTeam, S>(c, P, &results[ci]);
           if (PairTeam::rank() == 0 && threadIdx.x == 0 && pair_timeouts() > 0) results[ci].status = TG_E_TIMEOUT;
           pq = -1;
         }
@@ -921,8 +929,8 @@ __device__ __forceinline__ void batch_trajectory_body(const BatchChain* __restri
       const int ci = order[mine];
       if (threadIdx.x == 0) fill_ctx(c, chains[ci], F);
       __syncthreads();
-      if (c.mu == 0.0) chain_trajectory<true, BlockTeam>(c, P, &results[ci]);
-      else chain_trajectory<false, BlockTeam>(c, P, &results[ci]);
+      if (c.mu == 0.0) chain_trajectory<true, BlockTeam, S>(c, P, &results[ci]);
+      else chain_trajectory<false, BlockTeam, S>(c, P, &results[ci]);
       mine = -1;
     }
   }
