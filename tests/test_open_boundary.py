@@ -18,17 +18,13 @@ int main() {  // records: which link is open, angle, operand behind it -> accept
   while (fread(r, sizeof r, 1, stdin) == 1) {
     FxLink q[4];
     double2 w;
-    int marks = 0;
-    for (int i = 0; i < 4; i++) {
-      fx_link_of(r[1], i == (int)r[0] ? 0 : 1, w, q[i]);
-      if (i != (int)r[0]) marks |= q[i].y & 1;
-    }
+    for (int i = 0; i < 4; i++) fx_link_of(r[1], i == (int)r[0] ? 0 : 1, w, q[i]);
     FxC v[5];
     for (int i = 0; i < 5; i++) v[i] = to_fx(i == (int)r[0] + 1 ? double2{r[2], r[2]} : double2{1.0, -0.5});
     double2 o;
     const bool ok = fx_dslash<0, true>(make_opk(0.1, 1, -1, true), v[0], v[1], v[2], v[3], v[4], q[0], q[1], q[2], q[3], o);
     const double2 z = fx_link_value(q[(int)r[0]]);
-    const double out[4] = {(double)ok, z.x, z.y, (double)marks};
+    const double out[5] = {(double)ok, z.x, z.y, o.x, o.y};
     fwrite(out, sizeof out, 1, stdout);
   }
 }
@@ -40,14 +36,19 @@ def test_an_open_link_is_not_summed_at_the_scale_behind_it(tmp_path):
     subprocess.run([os.environ.get("NVCC", "nvcc"), "-std=c++17", "-O1", "-gencode", "arch=compute_103a,code=sm_103a",
                     f"-I{ROOT}/thirring2d_gb300/csrc", f"-I{ROOT}/include", "-o", str(tmp_path / "h"), str(tmp_path / "h.cu")],
                    check=True, capture_output=True)
-    rec = np.array([(k, a, v) for k in range(4) for a in (0.0, 0.3, -2.0, 5e6, np.nan, np.inf) for v in (1.0, 1e20, 1e200)])
+    values = (1.0, 0.0, 1e-320, 1e20, -1e200)
+    rec = np.array([(k, a, v) for k in range(4) for a in (0.0, 0.3, -2.0, 5e6, np.nan, np.inf) for v in values])
     out = np.frombuffer(subprocess.run([str(tmp_path / "h")], input=rec.tobytes(), capture_output=True, check=True).stdout)
-    for (k, a, v), (ok, zx, zy, marks) in zip(rec, out.reshape(-1, 4)):
-        assert ok == 0                       # the FP64 form, in which 0 times the operand is 0
+    want = {}
+    for (k, a, v), (ok, zx, zy, x, y) in zip(rec, out.reshape(-1, 5)):
         if np.isfinite(a):
-            assert zx == 0 and zy == 0 and marks == 0
+            assert ok == 1 and zx == 0 and zy == 0
+            assert want.setdefault((k, a), (x, y)) == (x, y)   # whatever lies behind the link
         else:
-            assert np.isnan(zx) and np.isnan(zy)
+            assert ok == 0 and np.isnan(zx) and np.isnan(zy)
+    rec = np.array([(k, 0.3, v) for k in range(4) for v in (np.inf, -np.inf, np.nan)])   # 0 times these is NaN: the FP64 form
+    out = np.frombuffer(subprocess.run([str(tmp_path / "h")], input=rec.tobytes(), capture_output=True, check=True).stdout)
+    assert not out.reshape(-1, 5)[:, 0].any()
 
 
 @pytest.mark.gpu

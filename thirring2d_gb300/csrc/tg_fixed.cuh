@@ -27,8 +27,8 @@
 //
 // Exponents outside [kFxEmin, kFxEmax] (operands all zero, denormal, huge, Inf
 // or NaN), operator constants that are not finite, and links that are not
-// finite or lie across an open boundary (marked by bit 0 of the real low limb) take
-// the FP64 form: fx_dslash returns false and the caller computes the site in FP64.
+// finite (marked by bit 0 of the real low limb) take the FP64 form: fx_dslash
+// returns false and the caller computes the site in FP64.
 #pragma once
 
 #include <math.h>
@@ -148,9 +148,9 @@ TG_HD FxLink to_fx_link(double2 w) {
   l.w = i.lo;
   return l;
 }
-// A link across an open boundary, W = 0: marked too, because the operand behind it does
-// not contribute and must not set the scale of the site's sum (beside one 2^60 times the
-// others nothing would be left of them).  Bit 0 of both low limbs.
+// A link across an open boundary, W = 0, is marked too, and says so in bit 0 of the
+// imaginary low limb: the operand behind it does not contribute and must not set the scale
+// of the site's sum (beside one 2^60 times the others nothing would be left of them).
 TG_HD FxLink fx_open_link() {
   FxLink l;
   l.x = l.z = 0;
@@ -167,7 +167,7 @@ TG_HD double2 fx_link_value(FxLink l) {
   return w;
 }
 
-// Not finite (bit 0)
+// Marked and not finite (bit 0)
 TG_HD int fx_link_bad(FxLink l) { return l.y & ~l.w; }
 
 // Operator constants.  out = m in + cf Wt in(+t) + cb conj(Wt(-t)) in(-t) + ...;
@@ -272,11 +272,20 @@ TG_HD double fx_round(const FxAcc& a, int e) {
 template <int DAG, bool MU0>
 TG_HD bool fx_dslash(const OpK<double>& k, const FxC& pc, const FxC& ptu, const FxC& ptd, const FxC& pxu,
                      const FxC& pxd, FxLink wt, FxLink wtd, FxLink wx, FxLink wxd, double2& out) {
-  const int etu = MU0 ? ptu.e : ptu.e + k.fe, etd = MU0 ? ptd.e : ptd.e + k.be, ec = pc.e + k.me;
-  const int E = imax(imax(imax(etu, etd), imax(pxu.e, pxd.e)), ec);
+  const int ec = pc.e + k.me;
+  int etu = MU0 ? ptu.e : ptu.e + k.fe, etd = MU0 ? ptd.e : ptd.e + k.be, exu = pxu.e, exd = pxd.e;
+  int bad = (wt.y | wtd.y | wx.y | wxd.y) & 1;
+  if (bad) {  // not finite, or operands behind open boundaries (of which one that is not finite makes the site NaN)
+    bad = (fx_link_bad(wt) | fx_link_bad(wtd) | fx_link_bad(wx) | fx_link_bad(wxd)) & 1;
+    if ((wt.w & wt.y & 1) && ptu.e <= kFxEmax) etu = -4096;
+    if ((wtd.w & wtd.y & 1) && ptd.e <= kFxEmax) etd = -4096;
+    if ((wx.w & wx.y & 1) && pxu.e <= kFxEmax) exu = -4096;
+    if ((wxd.w & wxd.y & 1) && pxd.e <= kFxEmax) exd = -4096;
+  }
+  const int E = imax(imax(imax(etu, etd), imax(exu, exd)), ec);
   // the largest operand exponent itself: E can lie below it by a constant's
-  const int eraw = MU0 ? imax(E, pc.e) : imax(imax(imax(ptu.e, ptd.e), imax(pxu.e, pxd.e)), pc.e);
-  const bool ok = E >= k.emin && E <= kFxEmax && eraw <= kFxEmax && !((wt.y | wtd.y | wx.y | wxd.y) & 1);
+  const int eraw = MU0 ? imax(E, pc.e) : imax(imax(imax(etu - k.fe, etd - k.be), imax(exu, exd)), pc.e);
+  const bool ok = E >= k.emin && E <= kFxEmax && eraw <= kFxEmax && !bad;
   FxAcc x = {0, 0, 0, 0}, y = {0, 0, 0, 0};
   {
     const int d = imin(E - ec, 63);
@@ -285,8 +294,8 @@ TG_HD bool fx_dslash(const OpK<double>& k, const FxC& pc, const FxC& ptu, const 
   }
   fx_cmac<false, DAG != 0>(x, y, MU0 ? wt : fx_scale_link(wt, k.ff), ptu, E - etu);
   fx_cmac<true, DAG == 0>(x, y, MU0 ? wtd : fx_scale_link(wtd, k.fb), ptd, E - etd);
-  fx_cmac<false, DAG != 0>(x, y, wx, pxu, E - pxu.e);
-  fx_cmac<true, DAG == 0>(x, y, wxd, pxd, E - pxd.e);
+  fx_cmac<false, DAG != 0>(x, y, wx, pxu, E - exu);
+  fx_cmac<true, DAG == 0>(x, y, wxd, pxd, E - exd);
   out.x = fx_round(x, E);
   out.y = fx_round(y, E);
   return ok;
