@@ -139,3 +139,13 @@ def test_mixed_residuals_whose_squares_are_denormal(tg, oracle_lib, scale):
         x, res = L.fmdm_invert_cg(b, tg.cg_params(rel_tol=1e-11, abs_tol2=0, precision=1))
     assert res.status == 0
     assert np.linalg.norm(b - o.Mdag(A, o.M(A, x))) <= 1.5e-11 * np.linalg.norm(b)
+
+
+# the largest lattices that the cluster takes and the next ones, which the grid's shared memory does:
+# 16 blocks of 512 sites in FP64, of 2400 mixed; and the cluster's own limit with the grid's turned off
+@pytest.mark.parametrize("nt,nx,precision,env", [(90, 91, 0, {}), (91, 91, 0, {}), (64, 128, 0, {}), (195, 196, 1, {}), (196, 196, 1, {}),
+                                                 (120, 320, 1, {}), (113, 120, 0, {"TG_GRID_CG": "0"}), (220, 240, 1, {"TG_GRID_CG": "0"})])
+def test_hand_over_to_the_grid(tg, oracle_lib, monkeypatch, nt, nx, precision, env):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    test_solution_against_oracle(tg, oracle_lib, monkeypatch, nt, nx, 0.0, precision)

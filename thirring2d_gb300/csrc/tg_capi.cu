@@ -296,7 +296,9 @@ bool use_persistent(const tg_cg_params& cp) {
 // M^dag M pass per iteration); smaller lattices, whose vectors stay in L2 and
 // where the fused pass's halo recomputation costs more latency than the second
 // sum, run the two-sum CG (k_pcgmx).  Measured on GB300 (us per iteration,
-// fused / two-sum): 1024^2 30.3 / 21.7, 1536^2 58.1 / 58.6, 2048^2 93.8 / 102.5.
+// fused / two-sum): 1024^2 20.6 / 18.9, 1280^2 30.5 / 28.6, 1536^2 49.7 / 55.3, 2048^2
+// 83.8 / 99.6, 2000^2 86.8 / 107.7.  (The line was drawn with earlier kernels, for which 1536^2 was
+// even; up to 1.1 million sites the on-chip solver comes before either.)
 // TG_MIXED_CG=twosum|onesum overrides.
 bool use_single_reduction(const tg_lattice* L) {
   if (!L->g.march) return false;

@@ -638,14 +638,15 @@ static int ccg_max_cluster() {
 
 // The cluster's shape for a lattice, or none.  About 64 sites a block, up to 16
 // blocks: a pass is bound by its own latency until then (us per FP64 / mixed
-// iteration at 4, 8, 16 blocks: 16^2 3.3 / 2.2, 3.3 / 2.2, 3.4 / 2.3; 32^2 4.0 / 2.5,
-// 3.2 / 2.3, 3.0 / 2.3; 64^2 9.5 / 3.8, 6.2 / 3.5, 4.4 / 2.9), a block owns at
-// least a row.  One site per thread in FP64, two to four in the mixed solver
-// beyond 256 sites a block, whose shorter passes gain less from more warps than the sums
-// lose (96^2 at 512 / 256 threads: FP64 7.8 / 7.7, mixed 4.0 / 3.5; 128^2 9.8 /
-// 10.3, 4.4 / 4.1).  The grid solver takes over where the two meet: FP64 (cluster /
-// grid) 96^2 7.7 / 9.2, 112^2 8.8 / 9.2, 128^2 9.8 / 9.3; mixed 128^2 4.1 / 6.3, 256x192
-// 6.5 / 7.0, 256^2 7.6 / 7.1.
+// iteration at 1, 2, 4, 8, 16 blocks: 16^2 4.0 / 2.6, 3.3 / 2.5, 3.3 / 2.4, 3.3 / 2.5,
+// 3.3 / 2.6; at 4, 8, 16: 32^2 4.0 / 2.5, 3.2 / 2.3, 3.0 / 2.3; 64^2 9.5 / 3.8,
+// 6.2 / 3.5, 4.3 / 2.9), a block owns at least a row.  One site per thread in
+// FP64, two to four in the mixed solver beyond 256 sites a block, whose shorter
+// passes gain less from more warps than the sums lose (96^2 at 512 / 256
+// threads: FP64 7.8 / 7.7, mixed 4.0 / 3.5).  It gives way to the grid's
+// shared memory at 512 sites a block in FP64 and 2400 mixed (gcg_shape, with the figures of
+// both); its own limits, 850 and 3300, are where the solver of tg_pcg.cu was met
+// (128^2 FP64 9.8 / 9.3, 256^2 mixed 7.6 / 7.1), and hold where the grid's is turned off.
 // TG_CLUSTER_CG=0 turns it off, =blocks:threads sets the shape; the overrides of
 // the grid solvers (TG_PCG_BLOCK, TG_MIXED_CG) turn it off as well.
 CcgShape ccg_shape(const Geo& g, bool mixed) {

@@ -30,11 +30,9 @@ __device__ __forceinline__ void march_mdagm(const Geo& g, const OpK<float>& km, 
   using Op = typename Ld::Op;
   const int nt = g.nt, nx = g.nx;
   const int lane = threadIdx.x & 31;
-  const int x0 = xw << 5;
-  const int last = min(nx - x0, 32) - 1;          // the strip's last lane
-  const int x = x0 + min(lane, last);
-  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;    // column left of the warp
-  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;  // column right of the warp
+  const Strip sp = strip_of(nx, xw, lane);
+  const int last = sp.last, x = sp.x;
+  const int xle = sp.xle, xre = sp.xre;  // the columns left and right of the warp
   auto wrap = [nt](int t) { return t < 0 ? t + nt : (t >= nt ? t - nt : t); };
   const float2 zero = make_float2(0.f, 0.f);
 

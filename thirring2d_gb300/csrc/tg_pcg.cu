@@ -308,7 +308,9 @@ __device__ __forceinline__ double stop_of(double rr0, double rel_tol, double abs
 // (12.8 KB a warp, 205 KB a 512-thread block).  The prefetched march against one
 // with two rows' loads in registers, us per iteration: 1024^2 53.2 / 58.7, 512^2
 // 21.2 / 21.2.  16 warps per SM beat 12 (61.5 at 1024^2), 18 and 20 (62.5, 58.5: 88 B of
-// spills); two rows per step, interleaved, gave 56.4.
+// spills); two rows per step, interleaved, gave 56.4.  A lattice that does not march is
+// launched with the ring too: the L1 that it takes is no loss to one site per thread (2000x100
+// 14.00 us with, 14.02 without; 3000x170 36.6, 36.8; 20000x40 52.3, 52.5).
 constexpr int kRingRows = 4;
 constexpr int kRingWarp = ring_bytes<kRingRows, 1, 3>() > ring_bytes<kRingRows, 2, 0>()
                               ? ring_bytes<kRingRows, 1, 3>() : ring_bytes<kRingRows, 2, 0>();
@@ -869,18 +871,18 @@ int pcg_grid(const Geo& g, int resident, int bs) {
   return grid > 0 ? grid : 1;
 }
 
-// TG_PCG_BLOCK=512 runs any lattice on the launch shape of a lattice that
-// fills the GPU (one 512-thread block per SM, warps beyond the lattice's rows
-// idle), so small test lattices can hold that shape to the reference's
-// outputs; TG_PCG_BLOCK=256 forces the small-lattice shape.  Unset: by size.
 // From how many sites on the persistent solvers march.  One site per thread starts
 // each pass with all its loads, a march with its first rows'; its fewer loads and
 // operations win when threads have three sites and more.  us per iteration, march /
 // site by site: FP64 256^2 13.2 / 11.9, 384^2 17.1 / 16.3, 448^2 19.4 / 20.2, 512^2
-// 21.8 / 24.5, 1000^2 60.3 / 64.3, 2048^2 167 / 266; mixed 256^2 8.3 / 7.1, 512^2 10.4 / 10.4,
+// 21.8 / 24.5, 1000^2 51.3 / 64.3, 2048^2 168 / 266; mixed 256^2 8.3 / 7.1, 512^2 10.4 / 10.4,
 // 768^2 14.6 / 14.7, 1024^2 18.9 / 21.4, 1000^2 19.3 / 20.8.
 constexpr int kPcgMarch64 = 200000, kPcgMarchMx = 550000;
 
+// TG_PCG_BLOCK=512 runs any lattice on the launch shape of a lattice that
+// fills the GPU (one 512-thread block per SM, warps beyond the lattice's rows
+// idle), so small test lattices can hold that shape to the reference's
+// outputs; TG_PCG_BLOCK=256 forces the small-lattice shape.  Unset: by size.
 int pcg_block_override() {
   const char* e = getenv("TG_PCG_BLOCK");
   if (e == nullptr) return 0;

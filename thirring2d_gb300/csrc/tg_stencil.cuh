@@ -11,6 +11,21 @@
 
 namespace tg {
 
+// A lane's place in strip xw: columns x0 .. x0 + last are the strip's, x the lane's (the
+// lanes beyond repeat the last one), xle and xre the columns beside the strip.
+struct Strip {
+  int x0, last, x, xle, xre;
+};
+TG_HD Strip strip_of(int nx, int xw, int lane) {
+  Strip p;
+  p.x0 = xw << 5;
+  p.last = imin(nx - p.x0, 32) - 1;
+  p.x = p.x0 + imin(lane, p.last);
+  p.xle = (p.x0 == 0) ? nx - 1 : p.x0 - 1;
+  p.xre = (p.x0 + p.last + 1 == nx) ? 0 : p.x0 + p.last + 1;
+  return p;
+}
+
 // One row t of a warp's FP32 march: the operator at the sites (t, x0 + lane), lane
 // <= last, from psi(t-1) = pm, psi(t) = pc, psi(t+1) = pp and the links, with the
 // operand across the warp's edge pe (used by lanes 0 and last) and the x link
@@ -71,11 +86,8 @@ __device__ __forceinline__ void march_segment32(const Geo& g, const OpK<float>& 
   using R = float;
   const int nx = g.nx;
   const int lane = threadIdx.x & 31;
-  const int x0 = xw << 5;
-  const int last = min(nx - x0, 32) - 1;             // the strip's last lane
-  const int x = x0 + min(lane, last);
-  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;       // column left of the warp
-  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;  // column right of the warp
+  const Strip sp = strip_of(nx, xw, lane);
+  const int last = sp.last, x = sp.x, xle = sp.xle, xre = sp.xre;
   const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
   C2<R> pm = ld(tm * nx + x);
   C2<R> wtm = Wt[tm * nx + x];
@@ -136,11 +148,8 @@ __device__ __forceinline__ void march_segment64(const Geo& g, const OpK<double>&
   static_assert(kMarchT % kChunk64 == 0, "a chunk's edge operands are fetched kMarchT rows at a time");
   const int nx = g.nx;
   const int lane = threadIdx.x & 31;
-  const int x0 = xw << 5;
-  const int last = min(nx - x0, 32) - 1;
-  const int x = x0 + min(lane, last);
-  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
-  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;
+  const Strip sp = strip_of(nx, xw, lane);
+  const int last = sp.last, x = sp.x, xle = sp.xle, xre = sp.xre;
   const int tm = (ta == 0) ? g.nt - 1 : ta - 1;
   FxC pm = to_fx(ld(tm * nx + x));
   FxLink wtm = Wt[tm * nx + x];
@@ -222,6 +231,16 @@ template <int D, int NS, int NE> __host__ __device__ constexpr int ring_bytes() 
   return D * (NS + 2 + NE) * 512 + 2 * (NS + 1) * 2 * kMarchT * 16;
 }
 
+// The index arithmetic, host-callable for its audit: the row above row t; the slots of
+// a march's row i and of its chunk's edges; the site of the edge operand that lane
+// < 2 kMarchT fetches with the chunk whose first row is t (rows up to tb).
+TG_HD int row_above(int nt, int t) { return t + 1 == nt ? 0 : t + 1; }
+TG_HD int ring_slot(int i) { return i & (kMarchT - 1); }
+TG_HD int ring_edge_slot(int i) { return (i / kMarchT) & 1; }
+TG_HD int ring_edge(int nx, const Strip& p, int t, int tb, int lane) {
+  return imin(t + (lane & (kMarchT - 1)), tb - 1) * nx + (lane < kMarchT ? p.xle : p.xre);
+}
+
 // src[NS]: the operand's sources (comb(v) gives the operand from their values at
 // a site); ext[NE]: what the epilogue reads, handed to epi(s, out, operand, e).
 template <int DAG, bool MU0, int D, int NS, int NE, class Comb, class Epi>
@@ -232,17 +251,16 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
   constexpr int NA = NS + 2 + NE, EL = 2 * kMarchT;
   const int nx = g.nx, n = tb - ta;
   const int lane = threadIdx.x & 31;
-  const int x0 = xw << 5, last = min(nx - x0, 32) - 1, x = x0 + min(lane, last);
-  const int xle = (x0 == 0) ? nx - 1 : x0 - 1;
-  const int xre = (x0 + last + 1 == nx) ? 0 : x0 + last + 1;
+  const Strip st = strip_of(nx, xw, lane);
+  const int last = st.last, x = st.x;
   double2* const rows = reinterpret_cast<double2*>(ring) + lane;
   double2* const edges = reinterpret_cast<double2*>(ring + D * NA * 512) + (lane & (EL - 1));
   const unsigned rows_a = smem_addr(rows), edges_a = smem_addr(edges);
   // row ta + i into slot `slot`; with every kMarchT-th row the edges of its chunk
   auto issue = [&](int i, int slot) {
-    const int t = ta + i, tp = (t + 1 == g.nt) ? 0 : t + 1;
+    const int t = ta + i;
     const unsigned d = rows_a + slot * (NA * 512);
-    const int so = t * nx + x, sp = tp * nx + x;
+    const int so = t * nx + x, sp = row_above(g.nt, t) * nx + x;
     if (lane <= last) {  // (the spare lanes' copies of one address took a ragged strip's warps 17% longer)
 #pragma unroll
       for (int j = 0; j < NS; j++) cp_async16(d + j * 512, src[j] + sp);
@@ -252,9 +270,8 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
       for (int j = 0; j < NE; j++) cp_async16(d + (NS + 2 + j) * 512, ext[j] + so);
     }
     if ((i & (kMarchT - 1)) == 0 && lane < EL) {
-      const int rr = min(t + (lane & (kMarchT - 1)), tb - 1);
-      const int c = rr * nx + (lane < kMarchT ? xle : xre);
-      const unsigned e = edges_a + ((i / kMarchT) & 1) * ((NS + 1) * EL * 16);
+      const int c = ring_edge(nx, st, t, tb, lane);
+      const unsigned e = edges_a + ring_edge_slot(i) * ((NS + 1) * EL * 16);
 #pragma unroll
       for (int j = 0; j < NS; j++) cp_async16(e + j * (EL * 16), src[j] + c);
       if (lane < kMarchT) cp_async16(e + NS * (EL * 16), Wx + c);
@@ -283,11 +300,11 @@ __device__ __forceinline__ void march_ring64(const Geo& g, const OpK<double>& k,
     for (int ic = 0; ic < kMarchT; ic++) {
       const int i = i0 + ic;
       if (i >= n) break;
-      if (i + D - 1 < n) issue(i + D - 1, (ic + D - 1) % D);
+      if (i + D - 1 < n) issue(i + D - 1, ring_slot(ic + D - 1));  // (i0 is a multiple of D)
       cp_async_commit();
       cp_async_wait<D - 1>();
       if (ic == 0) {
-        const double2* e = edges + ((i0 / kMarchT) & 1) * ((NS + 1) * EL);
+        const double2* e = edges + ring_edge_slot(i0) * ((NS + 1) * EL);
         double2 v[NS];
 #pragma unroll
         for (int j = 0; j < NS; j++) v[j] = e[j * EL];
