@@ -20,10 +20,15 @@
 // alignment is per site, so a small operand beside larger ones loses no more
 // than it does to FP64 addition, and the result is a function of the site's
 // operands alone: every path that computes a site returns the same bits.
+// This is a bound for the site, not for each component: a part of a result far
+// below P (the imaginary part for a real vector on a field next to the cold one; a part of
+// an operand 2^53 times below its other) has P's absolute accuracy, where multiply-adds in
+// FP64 would keep more of it.  (Links with a part below 2^-21 in the FP64 form instead: a
+// 1024^2 field of Gaussian angles of 0.3 has five, and they cost its trajectory 10%.)
 //
-// Measured on GB300: the FP64 apply at 1024^2 32 -> 18.8 us and at 2048^2 135 ->
-// 78.5 us, the FP64 CG iteration at 1024^2 86.8 -> 58.7 us (52.5 with the rows
-// prefetched, tg_stencil.cuh); error against exact arithmetic 1.1e-16 relative (FP64 FMA order: 1.4e-16).
+// Measured on GB300: the FP64 apply at 1024^2 32 -> 19.2 us (0.3 of it the test for open
+// boundaries) and at 2048^2 135 -> 79 us, the FP64 CG iteration at 1024^2 86.8 -> 58.7 us (52.8 with the
+// rows prefetched, tg_stencil.cuh); error against exact arithmetic 1.1e-16 relative (FP64 FMA order: 1.4e-16).
 //
 // Exponents outside [kFxEmin, kFxEmax] (operands all zero, denormal, huge, Inf
 // or NaN), operator constants that are not finite, and links that are not

@@ -13,8 +13,8 @@
 //
 // Bound: two grid barriers and sums, about 2.5 us of the 6.3 us at 128^2; above,
 // the window's upkeep (at 256^2 a block keeps 431 sites and 512 neighbours) and the
-// operator's integer instructions.  us per iteration before and after: FP64 128^2 9.3 -> 6.3, 256^2
-// 12.1 -> 8.7, 400^2 19.9 -> 13.5; mixed 256^2 7.2 -> 6.1, 512^2 10.4 -> 7.8, 700^2 13.7 -> 9.8.
+// operator's integer instructions.  us per iteration before and after: FP64 128^2 9.3 -> 6.8, 256^2
+// 12.1 -> 9.1, 400^2 19.9 -> 13.7; mixed 256^2 7.2 -> 5.8, 512^2 10.4 -> 7.8, 700^2 13.7 -> 9.8.
 // Mixed lattices whose links no longer fit keep p, M p and r on chip and stream the
 // links from L2, ahead of their use: 800^2 15.1 -> 12.0, 1000^2 19.5 -> 15.3, 1024^2 18.9 -> 16.1.
 //
@@ -729,10 +729,10 @@ static int gcg_resident() {
 
 // Where it runs (us per iteration on GB300: this solver / the cluster solver / the
 // grid solver of tg_pcg.cu, whose passes read everything from L2):
-//   FP64   64^2 5.8 / 4.3 / 9.3   90^2 6.2 / 6.3 / 9.3   128^2 6.3 / - / 9.3
-//          256^2 8.7 / - / 12.1   400^2 13.5 / - / 19.9  16x1000 8.9 / - / 9.3
-//   mixed  128^2 5.6 / 4.1 / 6.3  190^2 6.0 / 5.9 / 6.5  228^2 6.1 / 6.8 / 7.0
-//          256^2 6.1 / - / 7.2    512^2 7.8 / - / 10.4   700^2 9.8 / - / 13.7
+//   FP64   64^2 5.8 / 4.3 / 9.3   90^2 6.2 / 6.1 / 9.3   128^2 6.8 / - / 9.3
+//          256^2 9.1 / - / 12.1   400^2 13.7 / - / 19.9  16x1000 8.9 / - / 9.3
+//   mixed  128^2 5.6 / 4.1 / 6.3  190^2 6.0 / 5.3 / 6.5  228^2 6.0 / 6.8 / 7.0
+//          256^2 5.8 / - / 7.2    512^2 7.8 / - / 10.4   700^2 9.8 / - / 13.7
 // In FP64 a cluster of 16 blocks is faster while each of its threads has one site
 // (512 a block), mixed up to 2400 sites a block.  Beyond, this solver takes what its
 // shared memory holds: about 170 000 sites in FP64 and 650 000 mixed, less the
